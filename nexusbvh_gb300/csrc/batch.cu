@@ -190,7 +190,7 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
         // overlapping H-PLOC of group k+1
         for (uint32_t k = 0; k < g.count; ++k) {
             NXB_TRY(launch_hploc_batch(keys, perm, a.parent, a.bvh2, mb, g.prim[k], g.prim[k + 1], t.radius, tokens,
-                                       a.pol, a.ctrl->leaf_ctr + k, &a.ctrl->error_word, t.hploc_ctas_per_sm, s,
+                                       a.pol, a.ctrl->hploc_tile_ctr + k, &a.ctrl->error_word, t.hploc_ctas_per_sm, s,
                                        a.kids));
             const uint32_t m0 = g.mesh[k];
             const MeshBatch view{a.off + m0, a.off8 + m0, g.mesh[k + 1] - m0};

@@ -197,12 +197,11 @@ nxb_status enqueue_build(const void* prims, nxb_prim_type type, uint32_t n, cons
     }
     // an even number of passes leaves the sorted keys / permutation in A
     NXB_TRY(mark(3));
-    // the sort's second value buffer holds the H-PLOC cluster tokens
     // with a BVH8 to build, the climb also writes each internal node's
     // children side by side, which the collapse reads instead of the BVH2
     ChildPair* kids = bvh8 ? reinterpret_cast<ChildPair*>(ws + L.kids) : nullptr;
-    NXB_TRY(launch_hploc(L.key_bytes, keys_a, vals_a, parent, bvh2, n, radius_of(cfg), vals_b,
-                         &ctrl->parent_of_last, &ctrl->hploc_leaf_ctr, &ctrl->error_word, s,
+    NXB_TRY(launch_hploc(L.key_bytes, keys_a, vals_a, parent, bvh2, n, radius_of(cfg),
+                         &ctrl->parent_of_last, &ctrl->hploc_tile_ctr, &ctrl->error_word, s,
                          reinterpret_cast<Node2*>(ws + L.records), bvh8 ? pairs : nullptr,
                          bvh8 ? ctrl->bvh8_ctr : nullptr, kids));
     NXB_TRY(mark(4));
@@ -730,7 +729,7 @@ nxb_status nxb_stage_radix_sort(uint32_t key_bytes, const void* d_keys_in, void*
     return NXB_OK;
 }
 
-// parent slots (4n) | cluster tokens (4n) | 2 counters | cluster records (32n)
+// parent slots (4n) | unused (4n) | 2 counters | cluster records (32n)
 size_t nxb_hploc_scratch_bytes(uint32_t n) { return 2 * align_up(4ull * n) + kAlign + align_up(32ull * n); }
 
 nxb_status nxb_stage_hploc(uint32_t key_bytes, const void* d_sorted_keys, uint32_t* d_cluster_idx,
@@ -744,14 +743,13 @@ nxb_status nxb_stage_hploc(uint32_t key_bytes, const void* d_sorted_keys, uint32
     if (scratch_bytes < nxb_hploc_scratch_bytes(n)) return NXB_ERR_WORKSPACE_TOO_SMALL;
     unsigned char* base = (unsigned char*)d_scratch;
     uint32_t* parent = (uint32_t*)base;
-    uint32_t* tokens = reinterpret_cast<uint32_t*>(base + align_up(4ull * n));
     uint32_t* words = reinterpret_cast<uint32_t*>(base + 2 * align_up(4ull * n));
     NXB_TRY(launch_fill_u32(parent, kInvalid, n, stream));
     NXB_TRY(launch_fill_u32(words, kInvalid, 1, stream));  // parent_of_last
-    NXB_TRY(launch_fill_u32(words + 1, 0, 1, stream));      // leaf counter
+    NXB_TRY(launch_fill_u32(words + 1, 0, 1, stream));      // tile counter
     Node2* records = reinterpret_cast<Node2*>(base + 2 * align_up(4ull * n) + kAlign);
     NXB_TRY(launch_hploc(key_bytes, d_sorted_keys, d_cluster_idx, parent, reinterpret_cast<Node2*>(d_nodes), n,
-                         search_radius, tokens, words, words + 1, d_error_word, stream, records));
+                         search_radius, words, words + 1, d_error_word, stream, records));
     return NXB_OK;
 }
 

@@ -4,33 +4,30 @@
 // The decisions are the reference's, so the topology and every box are
 // identical; how they are computed on the GPU differs:
 //   * the bottom-up LBVH climb (Apetrei 2014; FindParentId/Delta,
-//     BinaryBuilder.cu:14-40) runs on a persistent grid whose lanes take a
-//     new leaf as soon as their climb stops (see hploc_kernel); ranges are
-//     handed over with relaxed exchanges, a pass that merges is bracketed by
-//     acquire/release fences, and all cross-CTA data is read through L2
-//     (the reference reads cluster ids and node boxes with plain,
-//     L1-cacheable loads, which can return stale lines written by another
-//     SM);
-//   * LoadIndices (:42-57) loads the left and right windows of 16 cluster
-//     ids in one round trip (lanes 0-15 and 16-31) and packs them with one
-//     shuffle, instead of two dependent loads;
+//     BinaryBuilder.cu:14-40) is cut into tiles of consecutive sorted leaves.
+//     One CTA loads a tile's key deltas, ids and leaf boxes into shared
+//     memory once, and every LBVH node whose range lies inside the tile is
+//     climbed to, merged and handed over there; only subtrees that touch the
+//     tile's edge publish their clusters and climb on through global
+//     hand-over slots (see hploc_kernel).  All cross-CTA data is read
+//     through L2 after an acquire fence (the reference reads cluster ids and
+//     node boxes with plain, L1-cacheable loads, which can return stale
+//     lines written by another SM);
+//   * LoadIndices (:42-57): a window inside a tile is read from shared
+//     memory, its cluster count carried by the hand-over; a published window
+//     is read as 16 {box, id, token} records in one round trip;
 //   * FindNearestNeighbor (:126-163) is evaluated as what it computes: for
 //     lane i, the first minimum of the union area (compared as uint32 bit
-//     patterns) over candidates i+1, i-1, i+2, i-2, ..., i+R, i-R.  Each
-//     pair's area is computed once and sent back to the partner with one
-//     shuffle (7 shuffles per radius step instead of 10); at radius 8 a lane
-//     fetches only 4 neighbour boxes, at the offsets of a difference cover
-//     of the distances 1..8, and every pair is computed by one lane and
-//     shuffled to both of its lanes (36 shuffles per round instead of 56;
-//     at radius 16, 8 fetches and 72 shuffles instead of 16 and 112; at
-//     radius 4, 3 fetches and 23 shuffles instead of 4 and 28);
+//     patterns) over candidates i+1, i-1, i+2, i-2, ..., i+R, i-R, every
+//     pair's area computed by one lane and shuffled to the lanes it belongs
+//     to (see nearest_neighbour);
 //   * the merge and the order-preserving compaction follow
 //     MergeClustersCreateBVH2Node (:71-124); internal nodes are numbered
 //     from the tokens of the clusters they absorb instead of from a global
 //     atomic counter (see merge_step), and the root still lands at 2n-2.
-// A window whose valid ids are not a prefix (impossible for a correct
-// climb) sets NXB_DEVERR_HPLOC_INVALID_CLUSTER instead of reading out of
-// bounds.
+// A published window whose valid ids are not a prefix (impossible for a
+// correct climb) sets NXB_DEVERR_HPLOC_INVALID_CLUSTER instead of reading
+// out of bounds.
 #include <algorithm>
 
 #include "pipeline.h"
@@ -38,7 +35,6 @@
 namespace nxb {
 namespace {
 
-constexpr int kThreads = 128;
 constexpr uint32_t kMergeThreshold = 16;  // MERGING_THRESHOLD, BinaryBuilder.cu:10
 
 // Delta (BinaryBuilder.cu:16-28) of sorted positions a and b of the mesh
@@ -56,190 +52,161 @@ __device__ __forceinline__ uint64_t delta(const MeshKey* k, uint32_t a, uint32_t
     const uint32_t ka = (uint32_t)__ldg(&k[a].v), kb = (uint32_t)__ldg(&k[b].v);
     return (((uint64_t)ka << 32) | (a - s)) ^ (((uint64_t)kb << 32) | (b - s));
 }
-
-// The warp's row of shared memory: cluster k of the window at row[k]
-// (min xyz, max x) and row[32 + k] (max yz, id, token).
-__device__ __forceinline__ void put_row(uint4* row, uint32_t k, const Box& b, uint32_t cid, uint32_t ctok) {
-    row[k] = make_uint4(__float_as_uint(b.mn.x), __float_as_uint(b.mn.y), __float_as_uint(b.mn.z),
-                        __float_as_uint(b.mx.x));
-    row[32 + k] = make_uint4(__float_as_uint(b.mx.y), __float_as_uint(b.mx.z), cid, ctok);
+// The mesh of sorted position p (the high half of its key).
+__device__ __forceinline__ uint32_t mesh_of(const MeshKey* k, uint32_t p) { return (uint32_t)(__ldg(&k[p].v) >> 32); }
+template <typename K>
+__device__ __forceinline__ uint32_t mesh_of(const K*, uint32_t) {
+    return 0;
 }
-__device__ __forceinline__ Box row_box(const uint4* row, uint32_t k) {
-    const uint4 a = row[k];
-    const uint2 b = *reinterpret_cast<const uint2*>(row + 32 + k);
-    Box r;
-    r.mn = make_float3(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z));
-    r.mx = make_float3(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y));
-    return r;
+template <typename K, typename Seg>
+__device__ __forceinline__ MeshSpan span_at(const K* keys, const Seg& seg, uint32_t p) {
+    if constexpr (Seg::kBatch)
+        return seg.span(mesh_of(keys, p));
+    else
+        return seg.of_prim(p);
 }
 
-// COVER selects the difference-cover search (single-mesh builds, where it
-// measured faster at every radius; the batched kernel keeps the plain one).
-// ROW: the neighbour boxes are read from the warp's row of shared memory
-// instead of shuffled (see merge_step).
-template <int R, bool COVER, bool ROW = false>
-__device__ __forceinline__ uint32_t nearest_neighbour(uint32_t num, const Box& cb, const uint4* row = nullptr) {
-    const uint32_t lane = lane_id();
-    auto fetch = [&](uint32_t k) -> Box {
-        if constexpr (ROW)
-            return row_box(row, (lane + k) & 31u);
-        else
-            return shfl_box(cb, (lane + k) & 31u);
-    };
-    uint32_t best = kInvalid, best_idx = kInvalid;
-    if constexpr (R == 4 && COVER) {
-        // marks {0, 1, 2, 4}: 1 = 1-0, 2 = 2-0, 3 = 4-1, 4 = 4-0
-        auto pair = [&](const Box& lo_box, const Box& hi_box, uint32_t a, uint32_t d) -> uint32_t {
-            if (((lane + a) & 31u) + d >= num) return kInvalid;
-            Box u = hi_box;
-            grow(u, lo_box);
-            return __float_as_uint(half_area(u));
-        };
-        auto pick = [&](uint32_t f, uint32_t a, uint32_t d) {
-            const uint32_t fwd = a ? __shfl_sync(kFullMask, f, (lane - a) & 31u) : f;
-            const uint32_t back = __shfl_sync(kFullMask, f, (lane - d - a) & 31u);
-            if (fwd < best) {
-                best = fwd;
-                best_idx = lane + d;
-            }
-            if (back < best) {
-                best = back;
-                best_idx = lane - d;
-            }
-        };
-        const Box b1 = fetch(1);
-        pick(pair(cb, b1, 0, 1), 0, 1);
-        {
-            const Box b2 = fetch(2);
-            pick(pair(cb, b2, 0, 2), 0, 2);
-        }
-        const Box b4 = fetch(4);
-        const uint32_t f3 = pair(b1, b4, 1, 3), f4 = pair(cb, b4, 0, 4);
-        pick(f3, 1, 3);
-        pick(f4, 0, 4);
-    } else if constexpr ((R == 8 || R == 16) && COVER) {
-        // The marks {0, 1, 2, 5, 8} have every distance 1..8 as a difference
-        // (1 = 1-0, 2 = 2-0, 3 = 5-2, 4 = 5-1, 5 = 5-0, 6 = 8-2, 7 = 8-1,
-        // 8 = 8-0).  Each lane fetches the boxes of lanes +1, +2, +5 and +8
-        // (4 boxes instead of 8) and computes, for each distance d, the area
-        // of the pair (lane + a_d, lane + a_d + d), lanes taken modulo 32; a
-        // pair that wraps or reaches past the last cluster is invalid.  Every
-        // pair of the window is thereby computed by exactly one lane, and its
-        // area is shuffled to the two lanes it belongs to: 36 shuffles per
-        // round instead of 56.  The union is grown in the same operand order
-        // as below (upper box grown by the lower one), so every area has the
-        // same bits, and the candidates are compared in the same order.
-        auto pair = [&](const Box& lo_box, const Box& hi_box, uint32_t a, uint32_t d) -> uint32_t {
-            if (((lane + a) & 31u) + d >= num) return kInvalid;
-            Box u = hi_box;
-            grow(u, lo_box);
-            return __float_as_uint(half_area(u));
-        };
-        // two pairs' areas at once (half_area2)
-        auto pair2 = [&](const Box& lo0, const Box& hi0, uint32_t a0, uint32_t d0, const Box& lo1, const Box& hi1,
-                         uint32_t a1, uint32_t d1, uint32_t& f0, uint32_t& f1) {
-            Box u0 = hi0, u1 = hi1;
-            grow(u0, lo0);
-            grow(u1, lo1);
-            float r0, r1;
-            half_area2(u0, u1, r0, r1);
-            f0 = ((lane + a0) & 31u) + d0 >= num ? kInvalid : __float_as_uint(r0);
-            f1 = ((lane + a1) & 31u) + d1 >= num ? kInvalid : __float_as_uint(r1);
-        };
-        auto pick = [&](uint32_t f, uint32_t a, uint32_t d) {
-            const uint32_t fwd = a ? __shfl_sync(kFullMask, f, (lane - a) & 31u) : f;
-            const uint32_t back = __shfl_sync(kFullMask, f, (lane - d - a) & 31u);
-            if (fwd < best) {
-                best = fwd;
-                best_idx = lane + d;
-            }
-            if (back < best) {
-                best = back;
-                best_idx = lane - d;
-            }
-        };
-        const Box b1 = fetch(1);
-        const Box b2 = fetch(2);
-        {
-            uint32_t f1, f2;
-            pair2(cb, b1, 0, 1, cb, b2, 0, 2, f1, f2);
-            pick(f1, 0, 1);
-            pick(f2, 0, 2);
-        }
-        {
-            const Box b5 = fetch(5);
-            uint32_t f3, f4;
-            pair2(b2, b5, 2, 3, b1, b5, 1, 4, f3, f4);
-            pick(f3, 2, 3);
-            pick(f4, 1, 4);
-            pick(pair(cb, b5, 0, 5), 0, 5);
-        }
-        {
-            const Box b8 = fetch(8);
-            uint32_t f6, f7;
-            pair2(b2, b8, 2, 6, b1, b8, 1, 7, f6, f7);
-            pick(f6, 2, 6);
-            pick(f7, 1, 7);
-            pick(pair(cb, b8, 0, 8), 0, 8);
-        }
-        if constexpr (R == 16) {
-            // distances 9..16 are 8 + (1..8): the same low boxes 0, 1, 2
-            // against the boxes of lanes +9, +10, +13 and +16
-            {
-                const Box b9 = fetch(9);
-                const Box b10 = fetch(10);
-                uint32_t f9, f10;
-                pair2(cb, b9, 0, 9, cb, b10, 0, 10, f9, f10);
-                pick(f9, 0, 9);
-                pick(f10, 0, 10);
-            }
-            {
-                const Box b13 = fetch(13);
-                uint32_t f11, f12;
-                pair2(b2, b13, 2, 11, b1, b13, 1, 12, f11, f12);
-                pick(f11, 2, 11);
-                pick(f12, 1, 12);
-                pick(pair(cb, b13, 0, 13), 0, 13);
-            }
-            const Box b16 = fetch(16);
-            uint32_t f14, f15;
-            pair2(b2, b16, 2, 14, b1, b16, 1, 15, f14, f15);
-            pick(f14, 2, 14);
-            pick(f15, 1, 15);
-            pick(pair(cb, b16, 0, 16), 0, 16);
-        }
-    } else {
-#pragma unroll
-        for (uint32_t r = 1; r <= (uint32_t)R; ++r) {
-            Box nb = shfl_box(cb, (lane + r) & 31u);
-            uint32_t a = kInvalid;
-            if (lane + r < num) {
-                grow(nb, cb);
-                a = __float_as_uint(half_area(nb));
-            }
-            const uint32_t back = __shfl_sync(kFullMask, a, (lane - r) & 31u);
-            if (a < best) {
-                best = a;
-                best_idx = lane + r;
-            }
-            if (back < best) {
-                best = back;
-                best_idx = lane - r;
-            }
-        }
+// A run of clusters in shared memory: min xyz and max x, max yz, {id,
+// token}.  Three arrays, so that consecutive lanes read each of them without
+// a bank conflict (8-byte reads out of 16-byte records took two wavefronts
+// where one suffices: 21 % of the kernel's shared-memory load wavefronts).
+struct Row {
+    uint32_t a, b, c;  // shared-memory addresses
+    __device__ __forceinline__ Row at(int32_t k) const { return {a + 16 * k, b + 8 * k, c + 8 * k}; }
+    __device__ __forceinline__ void put(int32_t k, const Box& x, uint32_t cid, uint32_t ctok) const {
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a + 16 * k), "f"(x.mn.x), "f"(x.mn.y),
+                     "f"(x.mn.z), "f"(x.mx.x)
+                     : "memory");
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(b + 8 * k), "f"(x.mx.y), "f"(x.mx.z) : "memory");
+        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(c + 8 * k), "r"(cid), "r"(ctok) : "memory");
     }
-    return best_idx;
+    template <int K = 0>
+    __device__ __forceinline__ Box box() const {
+        Box r;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4 + %5];"
+                     : "=f"(r.mn.x), "=f"(r.mn.y), "=f"(r.mn.z), "=f"(r.mx.x)
+                     : "r"(a), "n"(16 * K));
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2 + %3];" : "=f"(r.mx.y), "=f"(r.mx.z) : "r"(b), "n"(8 * K));
+        return r;
+    }
+    __device__ __forceinline__ Box box(int32_t k) const { return at(k).box<0>(); }
+    __device__ __forceinline__ uint2 ids(int32_t k) const {
+        uint2 r;
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(c + 8 * k));
+        return r;
+    }
+};
+
+// Slots a row reaches before its first cluster (marks -2, -1) and past its
+// 32nd lane (the highest mark is lane + 3, 6 and 15 at radius 4, 8 and 16).
+constexpr int kRowFront = 2;
+constexpr int row_back(int radius) { return 32 + (radius / 3) * 3; }
+
+// half_area of the unions of two pairs.
+__device__ __forceinline__ void pair_areas(const Box& lo0, const Box& hi0, const Box& lo1, const Box& hi1, uint32_t& r0,
+                                           uint32_t& r1) {
+    Box a = hi0, b = hi1;
+    grow(a, lo0);
+    grow(b, lo1);
+    float f0, f1;
+    half_area2(a, b, f0, f1);
+    r0 = __float_as_uint(f0);
+    r1 = __float_as_uint(f1);
+}
+__device__ __forceinline__ uint32_t pair_area(const Box& lo, const Box& hi) {
+    Box u = hi;
+    grow(u, lo);
+    return __float_as_uint(half_area(u));
 }
 
-struct MergeCtx {
+// The better of two candidates; the first one wins a tie.
+struct Pick {
+    uint32_t area;
+    int32_t code;
+};
+__device__ __forceinline__ Pick first_min(Pick a, Pick b) {
+    const bool t = b.area < a.area;
+    return {t ? b.area : a.area, t ? b.code : a.code};
+}
+__device__ __forceinline__ Pick both_ways(uint32_t fwd, uint32_t back, int32_t d) {
+    return first_min({fwd, d}, {back, -d});
+}
+
+// The candidates at distances H, H+1, H+2 and beyond, from the mark lane + H.
+// The comparisons form a tree, not a chain of 2R: 285 -> 270 million ALU
+// instructions at 4.19M clustered triangles, and a shorter round for a warp
+// that runs alone.
+template <int R, int H>
+__device__ __forceinline__ Pick pick_group(uint32_t num, const Box& cb, const Box& b1, const Box& b0, const Row& own) {
+    const uint32_t lane = lane_id();
+    const Box hi = own.box<H>();
+    const bool in = lane + H < num;
+    const int down = (int)(lane - H);  // (taken modulo 32)
+    Pick group;
+    if constexpr (H + 1 <= R) {
+        uint32_t f0, f1;
+        pair_areas(cb, hi, b1, hi, f0, f1);
+        f0 = in ? f0 : kInvalid;
+        f1 = in && lane >= 1 ? f1 : kInvalid;
+        group = first_min(both_ways(f0, __shfl_sync(kFullMask, f0, down), H),
+                          both_ways(__shfl_down_sync(kFullMask, f1, 1), __shfl_sync(kFullMask, f1, down), H + 1));
+    } else {
+        const uint32_t f0 = in ? pair_area(cb, hi) : kInvalid;
+        group = both_ways(f0, __shfl_sync(kFullMask, f0, down), H);
+    }
+    if constexpr (H + 2 <= R) {
+        const uint32_t a2 = pair_area(b0, hi);
+        const uint32_t f2 = in && lane >= 2 ? a2 : kInvalid;
+        group = first_min(group, both_ways(__shfl_down_sync(kFullMask, f2, 2), __shfl_sync(kFullMask, f2, down), H + 2));
+    }
+    if constexpr (H + 3 <= R)
+        return first_min(group, pick_group<R, H + 3>(num, cb, b1, b0, own));
+    else
+        return group;
+}
+
+// The nearest neighbour of every lane's cluster, as a signed lane distance
+// (0: none); `own` is the lane's place in the row of the window's clusters,
+// cb its own box.
+// Each lane reads the boxes at lane-2, lane-1 and lane + 3k and computes the
+// pairs (lane-1, lane), (lane-2, lane) and, for each k, (lane, lane+3k),
+// (lane-1, lane+3k), (lane-2, lane+3k): every distance 1..R once, every pair
+// of the window by exactly one lane, with four box reads instead of eight at
+// radius 8 (three at radius 4, seven instead of sixteen at radius 16) and no
+// wrap-around: a pair is valid if its lower lane is not negative and its
+// upper one below num, which depends only on the two marks.  Each area then
+// goes to its two lanes (12 shuffles at radius 8).  The union is grown in
+// the operand order of the reference (upper box grown by the lower one).
+template <int R>
+__device__ __forceinline__ int32_t nearest_neighbour(uint32_t num, const Box& cb, const Row& own) {
+    const uint32_t lane = lane_id();
+    const Box b1 = own.box<-1>(), b0 = own.box<-2>();
+    Pick best;
+    {
+        uint32_t f1, f2;
+        pair_areas(b1, cb, b0, cb, f1, f2);
+        f1 = lane >= 1 && lane < num ? f1 : kInvalid;
+        f2 = lane >= 2 && lane < num ? f2 : kInvalid;
+        best = first_min(both_ways(__shfl_sync(kFullMask, f1, (lane + 1) & 31u), f1, 1),
+                         both_ways(__shfl_sync(kFullMask, f2, (lane + 2) & 31u), f2, 2));
+    }
+    return first_min(best, pick_group<R, 3>(num, cb, b1, b0, own)).code;
+}
+
+struct Outputs {
     Node2* nodes;
-    uint32_t* tok;             // first-leaf token of each stored cluster
-    Node2* rec;                // if not null: stored clusters as {box, id, token} records
     ChildPair* kids;           // if not null: each internal node's two children, at node - n
-    uint32_t* parent_of_last;  // node whose child is node 2n-2 (root fix-up)
-    uint32_t n;
-    uint32_t node_limit;       // 2n-1
+    uint32_t* parent_of_last;  // per mesh: the node whose child is node 2n-2 (root fix-up)
     uint32_t* err;
+};
+// The mesh a merge works on: node i is out.nodes[2 * start + i], its
+// child-pair record out.kids[start + i - n].
+struct MergeCtx {
+    const Outputs& out;
+    uint32_t mesh, start, n;
+    __device__ __forceinline__ uint32_t limit() const { return 2 * n - 1; }
+    __device__ __forceinline__ Node2* node(uint32_t i) const { return out.nodes + (2ull * start + i); }
+    __device__ __forceinline__ ChildPair* kid(uint32_t i) const { return out.kids + (start + (i - n)); }
 };
 
 // One round of PLOC merging (MergeClustersCreateBVH2Node,
@@ -249,70 +216,46 @@ struct MergeCtx {
 // absorb the tokens 1..n-1 exactly once, and node n-1+token(j) is a
 // collision-free index in [n, 2n-1) that needs no global counter (the
 // reference takes one atomicAdd on a single counter per merge round).
-// ROW: the window's clusters also live in the warp's row of shared memory,
-// which holds them at the start of every round: the merge reads its
-// partner there, and the order-preserving compaction goes through it (each
-// kept cluster written at its rank, every lane reading its own slot)
-// instead of a find-n-th-set-bit and eight shuffles.
-template <bool ROW>
-__device__ __forceinline__ uint32_t merge_step(const MergeCtx& m, uint32_t num, uint32_t nn, uint32_t& cid,
-                                               uint32_t& ctok, Box& cb, uint4* row) {
+// The row holds the clusters at the start of every round: the merge reads
+// its partner there, and the order-preserving compaction goes through it
+// (each kept cluster that moved or merged is written at its rank, every
+// lane reads its own slot).
+__device__ __forceinline__ uint32_t merge_step(const MergeCtx& m, uint32_t num, int32_t code, uint32_t& cid,
+                                               uint32_t& ctok, Box& cb, const Row& row) {
     const uint32_t lane = lane_id();
-    const uint32_t nn_of_nn = __shfl_sync(kFullMask, nn, nn & 31u);
-    const bool mutual = lane < num && lane == nn_of_nn;
-    const bool merge = mutual && lane < nn;
-    const uint32_t mmask = __ballot_sync(kFullMask, merge);
-    const uint32_t mcount = __popc(mmask);
-    uint32_t ncid, ntok;
-    Box nb;
-    if constexpr (ROW) {
-        if (merge) {
-            nb = row_box(row, nn & 31u);
-            const uint2 it = *reinterpret_cast<const uint2*>(&row[32 + (nn & 31u)].z);
-            ncid = it.x;
-            ntok = it.y;
-        }
-    } else {
-        ncid = __shfl_sync(kFullMask, cid, nn & 31u);
-        ntok = __shfl_sync(kFullMask, ctok, nn & 31u);
-        nb = shfl_box(cb, nn & 31u);
-    }
+    const uint32_t nn = (lane + code) & 31u;
+    const int32_t back = __shfl_sync(kFullMask, code, nn);
+    const bool mutual = lane < num && back == -code;
+    const bool merge = mutual && code > 0;
+    const bool keep = lane < num && !(mutual && code < 0);
+    const uint32_t kmask = __ballot_sync(kFullMask, keep);
+    const uint32_t rank = __popc(kmask & lanemask_lt());
+    const uint32_t left = __popc(kmask);
     if (merge) {
-        const uint32_t idx = m.n - 1 + ntok;
-        const bool ok = idx < m.node_limit && ntok != 0;
-        if (ok && m.kids) store_child_pair(m.kids + (idx - m.n), cb, nb, cid, ncid);
+        const Box nb = row.box(nn);
+        const uint2 it = row.ids(nn);
+        const uint32_t idx = m.n - 1 + it.y;
+        const bool ok = idx < m.limit() && it.y != 0;
+        if (ok && m.out.kids) store_child_pair(m.kid(idx), cb, nb, cid, it.x);
         grow(cb, nb);
         if (ok) {
-            store_node(m.nodes, idx, cb, cid, ncid);
-            if (cid == m.node_limit - 1 || ncid == m.node_limit - 1) atomicExch(m.parent_of_last, idx);
+            store_node(m.node(idx), 0, cb, cid, it.x);
+            if (cid == m.limit() - 1 || it.x == m.limit() - 1) atomicExch(m.out.parent_of_last + m.mesh, idx);
         } else {
-            set_error(m.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
+            set_error(m.out.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
         }
         cid = idx;
     }
-    const uint32_t vmask = __ballot_sync(kFullMask, merge || !mutual);
-    if constexpr (ROW) {
-        const uint32_t rank = __popc(vmask & lanemask_lt());
-        __syncwarp();  // the previous round's reads of the row are done
-        if ((vmask >> lane) & 1u) put_row(row, rank, cb, cid, ctok);
-        __syncwarp();
-        if (lane < (uint32_t)__popc(vmask)) {
-            const uint4 a = row[lane], b = row[32 + lane];
-            cb.mn = make_float3(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z));
-            cb.mx = make_float3(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y));
-            cid = b.z;
-            ctok = b.w;
-        } else {
-            cid = kInvalid;
-        }
-    } else {
-        const int sh = __fns(vmask, 0, lane + 1);
-        cid = __shfl_sync(kFullMask, cid, (uint32_t)sh & 31u);
-        ctok = __shfl_sync(kFullMask, ctok, (uint32_t)sh & 31u);
-        cb = shfl_box(cb, (uint32_t)sh & 31u);
-        if (sh < 0) cid = kInvalid;
+    __syncwarp();  // every read of the row is done
+    if (keep && (merge || rank != lane)) row.put(rank, cb, cid, ctok);
+    __syncwarp();
+    if (lane < left) {
+        cb = row.box(lane);
+        const uint2 it = row.ids(lane);
+        cid = it.x;
+        ctok = it.y;
     }
-    return num - mcount;
+    return left;
 }
 
 // The last merge of the build (the root, two clusters left in lanes 0 and
@@ -326,21 +269,21 @@ __device__ __forceinline__ void merge_root(const MergeCtx& m, uint32_t& cid, uin
     const Box b_box = shfl_box(cb, 1);
     __syncwarp();
     if (lane == 0) {
-        const uint32_t root = m.node_limit - 1;
+        const uint32_t root = m.limit() - 1;
         const uint32_t natural = m.n - 1 + b_tok;
         uint32_t a = cid, b = b_cid;
         if (natural != root) {
-            if (natural >= m.node_limit) {
-                set_error(m.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
+            if (natural >= m.limit()) {
+                set_error(m.out.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
             } else {
-                const uint4* src = reinterpret_cast<const uint4*>(m.nodes + root);
-                uint4* dst = reinterpret_cast<uint4*>(m.nodes + natural);
+                const uint4* src = reinterpret_cast<const uint4*>(m.node(root));
+                uint4* dst = reinterpret_cast<uint4*>(m.node(natural));
                 const uint4 lo = __ldcg(src), hi = __ldcg(src + 1);
                 __stcg(dst, lo);
                 __stcg(dst + 1, hi);
-                if (m.kids) {  // the moved node's child pair moves with it
-                    const uint4* ks = reinterpret_cast<const uint4*>(m.kids + (root - m.n));
-                    uint4* kd = reinterpret_cast<uint4*>(m.kids + (natural - m.n));
+                if (m.out.kids) {  // the moved node's child pair moves with it
+                    const uint4* ks = reinterpret_cast<const uint4*>(m.kid(root));
+                    uint4* kd = reinterpret_cast<uint4*>(m.kid(natural));
                     const uint4 k0 = __ldcg(ks), k1 = __ldcg(ks + 1), k2 = __ldcg(ks + 2), k3 = __ldcg(ks + 3);
                     __stcg(kd, k0);
                     __stcg(kd + 1, k1);
@@ -352,281 +295,460 @@ __device__ __forceinline__ void merge_root(const MergeCtx& m, uint32_t& cid, uin
                 } else if (b == root) {
                     b = natural;
                 } else {
-                    const uint32_t p = __ldcg(m.parent_of_last);
-                    if (p < m.node_limit && p >= m.n) {
-                        uint32_t* pl = reinterpret_cast<uint32_t*>(m.nodes + p) + 6;
+                    const uint32_t p = __ldcg(m.out.parent_of_last + m.mesh);
+                    if (p < m.limit() && p >= m.n) {
+                        uint32_t* pl = reinterpret_cast<uint32_t*>(m.node(p)) + 6;
                         const uint32_t side = __ldcg(pl) == root ? 0u : 1u;
                         __stcg(pl + side, natural);
-                        if (m.kids) __stcg(&m.kids[p - m.n].li + side, natural);
+                        if (m.out.kids) __stcg(&m.kid(p)->li + side, natural);
                     } else {
-                        set_error(m.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
+                        set_error(m.out.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
                     }
                 }
             }
         }
-        if (m.kids) store_child_pair(m.kids + (root - m.n), cb, b_box, a, b);
+        if (m.out.kids) store_child_pair(m.kid(root), cb, b_box, a, b);
         grow(cb, b_box);
-        store_node(m.nodes, root, cb, a, b);
+        store_node(m.node(root), 0, cb, a, b);
         cid = root;
     }
-    if (lane == 1) cid = kInvalid;
 }
 
-// The mesh of the owner lane: `all` holds the bases of the concatenated
-// arrays; the context returned addresses this mesh's nodes and counter.
-template <typename Seg>
-__device__ __forceinline__ MergeCtx mesh_ctx(const MergeCtx& all, const Seg& seg, MeshSpan me, uint32_t owner,
-                                             uint32_t& start) {
-    if constexpr (Seg::kBatch) {
-        const uint32_t mesh = __shfl_sync(kFullMask, me.m, owner);
-        start = __shfl_sync(kFullMask, me.start, owner);
-        const uint32_t count = __shfl_sync(kFullMask, me.count, owner);
-        return MergeCtx{all.nodes + 2ull * start, all.tok, all.rec, all.kids ? all.kids + start : nullptr,
-                        all.parent_of_last + mesh, count, 2 * count - 1, all.err};
-    } else {
-        start = 0;
-        return all;
-    }
-}
-
-// PlocMerge (BinaryBuilder.cu:200-273, the merge part) for the range of
-// lane `owner`; `start` is the first sorted position of its mesh and m
-// addresses that mesh's nodes.
-template <int R, bool COVER, bool REC>
-__device__ __forceinline__ void merge_windows(uint32_t owner, uint32_t left, uint32_t right, uint32_t split,
-                                              bool final, uint32_t start, uint32_t* cluster, const MergeCtx& m,
-                                              uint4* row) {
-    const uint32_t lane = lane_id();
-    const uint32_t l_start = __shfl_sync(kFullMask, left, owner);
-    const uint32_t r_end = __shfl_sync(kFullMask, right, owner) + 1;
-    const uint32_t mid = __shfl_sync(kFullMask, split, owner);
-    const bool fin = __shfl_sync(kFullMask, final ? 1u : 0u, owner) != 0;
-
-    // LoadIndices (BinaryBuilder.cu:42-57) for both children at once: lanes
-    // 0-15 read the left window, lanes 16-31 the right one.  A child of at
-    // most 16 primitives was never merged, so its ids and tokens are the
-    // original ones (token = mesh-local position); a larger child was stored
-    // compacted.
-    const uint32_t l_len = mid - l_start, r_len = r_end - mid;
-    const uint32_t l_size = min(l_len, kMergeThreshold);
-    const uint32_t r_size = min(r_len, kMergeThreshold);
-    uint32_t v = kInvalid, t = kInvalid;
-    Box wb;  // REC: the window's box at its position, before compaction
-    wb.mn = make_float3(0.f, 0.f, 0.f);
-    wb.mx = wb.mn;
-    {
-        const bool lo = lane < 16;
-        const uint32_t k = lo ? lane : lane - 16;
-        if (k < (lo ? l_size : r_size)) {
-            const uint32_t pos = (lo ? l_start : mid) + k;
-            const bool stored = (lo ? l_len : r_len) > kMergeThreshold;
-            if constexpr (REC) {
-                if (stored) {
-                    // a stored window: id, token and box in one record, 16
-                    // consecutive records per window
-                    const uint4* p = reinterpret_cast<const uint4*>(m.rec + pos);
-                    const uint4 a = __ldcg(p), b = __ldcg(p + 1);
-                    wb.mn = make_float3(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z));
-                    wb.mx = make_float3(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y));
-                    v = b.z;
-                    t = b.w;
-                } else {
-                    v = __ldcg(cluster + pos);
-                    t = pos - start;
-                    if (v < m.node_limit) wb = load_box_cg(m.nodes, v);
-                }
-            } else {
-                v = __ldcg(cluster + pos);
-                t = stored ? __ldcg(m.tok + pos) : pos - start;
-            }
-        }
-    }
-    const uint32_t vb = __ballot_sync(kFullMask, v != kInvalid);
-    const uint32_t num_left = __popc(vb & 0xFFFFu), num_right = __popc(vb >> 16);
-    if ((vb & 0xFFFFu) != ((1u << num_left) - 1u) || (vb >> 16) != ((1u << num_right) - 1u)) {
-        if (lane == 0) set_error(m.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
-        return;
-    }
-    uint32_t num = num_left + num_right;
-    const uint32_t src = (lane < num_left ? lane : 16u + lane - num_left) & 31u;
-    uint32_t cid = __shfl_sync(kFullMask, v, src);
-    uint32_t ctok = __shfl_sync(kFullMask, t, src);
-    if (lane >= num) cid = kInvalid;
-    if (__ballot_sync(kFullMask, lane < num && (cid >= m.node_limit || ctok >= m.n))) {
-        if (lane == 0) set_error(m.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
-        return;
-    }
-    Box cb;
-    if constexpr (REC) {
-        cb = shfl_box(wb, src);
-        if (lane >= num) {
-            cb.mn = make_float3(0.f, 0.f, 0.f);
-            cb.mx = cb.mn;
-        }
-    } else {
-        if (lane < num) {
-            cb = load_box_cg(m.nodes, cid);
-        } else {
-            cb.mn = make_float3(0.f, 0.f, 0.f);
-            cb.mx = cb.mn;
-        }
-    }
-    if constexpr (REC) {
-        put_row(row, lane, cb, cid, ctok);
-        __syncwarp();
-    }
+// Merges the window's clusters (in the registers of lanes 0..num-1 and in
+// the row) down to at most 16, or to one for the last node of a mesh;
+// returns how many are left, in the same places.  Every round merges a pair,
+// whatever the boxes hold (areas compare as uint32): of the pairs with the
+// least area, then the least distance, the one with the highest lanes is
+// mutual, as its lower lane prefers forward and its upper lane has no such
+// pair ahead of it.
+template <int R>
+__device__ __forceinline__ uint32_t merge_window(const MergeCtx& m, uint32_t num, bool fin, uint32_t& cid,
+                                                 uint32_t& ctok, Box& cb, const Row& row) {
     const uint32_t threshold = fin ? 1u : kMergeThreshold;
     while (num > threshold) {
         if (fin && num == 2) {
             merge_root(m, cid, ctok, cb);
-            num = 1;
+            return 1;
+        }
+        const int32_t code = nearest_neighbour<R>(num, cb, row.at(lane_id()));
+        num = merge_step(m, num, code, cid, ctok, cb, row);
+    }
+    return num;
+}
+
+// Where subtrees that leave their tile keep their clusters.  A plain build
+// stores them as {box, id, token} records at the window's positions, so the
+// next merge reads 16 consecutive records in one round trip; a batch, which
+// has no room for records, stores id and token and reads the box from the
+// node array.
+struct Published {
+    Node2* rec;         // plain builds
+    uint32_t* cluster;  // batches
+    uint32_t* tok;
+    template <typename Seg>
+    __device__ __forceinline__ void store(uint32_t pos, const Box& b, uint32_t cid, uint32_t ctok) const {
+        if constexpr (Seg::kBatch) {
+            __stcg(cluster + pos, cid);
+            __stcg(tok + pos, ctok);
+        } else {
+            uint4* p = reinterpret_cast<uint4*>(rec + pos);
+            __stcg(p, make_uint4(__float_as_uint(b.mn.x), __float_as_uint(b.mn.y), __float_as_uint(b.mn.z),
+                                 __float_as_uint(b.mx.x)));
+            __stcg(p + 1, make_uint4(__float_as_uint(b.mx.y), __float_as_uint(b.mx.z), cid, ctok));
+        }
+    }
+};
+
+// ---------------------------------------------------------------- tiles
+// A tile is a run of consecutive sorted leaves held in shared memory by one
+// warp.  Gap j of a tile lies between its positions j-1 and j (0..cnt).
+// Largest tile and resident warps, measured on GB300 (H-PLOC of 12.58M
+// clustered triangles, 63-bit): 128 leaves x 31 warps (64 registers, spills)
+// 2.23 ms, 144 x 28 (72 registers, no spills at radius 8) 2.12, 160 x 26
+// 2.16, 176 x 24 2.17, 192 x 22 2.22.  Four CTAs of 7 warps and one of 28
+// measure the same; the small CTA leaves room beside it on the SM.
+constexpr int kTile = 144;
+constexpr int kTileWarps = 7;  // per CTA
+constexpr int kTileCtas = 4;   // per SM
+constexpr uint64_t kEdge = ~0ull;  // the delta across a mesh's end
+template <int R>
+struct __align__(16) WarpTile {
+    static constexpr int kRows = kTile + kRowFront + row_back(R);
+    uint4 a[kRows];
+    uint2 b[kRows];
+    uint2 c[kRows];
+    uint64_t gap[kTile + 2];   // deltas; then the list of subtrees that leave the tile
+    uint32_t hand[kTile + 4];  // hand-over slots: the range's other end | clusters << 16
+    __device__ __forceinline__ Row rows() {
+        return {(uint32_t)__cvta_generic_to_shared(a + kRowFront), (uint32_t)__cvta_generic_to_shared(b + kRowFront),
+                (uint32_t)__cvta_generic_to_shared(c + kRowFront)};
+    }
+};
+
+template <typename K, typename Seg>
+struct Climb {
+    const K* keys;
+    uint32_t* cluster;
+    uint32_t* parent;
+    Seg seg;
+    Outputs out;
+    Published pub;
+    uint32_t begin, end, tile;  // tile: leaves per tile
+    uint64_t* bvh8_pairs;
+};
+
+// LoadIndices (BinaryBuilder.cu:42-57): one lane's entry k of a published
+// window of `size` leaves at `pos`.
+template <typename K, typename Seg>
+__device__ __forceinline__ void load_entry(const Climb<K, Seg>& g, const MergeCtx& m, uint32_t pos, uint32_t k,
+                                           uint32_t size, uint32_t& v, uint32_t& t, Box& b) {
+    v = kInvalid;
+    t = 0;
+    b.mn = b.mx = make_float3(0.f, 0.f, 0.f);
+    if (k >= min(size, kMergeThreshold)) return;
+    if constexpr (Seg::kBatch) {
+        v = __ldcg(g.pub.cluster + pos + k);
+        t = __ldcg(g.pub.tok + pos + k);
+        if (v < m.limit()) b = load_box_cg(m.node(v), 0);
+    } else {
+        const uint4* p = reinterpret_cast<const uint4*>(g.pub.rec + pos + k);
+        const uint4 lo = __ldcg(p), hi = __ldcg(p + 1);
+        b.mn = make_float3(__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z));
+        b.mx = make_float3(__uint_as_float(lo.w), __uint_as_float(hi.x), __uint_as_float(hi.y));
+        v = hi.z;
+        t = hi.w;
+    }
+}
+
+// PlocMerge (BinaryBuilder.cu:200-273, the merge part) between tiles, for
+// the range of lane `owner`, whose two children were published; then on up
+// the tree for as long as the sibling has already arrived: its hand-over
+// slot is read (acquire) instead of exchanged, and the range's own clusters
+// stay in the row, so such a level has no fence, no exchange and one window
+// to load.  Returns the range reached and whether it is a whole mesh; the
+// clusters of a range that is not are stored (StoreIndices, :59-69).
+template <int R, typename K, typename Seg>
+__device__ __forceinline__ bool merge_between(const Climb<K, Seg>& g, uint32_t owner, uint32_t& left, uint32_t& right,
+                                              uint32_t split, const Row& row) {
+    const uint32_t lane = lane_id();
+    uint32_t l = __shfl_sync(kFullMask, left, owner), r = __shfl_sync(kFullMask, right, owner);
+    const uint32_t mid = __shfl_sync(kFullMask, split, owner);
+    const MeshSpan me = span_at(g.keys, g.seg, l);
+    const uint32_t start = me.start;
+    const MergeCtx m{g.out, me.m, start, me.count};
+    uint32_t cid, ctok, num, first;
+    Box cb;
+    bool bad;  // a window's valid ids must be a prefix of it, and in range
+    {
+        const bool lo = lane < 16;
+        load_entry(g, m, lo ? l : mid, lane & 15u, lo ? mid - l : r + 1 - mid, cid, ctok, cb);
+        const uint32_t vb = __ballot_sync(kFullMask, cid != kInvalid);
+        first = __popc(vb & 0xFFFFu);
+        num = __popc(vb);
+        bad = (vb & 0xFFFFu) != (1u << first) - 1u || vb >> 16 != (1u << (num - first)) - 1u;
+        __syncwarp();  // the row's last readers are done
+        if (cid != kInvalid) row.put(lo ? lane : first + lane - 16, cb, cid, ctok);
+    }
+    bool fin = false;
+    for (;;) {
+        __syncwarp();
+        cid = kInvalid;
+        if (lane < num) {
+            cb = row.box(lane);
+            const uint2 it = row.ids(lane);
+            cid = it.x;
+            ctok = it.y;
+        }
+        if (bad || __any_sync(kFullMask, lane < num && (cid >= m.limit() || ctok >= m.n))) {
+            if (lane == 0) set_error(m.out.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
+            fin = true;
             break;
         }
-        const uint32_t nn = nearest_neighbour<R, COVER, REC>(num, cb, row);
-        num = merge_step<REC>(m, num, nn, cid, ctok, cb, row);
+        fin = r - l + 1 == m.n;
+        num = merge_window<R>(m, num, fin, cid, ctok, cb, row);
+        if (fin) break;
+        const bool can_l = l != start, can_r = r != start + m.n - 1;
+        const uint32_t vl = can_l ? ld_acquire_u32(g.parent + l - 1) : kInvalid;
+        const uint32_t vr = can_r ? ld_acquire_u32(g.parent + r) : kInvalid;
+        const bool go_right =
+            !can_l || (can_r && delta(g.keys, r, r + 1, start) < delta(g.keys, l - 1, l, start));
+        const uint32_t other = __shfl_sync(kFullMask, go_right ? vr : vl, 0);
+        if (other == kInvalid) break;
+        uint32_t v, t;
+        Box b;
+        load_entry(g, m, go_right ? r + 1 : other, lane, go_right ? other - r : l - other, v, t, b);
+        const uint32_t vb = __ballot_sync(kFullMask, v != kInvalid);
+        const uint32_t ns = __popc(vb);
+        bad = (vb & (vb + 1)) != 0;
+        __syncwarp();
+        if (!go_right && lane < num) row.put(ns + lane, cb, cid, ctok);
+        if (v != kInvalid) row.put((go_right ? num : 0u) + lane, b, v, t);
+        num += ns;
+        if (go_right)
+            r = other;
+        else
+            l = other;
     }
-    // StoreIndices (BinaryBuilder.cu:59-69)
-    if (lane < num_left + num_right) {
-        if constexpr (REC) {
-            uint4* p = reinterpret_cast<uint4*>(m.rec + l_start + lane);
-            __stcg(p, make_uint4(__float_as_uint(cb.mn.x), __float_as_uint(cb.mn.y), __float_as_uint(cb.mn.z),
-                                 __float_as_uint(cb.mx.x)));
-            __stcg(p + 1, make_uint4(__float_as_uint(cb.mx.y), __float_as_uint(cb.mx.z), cid, ctok));
-        } else {
-            __stcg(cluster + l_start + lane, cid);
-            __stcg(m.tok + l_start + lane, ctok);
-        }
+    if (!fin && lane < min(r - l + 1, kMergeThreshold)) g.pub.template store<Seg>(l + lane, cb, lane < num ? cid : kInvalid, ctok);
+    if (lane == owner) {
+        left = l;
+        right = r;
     }
+    return fin;
 }
 
-// Inlined into the climb loop (measured on GB300: batch1024 9.74 -> 9.35 ms,
-// clustered12m H-PLOC 2.52 -> 2.49 ms against an out-of-line call; with the
-// launch bounds above neither kernel spills).
-template <int R, typename Seg>
-__device__ __forceinline__ void ploc_merge(uint32_t owner, uint32_t left, uint32_t right, uint32_t split, bool final,
-                                        MeshSpan me, uint32_t* cluster, const MergeCtx& all, const Seg& seg,
-                                        uint4* row) {
-    if constexpr (Seg::kBatch) {
-        uint32_t start;
-        const MergeCtx m = mesh_ctx<Seg>(all, seg, me, owner, start);
-        merge_windows<R, false, false>(owner, left, right, split, final, start, cluster, m, row);
-    } else {
-        merge_windows<R, true, true>(owner, left, right, split, final, 0u, cluster, all, row);
-    }
-}
-
-// The climb with lane refill.  Each lane climbs from a leaf as in the
-// reference (FindParentId, exchange on the parent's hand-over slot, merge
-// and continue when second to arrive), but a lane that stops takes the next
-// unclaimed leaf from its warp's chunk (chunks of `chunk` leaves are
-// claimed with one atomicAdd), instead of idling until every lane of its
-// warp has finished: the reference runs one thread per leaf, and a warp
-// stays resident for as long as any of its lanes still climbs (most stop
-// after a step or two).  Nothing waits on another warp.
-// Memory order: the hand-over exchanges are relaxed; a pass that merges
-// fences (acquire) after its exchanges, before reading the siblings'
-// clusters, and (release) after its merges, before the next exchanges.
-// Chunk size, measured on GB300 (12.58M clustered triangles, 6,080 resident
-// warps): 64 -> 2.91 ms, 256 -> 2.68 ms, 1024 -> 2.90 ms, 4096 -> 5.33 ms.
-// Larger chunks keep more of each subtree's climb inside one warp and
-// touch the shared counter less; too large leaves warps without work.  So
-// the chunk is about two per resident warp, rounded to a multiple of 32
-// between 32 and a cap (384 for one mesh, 256 for a batch: the best
-// measured caps).  65,536 triangles: 32 (H-PLOC 0.162 -> 0.125 ms against a
-// fixed 256); 4.19M: 384 (0.655 -> 0.614 ms); 12.58M: 384 (2.52 ms, as 256).
-uint32_t leaf_chunk(uint32_t leaves, uint32_t warps, bool batch) {
-    const uint32_t cap = batch ? 256u : 384u;
-    const uint32_t c = (leaves / (2u * std::max(warps, 1u)) + 16u) / 32u * 32u;
-    return std::max(32u, std::min(c, cap));
-}
-
-// Resident CTAs per SM, measured on GB300: a single-mesh build keeps the
-// neighbour boxes of its difference-cover search in registers (radius 8:
-// 56 registers, 9 CTAs; radius 16: 64 registers, 8 CTAs; with fewer
-// registers they spill and lose the gain); the batched kernel and radius 4
-// (3 boxes) run at 40 registers.
-template <int R, typename Seg>
-constexpr int hploc_ctas_per_sm() {
-    if constexpr (Seg::kBatch) return 12;
-    return R == 8 ? 9 : (R == 16 ? 8 : 12);
-}
-
-template <typename K, int R, typename Seg>
-__global__ __launch_bounds__(kThreads, hploc_ctas_per_sm<R, Seg>()) void hploc_kernel(const K* __restrict__ keys, uint32_t* cluster,
-                                                         uint32_t* parent, Node2* nodes, Seg seg, uint32_t begin,
-                                                         uint32_t* tok, uint32_t* parent_of_last, uint32_t* leaf_ctr,
-                                                         uint32_t* err, uint32_t end, uint32_t chunk, Node2* rec,
-                                                         uint64_t* bvh8_pairs, uint32_t* bvh8_ctr, ChildPair* kids) {
+// Loads leaves [base, base + cnt) into the warp's tile: the gaps' deltas,
+// the leaves' ids and boxes.
+template <int R, typename K, typename Seg>
+__device__ __forceinline__ void load_tile(const Climb<K, Seg>& g, WarpTile<R>& t, uint32_t base, uint32_t cnt) {
+    constexpr int kPer = (kTile + 31) / 32;
     const uint32_t lane = lane_id();
-    if (!Seg::kBatch && bvh8_ctr && blockIdx.x == 0 && threadIdx.x == 0) bvh8_queue_counters(bvh8_ctr);
-    const MergeCtx all{nodes, tok, rec, kids, parent_of_last, end, 2 * end - 1, err};
-    // each warp's row for the merge compaction (single-mesh builds)
-    __shared__ uint4 s_rows[Seg::kBatch ? 1 : kThreads / 32][64];
-    uint4* row = s_rows[Seg::kBatch ? 0 : threadIdx.x >> 5];
-    uint32_t left = 0, right = 0, split = 0;
-    // the lane's mesh; a plain build has one, known at compile time
-    MeshSpan me = Seg::kBatch ? MeshSpan{0, 0, 0} : seg.of_prim(0);
+    const Row rows = t.rows();
+    // most tiles of a batch lie inside one mesh
+    MeshSpan first = span_at(g.keys, g.seg, base);
+    const bool one = !Seg::kBatch || base + cnt <= first.start + first.count;
+    uint32_t id[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const uint32_t j = lane + 32 * q;
+        id[q] = j < cnt ? __ldcg(g.cluster + base + j) : kInvalid;
+    }
+#pragma unroll
+    for (int q = 0; q <= kPer; ++q) {
+        const uint32_t j = lane + 32 * q;
+        if (j > cnt) break;
+        const uint32_t p = base + j;
+        uint32_t start = first.start;
+        bool edge;
+        if (one) {
+            edge = p == start || p == start + first.count;
+        } else {
+            edge = p == g.begin || p == g.end || mesh_of(g.keys, p - 1) != mesh_of(g.keys, p);
+            if (!edge) start = span_at(g.keys, g.seg, p).start;
+        }
+        uint64_t d = kEdge;
+        if (!edge) {
+            d = delta(g.keys, p - 1, p, start);
+            d = d < kEdge ? d : kEdge - 1;  // only a mesh's end is an edge
+        }
+        t.gap[j] = d;
+        t.hand[j] = kInvalid;
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const uint32_t j = lane + 32 * q;
+        if (j < cnt) {
+            const MeshSpan me = one ? first : span_at(g.keys, g.seg, base + j);
+            Box b;
+            b.mn = b.mx = make_float3(0.f, 0.f, 0.f);
+            if (id[q] < me.count)
+                b = load_box(g.out.nodes + 2ull * me.start, id[q]);
+            else
+                set_error(g.out.err, NXB_DEVERR_HPLOC_INVALID_CLUSTER);
+            rows.put(j, b, id[q], base + j - me.start);
+            if (!Seg::kBatch && g.bvh8_pairs) g.bvh8_pairs[base + j] = bvh8_queue_slot(base + j, g.end);
+        }
+    }
+}
+
+// The climb inside the tile.  Each lane climbs from a leaf as in the
+// reference (FindParentId: a range hands over at the smaller of its two
+// bounding deltas; the second to arrive continues), with the hand-over slots
+// in shared memory: the value is the range's other end and its cluster
+// count.  A lane that stops takes the tile's next leaf.  A node of more than
+// 16 leaves is merged by the whole warp, and the warp goes on up the tree
+// while the sibling is there; the clusters stay in the rows at the range's
+// first positions, where the next merge finds them, so nothing in global
+// memory is waited for.  A range that arrives at a slot alone waits there:
+// its sibling reaches past the tile.
+template <int R, typename K, typename Seg>
+__device__ __forceinline__ void climb_tile(const Climb<K, Seg>& g, WarpTile<R>& t, uint32_t base, uint32_t cnt) {
+    const uint32_t lane = lane_id();
+    const Row rows = t.rows();
+    uint32_t range = 0;  // left | right << 16
+    uint32_t parts = 0;  // split | left clusters << 16 | right clusters << 24
+    uint32_t next = 0;
     bool active = false;
-    uint32_t chunk_next = 0, chunk_end = 0;  // warp-uniform
-    bool exhausted = false;                  // warp-uniform
-    bool release_due = false;                // warp-uniform: a pass merged, its release fence is pending
     for (;;) {
-        // refill stopped lanes with fresh leaves
-        uint32_t need = __ballot_sync(kFullMask, !active);
-        while (need && !exhausted) {
-            if (chunk_next == chunk_end) {
-                uint32_t b = 0;
-                if (lane == 0) b = begin + atomicAdd(leaf_ctr, chunk);
-                b = __shfl_sync(kFullMask, b, 0);
-                if (b >= end) {
-                    exhausted = true;
-                    break;
-                }
-                chunk_next = b;
-                chunk_end = min(b + chunk, end);
-            }
-            const uint32_t avail = chunk_end - chunk_next;
-            const uint32_t rank = __popc(need & lanemask_lt());
-            if (!active && ((need >> lane) & 1u) && rank < avail) {
-                left = right = chunk_next + rank;
+        const uint32_t need = __ballot_sync(kFullMask, !active);
+        if (next < cnt && need) {
+            const uint32_t mine = next + __popc(need & lanemask_lt());
+            if (!active && mine < cnt) {
+                range = mine | mine << 16;
+                parts = 1u << 16;
                 active = true;
-                if constexpr (Seg::kBatch) {
-                    me = seg.of_prim(left);
-                } else if (bvh8_pairs) {
-                    bvh8_pairs[left] = bvh8_queue_slot(left, end);
+            }
+            next += __popc(need);
+        }
+        if (!__any_sync(kFullMask, active)) break;
+        bool second = false, final = false;
+        if (active) {
+            uint32_t left = range & 0xFFFFu, right = range >> 16;
+            const uint64_t dl = t.gap[left], dr = t.gap[right + 1];
+            active = false;
+            if (dl != kEdge || dr != kEdge) {  // else a mesh's root
+                const bool go_right = dr < dl;
+                const uint32_t gp = go_right ? right + 1 : left;
+                const uint32_t have = (parts >> 16 & 0xFFu) + (parts >> 24);
+                const uint32_t prev = atomicExch(&t.hand[gp], (go_right ? left : right) | have << 16);
+                if (prev != kInvalid) {
+                    t.hand[gp] = kInvalid;
+                    const uint32_t sib = prev >> 16;
+                    if (go_right) {
+                        right = prev & 0xFFFFu;
+                        parts = gp | have << 16 | sib << 24;
+                    } else {
+                        left = prev & 0xFFFFu;
+                        parts = gp | sib << 16 | have << 24;
+                    }
+                    range = left | right << 16;
+                    active = second = true;
+                    final = t.gap[left] == kEdge && t.gap[right + 1] == kEdge;
                 }
             }
-            const uint32_t took = min((uint32_t)__popc(need), avail);
-            chunk_next += took;
-            need = __ballot_sync(kFullMask, !active);
         }
-        if (!__any_sync(kFullMask, active)) {
-            if (release_due) fence_acq_rel_gpu();
-            return;
+        uint32_t todo =
+            __ballot_sync(kFullMask, second && ((range >> 16) - (range & 0xFFFFu) >= kMergeThreshold || final));
+        while (todo) {
+            const uint32_t owner = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t lr = __shfl_sync(kFullMask, range, owner), ps = __shfl_sync(kFullMask, parts, owner);
+            uint32_t l = lr & 0xFFFFu, r = lr >> 16, mid = ps & 0xFFFFu, cl = ps >> 16 & 0xFFu, num = cl + (ps >> 24);
+            bool fin = t.gap[l] == kEdge && t.gap[r + 1] == kEdge;
+            const MeshSpan me = span_at(g.keys, g.seg, base + l);
+            const MergeCtx m{g.out, me.m, me.start, me.count};
+            uint32_t cid, ctok = 0;
+            Box cb;
+            for (;;) {
+                // both windows, side by side at the range's first positions
+                const Row row = rows.at(l);
+                cid = kInvalid;
+                __syncwarp();
+                if (lane < num) {
+                    const uint32_t k = lane < cl ? lane : mid - l + lane - cl;
+                    cb = row.box(k);
+                    const uint2 it = row.ids(k);
+                    cid = it.x;
+                    ctok = it.y;
+                }
+                __syncwarp();
+                if (mid - l != cl && lane >= cl && lane < num) row.put(lane, cb, cid, ctok);
+                __syncwarp();
+                num = merge_window<R>(m, num, fin, cid, ctok, cb, row);
+                // on up the tree while the sibling is there
+                const uint64_t dl = t.gap[l], dr = t.gap[r + 1];
+                if (dl == kEdge && dr == kEdge) break;
+                const bool go_right = dr < dl;
+                const uint32_t gp = go_right ? r + 1 : l;
+                const uint32_t prev = t.hand[gp];
+                if (prev == kInvalid) break;
+                __syncwarp();
+                if (lane == 0) t.hand[gp] = kInvalid;
+                mid = gp;
+                if (go_right) {
+                    r = prev & 0xFFFFu;
+                    cl = num;
+                } else {
+                    l = prev & 0xFFFFu;
+                    cl = prev >> 16;
+                }
+                num += prev >> 16;
+                fin = t.gap[l] == kEdge && t.gap[r + 1] == kEdge;
+            }
+            if (lane == owner) {
+                range = l | r << 16;
+                parts = num << 16;
+            }
         }
-        bool second = false;
-        bool go_right = false;
-        if (active)
+        __syncwarp();
+    }
+}
+
+// The subtrees left alone in a hand-over slot reach past the tile: lists
+// them (in t.gap) and stores their clusters; returns how many.
+template <int R, typename K, typename Seg>
+__device__ __forceinline__ uint32_t leave_tile(const Climb<K, Seg>& g, WarpTile<R>& t, uint32_t base, uint32_t cnt) {
+    const uint32_t lane = lane_id();
+    const Row rows = t.rows();
+    uint32_t leaving = 0;
+    __syncwarp();
+    for (uint32_t g0 = 0; g0 <= cnt; g0 += 32) {
+        const uint32_t gap = g0 + lane;
+        const uint32_t v = gap <= cnt ? t.hand[gap] : kInvalid;
+        const uint32_t mask = __ballot_sync(kFullMask, v != kInvalid);
+        if (v != kInvalid) {
+            const uint32_t other = v & 0xFFFFu;
+            const bool is_left = other < gap;  // the range ends at the gap, else it starts there
+            const uint32_t l = is_left ? other : gap, r = is_left ? gap - 1 : other;
+            t.gap[leaving + __popc(mask & lanemask_lt())] =
+                (uint64_t)(l | r << 16) | ((uint64_t)(v >> 16 | (is_left ? 0x100u : 0u)) << 32);
+        }
+        leaving += __popc(mask);
+    }
+    __syncwarp();
+    for (uint32_t i = lane >> 4; i < leaving; i += 2) {
+        const uint64_t e = t.gap[i];
+        const uint32_t l = (uint32_t)e & 0xFFFFu, size = (((uint32_t)e >> 16) & 0xFFFFu) - l + 1;
+        const uint32_t num = (uint32_t)(e >> 32) & 0xFFu, k = lane & 15u;
+        if (k < min(size, kMergeThreshold)) {
+            const uint2 it = rows.ids(l + k);
+            g.pub.template store<Seg>(base + l + k, rows.box(l + k), k < num ? it.x : kInvalid, it.y);
+        }
+    }
+    __syncwarp();
+    return leaving;
+}
+
+// The climb between tiles, for the `leaving` subtrees listed in t.gap: their
+// lanes hand over through slots in global memory (parent[g] for the gap
+// after position g; the value is the range's other end).  The exchanges are
+// relaxed; a pass that found siblings fences (acquire) after its exchanges,
+// before reading the siblings' clusters, and (release) before the next
+// pass's exchanges.  Nothing waits on another warp.
+template <int R, typename K, typename Seg>
+__device__ __forceinline__ void climb_between(const Climb<K, Seg>& g, WarpTile<R>& t, uint32_t base,
+                                              uint32_t leaving) {
+    const uint32_t lane = lane_id();
+    const Row row = t.rows();
+    uint32_t item = lane;
+    uint32_t left = 0, right = 0, split = 0;
+    bool active = false;
+    bool release_due = true;  // warp-uniform: stores since the last release fence
+    for (;;) {
+        bool fresh = false, go_right = false;
+        if (!active && item < leaving) {
+            const uint64_t e = t.gap[item];
+            item += 32;
+            left = base + ((uint32_t)e & 0xFFFFu);
+            right = base + (((uint32_t)e >> 16) & 0xFFFFu);
+            go_right = (e >> 40) & 1u;
+            active = fresh = true;
+        }
+        if (!__any_sync(kFullMask, active)) break;
+        MeshSpan me = Seg::kBatch ? MeshSpan{0, 0, 0} : g.seg.of_prim(0);
+        if (Seg::kBatch && active) me = span_at(g.keys, g.seg, left);
+        if (active && !fresh)
             go_right = left == me.start ||
                        (right != me.start + me.count - 1 &&
-                        delta(keys, right, right + 1, me.start) < delta(keys, left - 1, left, me.start));
+                        delta(g.keys, right, right + 1, me.start) < delta(g.keys, left - 1, left, me.start));
         if (release_due) {
-            // release: the previous pass's clusters and nodes before this
-            // pass's hand-overs (the store drain overlaps the refill and the
-            // key loads above)
+            // the clusters and nodes stored before this pass's hand-overs
+            // (the store drain overlaps the key loads)
+            __syncwarp();
             fence_acq_rel_gpu();
             release_due = false;
         }
+        bool second = false;
         if (active) {
             uint32_t prev;
             if (go_right) {
-                prev = atomicExch(parent + right, left);
+                prev = atomicExch(g.parent + right, left);
                 if (prev != kInvalid) {
                     split = right + 1;
                     right = prev;
                 }
             } else {
-                prev = atomicExch(parent + left - 1, right);
+                prev = atomicExch(g.parent + left - 1, right);
                 if (prev != kInvalid) {
                     split = left;
                     left = prev;
@@ -635,78 +757,123 @@ __global__ __launch_bounds__(kThreads, hploc_ctas_per_sm<R, Seg>()) void hploc_k
             second = prev != kInvalid;
             active = second;
         }
-        const uint32_t size = right - left + 1;
-        const bool final = second && size == me.count;
-        uint32_t todo = __ballot_sync(kFullMask, second && (size > kMergeThreshold || final));
-        if (todo) {
+        if (__any_sync(kFullMask, second)) {
             fence_acq_rel_gpu();  // acquire: the siblings' clusters
+            uint32_t todo = __ballot_sync(
+                kFullMask, second && (right - left >= kMergeThreshold || right - left + 1 == me.count));
             while (todo) {
                 const uint32_t owner = __ffs(todo) - 1;
-                ploc_merge<R, Seg>(owner, left, right, split, final, me, cluster, all, seg, row);
                 todo &= todo - 1;
+                if (merge_between<R>(g, owner, left, right, split, row) && lane == owner) active = false;
             }
-            __syncwarp();  // every lane's stores before the owners' next hand-overs
             release_due = true;
         }
+    }
+    __syncwarp();
+}
+
+// Persistent warps, each with a tile of its own in shared memory; nothing
+// waits on another warp.
+//
+// What bounds it: the ALU (62 % busy while active at 4.19M clustered
+// triangles; a round of neighbour search takes about 130 ALU instructions of
+// 240), the shared-memory pipe (59 %) and, for small or deep trees, the chain
+// of merges from a leaf to the root, one after another.  A climb through
+// global hand-over slots alone (a persistent grid whose warps take leaves)
+// costs two fences, an exchange and two dependent loads at every level; with
+// most levels inside a tile a merge takes 6 us of a warp instead of 9.
+// Measured against that form (H-PLOC, before -> now): 12.58M clustered
+// triangles 2.33 -> 2.12 ms, 4.19M sphere 0.576 -> 0.470, 3.0M at radius 16
+// 1.14 -> 0.95, 500,009 clustered boxes 0.38 -> 0.20, 65,536 soup triangles
+// 0.092 -> 0.071 ms.  A tile shared by the four warps of a CTA (512 leaves)
+// left 45 % of the warp time at its barrier (clustered trees are chains, with
+// about two merges ready at a time), and one-warp CTAs that are not
+// persistent start too slowly (one per 27 ns).
+template <typename K, int R, typename Seg>
+__global__ __launch_bounds__(32 * kTileWarps, kTileCtas) void hploc_kernel(Climb<K, Seg> g, uint32_t tiles, uint32_t* tile_ctr,
+                                                            uint32_t* bvh8_ctr) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    WarpTile<R>& t = reinterpret_cast<WarpTile<R>*>(smem)[threadIdx.x >> 5];
+    if (!Seg::kBatch && bvh8_ctr && blockIdx.x == 0 && threadIdx.x == 0) bvh8_queue_counters(bvh8_ctr);
+    // the first tile of each warp spreads small builds over the SMs
+    uint32_t tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    while (tile < tiles) {
+        const uint32_t base = g.begin + tile * g.tile, cnt = min(g.tile, g.end - base);
+        load_tile<R>(g, t, base, cnt);
+        __syncwarp();
+        climb_tile<R>(g, t, base, cnt);
+        const uint32_t leaving = leave_tile<R>(g, t, base, cnt);
+        if (leaving) climb_between<R>(g, t, base, leaving);
+        if (lane_id() == 0) tile = gridDim.x * (blockDim.x >> 5) + atomicAdd(tile_ctr, 1u);
+        tile = __shfl_sync(kFullMask, tile, 0);
     }
 }
 
 template <typename K, int R, typename Seg>
-cudaError_t launch_r(const K* keys, uint32_t* cluster, uint32_t* parent, Node2* nodes, Seg seg, uint32_t begin,
-                     uint32_t end, uint32_t* tok, uint32_t* pol, uint32_t* leaf_ctr, uint32_t* err,
-                     uint32_t max_per_sm, cudaStream_t s, Node2* rec, uint64_t* pairs, uint32_t* ctr,
-                     ChildPair* kids) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hploc_kernel<K, R, Seg>, kThreads, 0);
-    if (max_per_sm && (uint32_t)per_sm > max_per_sm) per_sm = (int)max_per_sm;
-    if (per_sm < 1) per_sm = 1;
-    const uint32_t want = (end - begin + kThreads - 1) / kThreads;
-    const uint32_t grid = std::max(1u, std::min(want, (uint32_t)(device_info().sms * per_sm)));
-    const uint32_t chunk = leaf_chunk(end - begin, grid * (kThreads / 32), Seg::kBatch);
-    hploc_kernel<K, R, Seg><<<grid, kThreads, 0, s>>>(keys, cluster, parent, nodes, seg, begin, tok, pol, leaf_ctr,
-                                                      err, end, chunk, rec, pairs, ctr, kids);
+cudaError_t launch_r(const Climb<K, Seg>& g, uint32_t* tile_ctr, uint32_t* bvh8_ctr, uint32_t max_per_sm,
+                     cudaStream_t s) {
+    constexpr size_t smem = sizeof(WarpTile<R>) * kTileWarps;
+    static_assert(kTileCtas * (smem + 1024) <= 228 * 1024, "shared memory of an SM");
+    const cudaError_t e = once_per_device([] {
+        cudaError_t r = cudaFuncSetAttribute(hploc_kernel<K, R, Seg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+        if (!r)
+            r = cudaFuncSetAttribute(hploc_kernel<K, R, Seg>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        return r;
+    });
+    if (e) return e;
+    const uint32_t sms = (uint32_t)device_info().sms;
+    const uint32_t tiles = (g.end - g.begin + g.tile - 1) / g.tile;
+    // resident warps per SM; the batch tuning's cap counts CTAs of four warps
+    uint32_t per_sm = std::min((tiles + sms - 1) / sms, (uint32_t)(kTileWarps * kTileCtas));
+    if (max_per_sm) per_sm = std::min(per_sm, 4 * max_per_sm);
+    const uint32_t ctas = (per_sm + kTileWarps - 1) / kTileWarps, warps = (per_sm + ctas - 1) / ctas;
+    hploc_kernel<K, R, Seg><<<std::min(tiles, sms * ctas), 32 * warps, sizeof(WarpTile<R>) * warps, s>>>(
+        g, tiles, tile_ctr, bvh8_ctr);
     return cudaGetLastError();
 }
 
 template <typename K, typename Seg>
 cudaError_t launch_t(const K* keys, uint32_t* cluster, uint32_t* parent, Node2* nodes, Seg seg, uint32_t begin,
-                     uint32_t end, uint32_t radius, uint32_t* tok, uint32_t* pol, uint32_t* leaf_ctr, uint32_t* err,
+                     uint32_t end, uint32_t radius, uint32_t* tok, uint32_t* pol, uint32_t* tile_ctr, uint32_t* err,
                      uint32_t max_per_sm, cudaStream_t s, Node2* rec = nullptr, uint64_t* pairs = nullptr,
                      uint32_t* ctr = nullptr, ChildPair* kids = nullptr) {
+    // one tile per resident warp while that is at most kTile leaves, so that
+    // small builds use every SM: 65,536 triangles take 71 us with 32 leaves
+    // per tile, 88 with 144; below 32 leaves (two windows) a tile has no merge
+    const uint32_t warps = (uint32_t)device_info().sms * kTileWarps * kTileCtas;
+    const uint32_t tile = std::max(32u, std::min((end - begin + warps - 1) / warps, (uint32_t)kTile));
+    const Climb<K, Seg> g{keys, cluster, parent, seg,  {nodes, kids, pol, err}, {rec, cluster, tok},
+                          begin, end,   tile,   pairs};
     switch (radius) {
-        case 4:
-            return launch_r<K, 4>(keys, cluster, parent, nodes, seg, begin, end, tok, pol, leaf_ctr, err, max_per_sm,
-                                  s, rec, pairs, ctr, kids);
-        case 16:
-            return launch_r<K, 16>(keys, cluster, parent, nodes, seg, begin, end, tok, pol, leaf_ctr, err,
-                                   max_per_sm, s, rec, pairs, ctr, kids);
-        default:
-            return launch_r<K, 8>(keys, cluster, parent, nodes, seg, begin, end, tok, pol, leaf_ctr, err, max_per_sm,
-                                  s, rec, pairs, ctr, kids);
+        case 4: return launch_r<K, 4, Seg>(g, tile_ctr, ctr, max_per_sm, s);
+        case 16: return launch_r<K, 16, Seg>(g, tile_ctr, ctr, max_per_sm, s);
+        default: return launch_r<K, 8, Seg>(g, tile_ctr, ctr, max_per_sm, s);
     }
 }
 
 }  // namespace
 
 cudaError_t launch_hploc(uint32_t key_bytes, const void* keys, uint32_t* cluster_idx, uint32_t* parent, Node2* nodes,
-                         uint32_t n, uint32_t radius, uint32_t* tokens, uint32_t* parent_of_last, uint32_t* leaf_ctr,
-                         uint32_t* err, cudaStream_t s, Node2* records, uint64_t* bvh8_pairs, uint32_t* bvh8_ctr,
+                         uint32_t n, uint32_t radius, uint32_t* parent_of_last, uint32_t* ctr, uint32_t* err,
+                         cudaStream_t s, Node2* records, uint64_t* bvh8_pairs, uint32_t* bvh8_ctr,
                          ChildPair* child_pairs) {
     const SingleMesh seg{n};
     if (!bvh8_pairs != !bvh8_ctr) return cudaErrorInvalidValue;
     if (key_bytes == 4)
-        return launch_t((const uint32_t*)keys, cluster_idx, parent, nodes, seg, 0u, n, radius, tokens,
-                        parent_of_last, leaf_ctr, err, 0u, s, records, bvh8_pairs, bvh8_ctr, child_pairs);
-    return launch_t((const uint64_t*)keys, cluster_idx, parent, nodes, seg, 0u, n, radius, tokens, parent_of_last,
-                    leaf_ctr, err, 0u, s, records, bvh8_pairs, bvh8_ctr, child_pairs);
+        return launch_t((const uint32_t*)keys, cluster_idx, parent, nodes, seg, 0u, n, radius, nullptr,
+                        parent_of_last, ctr, err, 0u, s, records, bvh8_pairs, bvh8_ctr,
+                        child_pairs);
+    return launch_t((const uint64_t*)keys, cluster_idx, parent, nodes, seg, 0u, n, radius, nullptr, parent_of_last,
+                    ctr, err, 0u, s, records, bvh8_pairs, bvh8_ctr, child_pairs);
 }
 
 cudaError_t launch_hploc_batch(const uint64_t* keys, uint32_t* cluster_idx, uint32_t* parent, Node2* nodes,
                                const MeshBatch& batch, uint32_t begin, uint32_t end, uint32_t radius,
-                               uint32_t* tokens, uint32_t* parent_of_last, uint32_t* leaf_ctr, uint32_t* err,
+                               uint32_t* tokens, uint32_t* parent_of_last, uint32_t* ctr, uint32_t* err,
                                uint32_t ctas_per_sm, cudaStream_t s, ChildPair* child_pairs) {
     return launch_t(reinterpret_cast<const MeshKey*>(keys), cluster_idx, parent, nodes, batch, begin, end, radius,
-                    tokens, parent_of_last, leaf_ctr, err, ctas_per_sm, s, nullptr, nullptr, nullptr, child_pairs);
+                    tokens, parent_of_last, ctr, err, ctas_per_sm, s, nullptr, nullptr, nullptr, child_pairs);
 }
 
 }  // namespace nxb

@@ -54,7 +54,7 @@ struct Control {
     uint32_t pad0[16];
     alignas(128) uint32_t bvh8_ctr[160];  // BVH8 counters, one per 128-byte line (kBvh8* below)
     uint32_t parent_of_last; // H-PLOC: the node whose child is node 2n-2 (seeded INVALID)
-    uint32_t hploc_leaf_ctr; // H-PLOC: next unclaimed leaf
+    uint32_t hploc_tile_ctr; // H-PLOC: next unclaimed tile
     uint32_t pad[2];
     uint32_t tile_ctr[kMaxSortPasses];
     // histograms: kMaxSortPasses x 256 words, or 4 passes x 512 words of the
@@ -172,11 +172,10 @@ cudaError_t launch_sort63_hybrid(const uint64_t* keys_in, const uint32_t* vals_i
                                  uint32_t* lookback, uint32_t* tile_ctr, uint32_t* overflow, uint32_t* fb_hist,
                                  uint32_t* fb_ticket, uint32_t* fb_done, uint32_t* err, cudaStream_t s);
 // ---------------------------------------------------------------- stage 4
-// tokens: n words of scratch (no initialisation needed); parent_of_last:
-// one word that must hold INVALID on entry; leaf_ctr: one word that must
-// be zero on entry.
-// records: n records of 32 bytes (no initialisation needed), where merges
-// store each window's clusters as {box, id, token}.
+// parent: n words holding INVALID on entry; parent_of_last: one word that
+// must hold INVALID on entry; tile_ctr: one word that must be zero on entry.
+// records: n records of 32 bytes (no initialisation needed), where subtrees
+// that leave their tile store their clusters as {box, id, token}.
 // bvh8_pairs / bvh8_ctr (both or neither): the BVH8 work queue of stage 5,
 // which the climb initialises as launch_bvh8_init would (each lane writes
 // the slot of the leaf it takes), so that the collapse can follow without
@@ -185,9 +184,9 @@ cudaError_t launch_sort63_hybrid(const uint64_t* keys_in, const uint32_t* vals_i
 // X - n receives the children of internal node X (boxes and indices), for
 // launch_bvh8 to read instead of the BVH2 nodes.
 cudaError_t launch_hploc(uint32_t key_bytes, const void* keys, uint32_t* cluster_idx, uint32_t* parent, Node2* nodes,
-                         uint32_t n, uint32_t radius, uint32_t* tokens, uint32_t* parent_of_last, uint32_t* leaf_ctr,
-                         uint32_t* err, cudaStream_t s, Node2* records, uint64_t* bvh8_pairs = nullptr,
-                         uint32_t* bvh8_ctr = nullptr, ChildPair* child_pairs = nullptr);
+                         uint32_t n, uint32_t radius, uint32_t* parent_of_last, uint32_t* tile_ctr, uint32_t* err,
+                         cudaStream_t s, Node2* records, uint64_t* bvh8_pairs = nullptr, uint32_t* bvh8_ctr = nullptr,
+                         ChildPair* child_pairs = nullptr);
 // ---------------------------------------------------------------- stage 5
 // pairs: n uint64 slots; ctr: kBvh8CtrWords words (128-byte aligned).
 // Both are initialised by launch_bvh8_init.
@@ -222,7 +221,7 @@ cudaError_t launch_batch_morton(const Node2* nodes, const MeshBatch& batch, uint
 // primitive of the batch; mesh m's internal node X gets record off[m] + X - n_m.
 cudaError_t launch_hploc_batch(const uint64_t* keys, uint32_t* cluster_idx, uint32_t* parent, Node2* nodes,
                                const MeshBatch& batch, uint32_t begin, uint32_t end, uint32_t radius,
-                               uint32_t* tokens, uint32_t* parent_of_last, uint32_t* leaf_ctr, uint32_t* err,
+                               uint32_t* tokens, uint32_t* parent_of_last, uint32_t* tile_ctr, uint32_t* err,
                                uint32_t ctas_per_sm, cudaStream_t s, ChildPair* child_pairs = nullptr);
 // Meshes cut into consecutive groups whose BVH8 collapses are separate
 // launches: group g holds meshes [mesh[g], mesh[g+1]), primitives
@@ -255,7 +254,7 @@ cudaError_t launch_batch_finalize(const MeshBatch& batch, const uint32_t* scene_
 struct BatchCtrl {
     uint32_t error_word;
     uint32_t pad[31];
-    uint32_t leaf_ctr[kMaxMeshGroups];  // one H-PLOC leaf counter per mesh group
+    uint32_t hploc_tile_ctr[kMaxMeshGroups];  // one H-PLOC tile counter per mesh group
     uint32_t pad2[32 - kMaxMeshGroups];
     uint32_t tile_ctr[kMaxSortPasses];
     uint32_t hist[kMaxSortPasses][kRadixBins];
