@@ -587,6 +587,392 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
     }
 }
 
+// ---------------------------------------------------------------- groups
+// The same collapse with eight lanes per work item: lane c of a group holds
+// child c while the node is opened, and slot c when slots are assigned,
+// quantised and written.  What bounds it is the chain of levels: per level
+// 2.3 us of dependent record loads (up to seven), 0.6 us of assignment (0.8
+// in one lane), 0.3 us each for the poll and the allocation; the 2 us that
+// one lane takes to quantise and write a node are 0.15.
+constexpr uint32_t kGroupsPerCta = kThreads / 8;
+
+// Monotone key of a cost for comparing as uint32; 0 for one that the
+// sequential search would never take (not above -FLT_MAX, or NaN).  -0 and
+// +0 compare equal, so both get +0's key.
+__device__ __forceinline__ uint32_t cost_key(float cost) {
+    const uint32_t u = __float_as_uint(cost);
+    return cost > -3.402823466e+38f ? f2ord(u == 0x80000000u ? 0.0f : cost) : 0u;
+}
+
+// The first lane of the group with the largest key (a slot index), or 0xF.
+__device__ __forceinline__ uint32_t group_first(uint32_t key, uint32_t best, uint32_t base) {
+    const uint32_t m = __ballot_sync(kFullMask, key == best) >> base & 0xFFu;
+    return best ? (uint32_t)__ffs(m) - 1u : 0xFu;
+}
+
+// greedy_assign over a group: lane s returns the child of slot s (0xF: none).
+// Every lane rates the slots for its own child; then the children choose in
+// order, lane c telling the others its first best slot among those left.
+__device__ __forceinline__ uint32_t group_greedy(float3 off, uint32_t count, uint32_t sub) {
+    uint32_t key[8];
+#pragma unroll
+    for (uint32_t s = 0; s < 8; ++s) key[s] = cost_key(slot_cost(s, off));
+    uint32_t mine = 0xFu, taken = 0;
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c) {
+        uint32_t k[8], at[8];
+#pragma unroll
+        for (uint32_t s = 0; s < 8; ++s) {
+            k[s] = (taken >> s) & 1u ? 0u : key[s];
+            at[s] = s;
+        }
+#pragma unroll
+        for (uint32_t w = 1; w < 8; w *= 2)
+#pragma unroll
+            for (uint32_t s = 0; s < 8; s += 2 * w) {
+                const bool t = k[s + w] > k[s];
+                k[s] = t ? k[s + w] : k[s];
+                at[s] = t ? at[s + w] : at[s];
+            }
+        const uint32_t slot = __shfl_sync(kFullMask, k[0] ? at[0] : 0xFu, c, 8);
+        if (c < count && slot < 8) {
+            taken |= 1u << slot;
+            if (sub == slot) mine = c;
+        }
+    }
+    return mine;
+}
+
+// auction_assign over a group; kFallback in every lane where the sequential
+// form falls back.
+__device__ __forceinline__ uint32_t group_auction(const Box& pb, const Box& cb, uint32_t count, bool run, uint32_t sub,
+                                                  uint32_t base) {
+    const float max_dim = fmaxf(pb.mx.x - pb.mn.x, fmaxf(pb.mx.y - pb.mn.y, pb.mx.z - pb.mn.z));
+    float cost_scale = max_dim == 0.0f ? 0.0f : 10.0f / max_dim;
+    cost_scale *= 0.5f;
+    const float3 pc = make_float3(pb.mn.x + pb.mx.x, pb.mn.y + pb.mx.y, pb.mn.z + pb.mx.z);
+    const float3 off = make_float3((pc.x - (cb.mn.x + cb.mx.x)) * cost_scale, (pc.y - (cb.mn.y + cb.mx.y)) * cost_scale,
+                                   (pc.z - (cb.mn.z + cb.mx.z)) * cost_scale);
+    float max_cost = sub < count ? fmaxf(-3.402823466e+38f, fabsf(off.x) + fabsf(off.y) + fabsf(off.z))
+                                 : -3.402823466e+38f;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) max_cost = fmaxf(max_cost, __shfl_xor_sync(kFullMask, max_cost, o));
+    const float threshold = 1.0f / (float)count;
+    float epsilon = fmaxf(max_cost, threshold);
+    float price = 0.0f;
+    uint32_t mine = 0xFu, bids = 0, bidders = 0x76543210u, waiting = count;
+    run = run && epsilon >= threshold;
+    while (__any_sync(kFullMask, run)) {
+        // one bid per group
+        const uint32_t c = nib(bidders, (waiting - 1u) & 7u) & 7u;
+        const float3 o = make_float3(__shfl_sync(kFullMask, off.x, c, 8), __shfl_sync(kFullMask, off.y, c, 8),
+                                     __shfl_sync(kFullMask, off.z, c, 8));
+        const uint32_t key = cost_key(slot_cost(sub, o) - price);
+        uint32_t first = key, second = 0;
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) {
+            const uint32_t f = __shfl_xor_sync(kFullMask, first, d), g = __shfl_xor_sync(kFullMask, second, d);
+            second = max(min(first, f), max(second, g));
+            first = max(first, f);
+        }
+        const uint32_t slot = group_first(key, first, base);
+        const uint32_t prev = __shfl_sync(kFullMask, mine, slot, 8);
+        if (run) {
+            if (slot > 7 || ++bids > kAuctionBidLimit) {
+                mine = kFallback;
+                run = false;
+            } else {
+                --waiting;
+                if (sub == slot) {
+                    price += (ord2f(first) - (second ? ord2f(second) : -3.402823466e+38f)) + epsilon;
+                    mine = c;
+                }
+                if (prev != 0xFu) {
+                    bidders = (bidders & ~(0xFu << (4 * waiting))) | (prev << (4 * waiting));
+                    ++waiting;
+                }
+                if (waiting == 0) {
+                    epsilon *= 0.125f;
+                    run = epsilon >= threshold;
+                    if (run) {
+                        mine = 0xFu;
+                        bidders = 0x76543210u;
+                        waiting = count;
+                    }
+                }
+            }
+        }
+    }
+    return mine;
+}
+
+template <typename Seg, bool AUCTION>
+__global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __restrict__ b2, Seg seg, Node8* out,
+                                                              uint32_t cap, uint32_t slots, uint32_t* prim_idx,
+                                                              uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
+                                                              uint32_t* mesh_leaves, uint32_t* err,
+                                                              const ChildPair* __restrict__ kids) {
+    __shared__ __align__(8) uint8_t s_rows[kGroupsPerCta][64];  // meta and quantised bytes of a group's node
+    const uint32_t lane = lane_id(), sub = lane & 7u, base = lane & 24u;
+    uint8_t* rows = s_rows[threadIdx.x >> 3];
+    if constexpr (!Seg::kBatch) {
+        if (seg.n == 1) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                write_node8(out, load_box(b2, 0), LeafZero{b2}, 0, 0, 0xFFFFFFF0u, 0u, 1u);
+                prim_idx[0] = 0;
+                ctr[kBvh8Leaves] = 1;
+                ctr[kBvh8Pending] = 0;
+            }
+            return;
+        }
+    }
+    uint32_t slot = kInvalid;
+    bool retired = false;
+    uint32_t idle = 0;
+    for (;;) {
+        // groups without a slot claim the next ones (see bvh8_kernel)
+        const bool want = !retired && slot == kInvalid;
+        const uint32_t wmask = __ballot_sync(kFullMask, want && sub == 0);
+        if (wmask) {
+            uint32_t first = 0;
+            if (lane == 0) first = atomicAdd(ctr + kBvh8Claim, (uint32_t)__popc(wmask));
+            first = __shfl_sync(kFullMask, first, 0);
+            if (want) {
+                const uint32_t claimed = first + __popc(wmask & ((1u << base) - 1u));
+                if (claimed < slots && claimed >= first)
+                    slot = claimed;
+                else
+                    retired = true;
+            }
+        }
+        if (__all_sync(kFullMask, retired)) return;
+        uint64_t pr = ~0ull;
+        if (slot != kInvalid) pr = ld_relaxed_u64(pairs + slot);
+        pr = __shfl_sync(kFullMask, pr, 0, 8);  // one lane's view for the whole group
+        const bool ready = (uint32_t)(pr >> 32) != kInvalid;
+        if (!__any_sync(kFullMask, ready)) {
+            if (ld_relaxed_u32(ctr + kBvh8Pending) == 0) return;
+            if (++idle > kQueueSpinLimit) {
+                if (lane == 0) set_error(err, NXB_DEVERR_BVH8_QUEUE_TIMEOUT);
+                return;
+            }
+            __nanosleep(min(32u << min(idle, 5u), 128u));
+            continue;
+        }
+        idle = 0;
+        const uint32_t b2i = (uint32_t)(pr >> 32), b8i = (uint32_t)pr;
+        MeshSpan me{0, 0, 0};
+        const Node2* mb2 = b2;
+        uint32_t base8 = 0, cap8 = cap;
+        bool internal = false;
+        ChildPair kp;
+        if (ready) {
+            if constexpr (Seg::kBatch) {
+                me = seg.span(owner_of(seg.off8, 0, seg.meshes - 1, b8i));
+                mb2 = b2 + 2ull * me.start;
+                base8 = __ldg(seg.off8 + me.m);
+                cap8 = __ldg(seg.off8 + me.m + 1) - base8;
+            } else {
+                me.count = seg.n;
+            }
+            if (Seg::kBatch && me.count <= 1) {
+                if (me.count == 1 && sub == 0) {
+                    write_node8(out + b8i, load_box(mb2, 0), LeafZero{mb2}, 0, 0, 0xFFFFFFF0u, 0u, 1u);
+                    prim_idx[me.start] = 0;
+                    mesh_leaves[me.m] = 1;
+                }
+            } else if (b2i >= 2 * me.count - 1 || b8i - base8 >= cap8 || b2i < me.count) {
+                if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
+            } else {
+                kp = load_child_pair(kids + me.start + (b2i - me.count));
+                if (kp.li >= 2 * me.count - 1 || kp.ri >= 2 * me.count - 1) {
+                    if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
+                } else {
+                    internal = true;
+                }
+            }
+            if (!internal) slot = kInvalid;  // done (or reported); the item counts as finished
+        }
+        const uint32_t node_limit = 2 * me.count - 1;
+        Box nb, cb;  // the node's box, this lane's child's box
+        nb.mn = nb.mx = cb.mn = cb.mx = make_float3(0.f, 0.f, 0.f);
+        uint32_t idx = 0, inner = 0, count = 0, msb = 0;
+        if (internal) {
+            nb = kp.l;
+            grow(nb, kp.r);
+        }
+        // open BVH2 nodes top-down until 8 children or no inner child; every
+        // lane of the group has the record, the two lanes concerned keep a child
+        bool open = internal;
+        while (__any_sync(kFullMask, open)) {
+            if (open) {
+                const bool in0 = kp.li >= me.count, in1 = kp.ri >= me.count;
+                const bool first = !(half_area(kp.l) < half_area(kp.r));
+                // the smaller-area child takes the re-opened position
+                const bool low = sub == msb, high = sub == count + 1;
+                if (low || high) {
+                    const bool right = low == first;
+                    cb = right ? kp.r : kp.l;
+                    idx = right ? kp.ri : kp.li;
+                    if (idx >= me.count) prefetch_l2(kids + me.start + (idx - me.count));
+                }
+                if (first ? in1 : in0) inner |= 1u << msb;
+                if (first ? in0 : in1) inner |= 1u << (count + 1);
+                count += 2;
+                if (inner == 0 || count == 8) {
+                    open = false;
+                } else {
+                    msb = 31 - __clz(inner);
+                    inner &= ~(1u << msb);
+                    count--;
+                }
+            }
+            const uint32_t next = __shfl_sync(kFullMask, idx, msb, 8);
+            if (open) {
+                kp = load_child_pair(kids + me.start + (next - me.count));
+                if (kp.li >= node_limit || kp.ri >= node_limit) {  // corrupt BVH2: report, stop expanding
+                    if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
+                    inner |= 1u << msb;
+                    count++;
+                    open = false;
+                }
+            }
+        }
+        const float3 pc = make_float3(nb.mn.x + nb.mx.x, nb.mn.y + nb.mx.y, nb.mn.z + nb.mx.z);
+        const float3 off = make_float3(pc.x - (cb.mx.x + cb.mn.x), pc.y - (cb.mx.y + cb.mn.y),
+                                       pc.z - (cb.mx.z + cb.mn.z));
+        uint32_t mine;  // the child of slot `sub`
+        if constexpr (AUCTION) {
+            mine = group_auction(nb, cb, max(count, 1u), internal, sub, base);
+            const bool failed = mine == kFallback;
+            if (__any_sync(kFullMask, failed)) {
+                const uint32_t g = group_greedy(off, count, sub);
+                if (failed) mine = g;
+            }
+        } else {
+            mine = group_greedy(off, count, sub);
+        }
+        const bool used = internal && mine != 0xFu;
+        const bool is_inner = used && ((inner >> mine) & 1u);
+        const uint32_t imask = __ballot_sync(kFullMask, is_inner) >> base & 0xFFu;
+        const uint32_t lmask = __ballot_sync(kFullMask, used && !is_inner) >> base & 0xFFu;
+        const uint32_t child = __shfl_sync(kFullMask, idx, mine, 8);
+        Box qb;
+        qb.mn.x = __shfl_sync(kFullMask, cb.mn.x, mine, 8);
+        qb.mn.y = __shfl_sync(kFullMask, cb.mn.y, mine, 8);
+        qb.mn.z = __shfl_sync(kFullMask, cb.mn.z, mine, 8);
+        qb.mx.x = __shfl_sync(kFullMask, cb.mx.x, mine, 8);
+        qb.mx.y = __shfl_sync(kFullMask, cb.mx.y, mine, 8);
+        qb.mx.z = __shfl_sync(kFullMask, cb.mx.z, mine, 8);
+        // allocation of work slots (one mesh: = BVH8 nodes) and leaves, one
+        // atomic for the warp's four groups
+        const uint32_t ic = internal ? (uint32_t)__popc(imask) : 0u;
+        const uint32_t lc = internal ? count - (uint32_t)__popc(imask) : 0u;
+        const uint32_t packed = ic | (lc << 16);
+        uint32_t excl = 0, total = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            const uint32_t v = __shfl_sync(kFullMask, packed, 8 * q);
+            if (8 * q < base) excl += v;
+            total += v;
+        }
+        const uint32_t done = __popc(__ballot_sync(kFullMask, ready && sub == 0));
+        const uint32_t new_items = total & 0xFFFFu;
+        const uint64_t tl = Seg::kBatch ? 0u : total >> 16;
+        uint64_t bases = 0;
+        if (lane == 0 && (tl | new_items))
+            bases = atomicAdd(reinterpret_cast<unsigned long long*>(ctr + kBvh8Alloc),
+                              (unsigned long long)((tl << 32) | new_items));
+        uint32_t child_base = 0, prim_base = 0;
+        if (Seg::kBatch && internal && sub == 0) {
+            child_base = ic ? atomicAdd(mesh_nodes + me.m, ic) : 0u;
+            prim_base = lc ? atomicAdd(mesh_leaves + me.m, lc) : 0u;
+        }
+        bases = __shfl_sync(kFullMask, bases, 0);
+        const uint32_t work_base = (uint32_t)bases + (excl & 0xFFFFu);
+        if constexpr (Seg::kBatch) {
+            child_base = __shfl_sync(kFullMask, child_base, 0, 8);
+            prim_base = __shfl_sync(kFullMask, prim_base, 0, 8);
+        } else {
+            child_base = work_base;
+            prim_base = lc ? (uint32_t)(bases >> 32) + (excl >> 16) : 0u;
+        }
+        bool write = internal;
+        if (write && (child_base + ic > cap8 || work_base + ic > slots || prim_base + lc > me.count)) {
+            if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
+            write = false;
+        }
+        if (write) {
+            if (is_inner) {
+                const uint32_t k = popc_below(imask, sub);
+                st_relaxed_u64(pairs + work_base + k, ((uint64_t)child << 32) | (base8 + child_base + k));
+            } else if (used) {
+                prim_idx[me.start + prim_base + popc_below(lmask, sub)] = child;  // leaf i is primitive i
+            }
+        }
+        if (internal) slot = kInvalid;
+        // pending += items allocated - items finished (see bvh8_kernel)
+        __syncwarp();
+        if (lane == 0 && new_items != done) atomicAdd(ctr + kBvh8Pending, new_items - done);
+        // the node: lane s quantises slot s (write_node8)
+        if (__any_sync(kFullMask, write)) {
+            const uint8_t ex = (uint8_t)ceil_log2_biased((nb.mx.x - nb.mn.x) * kQuantStep);
+            const uint8_t ey = (uint8_t)ceil_log2_biased((nb.mx.y - nb.mn.y) * kQuantStep);
+            const uint8_t ez = (uint8_t)ceil_log2_biased((nb.mx.z - nb.mn.z) * kQuantStep);
+            const float3 inv = make_float3(inv_pow2(ex), inv_pow2(ey), inv_pow2(ez));
+            rows[sub] = (uint8_t)(!used ? 0u : is_inner ? 0x20u | (24u + sub) : 0x20u | popc_below(lmask, sub));
+            rows[8 + sub] = used ? (uint8_t)floorf((qb.mn.x - nb.mn.x) * inv.x) : (uint8_t)0;
+            rows[16 + sub] = used ? (uint8_t)floorf((qb.mn.y - nb.mn.y) * inv.y) : (uint8_t)0;
+            rows[24 + sub] = used ? (uint8_t)floorf((qb.mn.z - nb.mn.z) * inv.z) : (uint8_t)0;
+            rows[32 + sub] = used ? (uint8_t)ceilf((qb.mx.x - nb.mn.x) * inv.x) : (uint8_t)0;
+            rows[40 + sub] = used ? (uint8_t)ceilf((qb.mx.y - nb.mn.y) * inv.y) : (uint8_t)0;
+            rows[48 + sub] = used ? (uint8_t)ceilf((qb.mx.z - nb.mn.z) * inv.z) : (uint8_t)0;
+            __syncwarp();
+            if (write) {
+                uint2* d = reinterpret_cast<uint2*>(out + b8i);
+                if (sub == 0) d[0] = make_uint2(__float_as_uint(nb.mn.x), __float_as_uint(nb.mn.y));
+                if (sub == 1)
+                    d[1] = make_uint2(__float_as_uint(nb.mn.z), (uint32_t)ex | ((uint32_t)ey << 8) |
+                                                                   ((uint32_t)ez << 16) | (imask << 24));
+                if (sub == 2) d[2] = make_uint2(child_base, prim_base);
+                if (sub < 7) d[3 + sub] = reinterpret_cast<const uint2*>(rows)[sub];
+            }
+            __syncwarp();
+        }
+    }
+}
+
+template <typename Seg, bool AUCTION>
+cudaError_t launch_group(const Node2* bvh2, Seg seg, uint32_t items, Node8* out, uint32_t cap, uint32_t slots,
+                         uint32_t* prim_idx, uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
+                         uint32_t* mesh_leaves, uint32_t* err, cudaStream_t s, const ChildPair* kids) {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bvh8_group_kernel<Seg, AUCTION>, kThreads, 0);
+    // Groups that wait poll the pending counter, and too many of them saturate
+    // its L2 line: 65,536 triangles take 104 us with a group per item, 70 with
+    // one per 16 primitives; 256,000 take 117 us at 8 CTAs per SM, 96 at 4.
+    // Auctions keep their groups busy: 1.05M triangles 631 us at 4, 512 at 8.
+    if (!AUCTION) per_sm = std::min(per_sm, 4);
+    if (per_sm < 1) per_sm = 1;
+    const uint32_t want = (items + 16 * kGroupsPerCta - 1) / (16 * kGroupsPerCta);
+    const uint32_t grid = std::max(1u, std::min(want, (uint32_t)(device_info().sms * per_sm)));
+    bvh8_group_kernel<Seg, AUCTION><<<grid, kThreads, 0, s>>>(bvh2, seg, out, cap, slots, prim_idx, pairs, ctr,
+                                                              mesh_nodes, mesh_leaves, err, kids);
+    return cudaGetLastError();
+}
+
+// Which form of the collapse a build with child-pair records takes.  Small
+// greedy collapses are a chain of levels (12 at 65,536 triangles), where a
+// group gets an item done sooner and no item waits for the other 31 of its
+// warp; large ones are bound by random memory traffic, where one lane per
+// item keeps eight times the items in flight.  Measured (one lane / a group
+// per item): 16,411 clustered boxes 98 / 76 us, 65,536 soup triangles
+// 100 / 70, 256,000 129 / 96, 512,000 143 / 129, 1.0M 170 / 184, 4.19M sphere
+// 254 / 473.  An auction is a long sequential search per item, eight times
+// shorter in a group: 1.05M sphere 1042 / 512 us.
+constexpr uint32_t kGroupMaxPrims = 600000;
+inline bool takes_groups(uint32_t prims, bool auction) { return auction || prims <= kGroupMaxPrims; }
+
 template <typename Seg, bool AUCTION, bool KIDS>
 cudaError_t configure_smem() {
     return once_per_device([] {
@@ -657,13 +1043,16 @@ cudaError_t launch_bvh8_init(uint64_t* pairs, uint32_t n, uint32_t* ctr, cudaStr
 cudaError_t launch_bvh8(const Node2* bvh2, uint32_t n, Node8* out, uint32_t cap, uint32_t* prim_idx, uint64_t* pairs,
                         uint32_t* ctr, uint32_t* err, bool auction, cudaStream_t s, const ChildPair* child_pairs) {
     const SingleMesh seg{n};
-    if (child_pairs) {
+    if (child_pairs && takes_groups(n, auction)) {
         if (auction)
-            return launch_wide<SingleMesh, true, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr,
-                                                       nullptr, err, s, child_pairs);
+            return launch_group<SingleMesh, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr,
+                                                  err, s, child_pairs);
+        return launch_group<SingleMesh, false>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr, err,
+                                               s, child_pairs);
+    }
+    if (child_pairs)
         return launch_wide<SingleMesh, false, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr,
                                                     nullptr, err, s, child_pairs);
-    }
     if (auction)
         return launch_wide<SingleMesh, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr, err,
                                              s);
@@ -682,13 +1071,16 @@ cudaError_t launch_bvh8_batch(const Node2* bvh2, const MeshBatch& batch, uint32_
                               uint32_t* prim_idx, uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
                               uint32_t* mesh_leaves, uint32_t* err, bool auction, cudaStream_t s,
                               const ChildPair* child_pairs) {
-    if (child_pairs) {
+    if (child_pairs && takes_groups(total, auction)) {
         if (auction)
-            return launch_wide<MeshBatch, true, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr,
-                                                      mesh_nodes, mesh_leaves, err, s, child_pairs);
+            return launch_group<MeshBatch, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
+                                                 mesh_leaves, err, s, child_pairs);
+        return launch_group<MeshBatch, false>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
+                                              mesh_leaves, err, s, child_pairs);
+    }
+    if (child_pairs)
         return launch_wide<MeshBatch, false, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr,
                                                    mesh_nodes, mesh_leaves, err, s, child_pairs);
-    }
     if (auction)
         return launch_wide<MeshBatch, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
                                             mesh_leaves, err, s);
