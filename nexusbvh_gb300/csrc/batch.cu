@@ -94,6 +94,7 @@ bool batch_layout(const uint32_t* h_off, uint32_t meshes, uint32_t* h_off8, Batc
     uint64_t acc = 0;
     for (uint32_t m = 0; m < meshes; ++m) {
         h_off8[m] = (uint32_t)acc;
+        a->max_mesh = std::max(a->max_mesh, h_off[m + 1] - h_off[m]);
         acc += batch_bvh8_capacity(h_off[m + 1] - h_off[m]);
         if (acc > 0xFFFFFFF0ull) return false;
     }
@@ -159,7 +160,8 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
     one.slot[1] = a.slots;
     const MeshGroups& g = (groups && fork && groups->count > 1) ? *groups : one;
     const MeshBatch mb{a.off, a.off8, a.meshes};
-    const SortPlan plan = make_sort_plan(2, 32 + a.mesh_bits, t.digit_bits);
+    const bool local = local_sort_takes(a.max_mesh);
+    const SortPlan plan = local ? SortPlan{} : make_sort_plan(2, 32 + a.mesh_bits, t.digit_bits);
     NXB_TRY(cudaMemsetAsync(a.zero_begin, 0, a.zero_bytes, s));
     if (a.total > 0) {
         NXB_TRY(launch_batch_tile_ranges(mb, a.total, t.block, a.tile_rng, s));
@@ -171,6 +173,7 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
         f.ones_words = a.ones_words;
         NXB_TRY(launch_batch_morton(a.bvh2, mb, a.total, a.scene_ord, a.keys_a, a.vals_a, plan, &a.ctrl->hist[0][0],
                                     f, t.block, a.tile_rng, s));
+        if (local) NXB_TRY(launch_local_sort_batch(a.keys_a, a.vals_a, mb, a.max_mesh, s));
         for (int p = 0; p < plan.passes; ++p) {
             const bool even = (p % 2) == 0;
             NXB_TRY(launch_sort_pass(8, even ? a.keys_a : a.keys_b, even ? a.keys_b : a.keys_a,

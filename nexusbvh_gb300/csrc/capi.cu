@@ -170,17 +170,20 @@ nxb_status enqueue_build(const void* prims, nxb_prim_type type, uint32_t n, cons
     NXB_TRY(mark(0));
     NXB_TRY(launch_scene_bounds(prims, type, n, bvh2, ctrl->scene_ord, s));
     NXB_TRY(mark(1));
+    const bool local = local_sort_takes(n);
     MortonFused f{};
-    f.plan = &L.plan;
+    f.plan = local ? nullptr : &L.plan;
     f.cluster_idx = nullptr;  // the first sort pass generates the values
     f.parent = parent;
     f.zero_ptr = lookback;
-    f.zero_words = align_up(4ull * L.tiles_words) / 4;  // both plans: the top passes' words, all of them
+    f.zero_words = local ? 0 : align_up(4ull * L.tiles_words) / 4;  // both plans: the top passes' words, all of them
     f.scene_out = nullptr;
     f.seed_counters = true;
     NXB_TRY(launch_morton(bvh2, n, ctrl, (int)key_bits, keys_a, f, s));
     NXB_TRY(mark(2));
-    if (key_bits == 30) {
+    if (local) {
+        NXB_TRY(launch_local_sort(L.key_bytes, keys_a, vals_a, n, s));
+    } else if (key_bits == 30) {
         const size_t tiles_per_pass = L.tiles_words / L.plan.passes;
         for (int p = 0; p < L.plan.passes; ++p) {
             const bool even = (p % 2) == 0;

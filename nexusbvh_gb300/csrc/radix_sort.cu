@@ -16,6 +16,7 @@
 //     runs of consecutive addresses.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "pipeline.h"
 
@@ -789,6 +790,302 @@ __global__ __launch_bounds__(kThreads, 4) void sort_fallback_kernel(K* ka, K* kb
     }
 }
 
+// ---------------------------------------------------------------- cluster sort
+// Small sorts as one launch: a mesh's keys live in the shared memory of a
+// thread-block cluster (2^k keys per CTA, up to 16 CTAs) from the first pass
+// to the last.  Per pass each CTA ranks its keys (per-warp histograms by
+// ballots, as in sort_tile), publishes its digit counts in shared memory,
+// reads the other CTAs' counts, and stores its keys, in digit order, into the
+// CTAs that own their next positions; two cluster barriers per pass take the
+// place of a launch, a look-back and a trip through global memory.
+//
+// What bounds it: the chain of steps of a pass (2 us in one CTA, 6 to 8 in a
+// cluster), not bandwidth.  The sort stage on GB300, onesweep passes -> this:
+// 1,021 30-bit keys 35.5 -> 9.9 us, 32,000 44 -> 24, 65,536 47.7 -> 32.4;
+// 16,411 63-bit keys 60 -> 45.  Stores to peers straight from the ranking
+// order, without sorting the CTA's keys by digit first, took 46.7 us at
+// 65,536 keys: one request per lane instead of runs.
+constexpr int kLocalThreads = 512;
+constexpr int kLocalWarps = kLocalThreads / 32;
+constexpr uint32_t kLocalMaxCtas = 16;
+constexpr int kLocalMaxKpt = 8;
+constexpr uint32_t kLocalMaxKeys = kLocalMaxCtas * kLocalThreads * kLocalMaxKpt;  // 65,536
+
+template <typename K, int RB, int KPT>
+struct __align__(16) LocalSmem {
+    static constexpr int kTile = kLocalThreads * KPT, kBins = 1 << RB;
+    K key[kTile];
+    K out_key[kTile];  // a pass's keys in digit order, on their way to other CTAs
+    uint32_t val[kTile];
+    uint32_t out_val[kTile];
+    uint16_t wh[kLocalWarps][kBins];  // per-warp digit counts, then offsets
+    uint32_t cnt[kBins];              // this CTA's digit counts, read by the cluster
+    uint32_t base[kBins];             // first position of this CTA's keys of a digit
+    uint32_t tmp[kLocalWarps];
+};
+
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// The address of this CTA's shared variable p in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(a)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ uint32_t ld_peer(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_peer(uint32_t a, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_peer(uint32_t a, uint64_t v) {
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+
+// Sorts `count` keys, loaded by the caller into key/val of the cluster's
+// CTAs in order, stably on `passes` digits of RB bits from bit `shift` on.
+// ctas: CTAs of the cluster (uniform); me: this CTA's rank in it.
+template <typename K, int RB, int KPT>
+__device__ __forceinline__ void local_sort(LocalSmem<K, RB, KPT>& sm, uint32_t count, uint32_t shift, int passes,
+                                           uint32_t ctas, uint32_t me) {
+    using S = LocalSmem<K, RB, KPT>;
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const uint32_t first = me * S::kTile;
+    const uint32_t own = warp * 32u * KPT + lane;
+    uint16_t* wh = sm.wh[warp];
+    const uint32_t lt_mask = lanemask_lt();
+    for (int p = 0; p < passes; ++p, shift += RB) {
+        for (uint32_t i = lane; i < S::kBins / 2; i += 32) reinterpret_cast<uint32_t*>(wh)[i] = 0;
+        K key[KPT];
+        uint32_t val[KPT], rank[KPT];
+#pragma unroll
+        for (int j = 0; j < KPT; ++j) {
+            key[j] = sm.key[own + 32 * j];
+            val[j] = sm.val[own + 32 * j];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < KPT; ++j) {
+            const bool valid = first + own + 32 * j < count;
+            const uint32_t d = (uint32_t)(key[j] >> shift) & (S::kBins - 1u);
+            uint32_t peers = __ballot_sync(kFullMask, valid);
+#pragma unroll
+            for (int b = 0; b < RB; ++b) {
+                const bool bit = (d >> b) & 1u;
+                const uint32_t bb = __ballot_sync(kFullMask, bit);
+                peers &= bit ? bb : ~bb;
+            }
+            const uint32_t below = __popc(peers & lt_mask);
+            const uint32_t leader = (uint32_t)(__ffs(peers) - 1) & 31u;
+            uint32_t at = 0;
+            if (valid && below == 0) {
+                at = wh[d];
+                wh[d] = (uint16_t)(at + __popc(peers));
+            }
+            rank[j] = __shfl_sync(kFullMask, at, leader) + below;
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t x[kLocalWarps], mine = 0, total = 0, before = 0;
+        if (tid < S::kBins) {
+#pragma unroll
+            for (int w = 0; w < kLocalWarps; ++w) {
+                x[w] = sm.wh[w][tid];
+                mine += x[w];
+            }
+            sm.cnt[tid] = mine;
+            total = mine;
+        }
+        if (ctas > 1) {
+            cluster_sync();  // every CTA's counts; and all its keys are in registers
+            if (tid < S::kBins) {
+                total = 0;
+#pragma unroll 4
+                for (uint32_t r = 0; r < ctas; ++r) {
+                    const uint32_t v = ld_peer(peer_addr(&sm.cnt[tid], r));
+                    before += r < me ? v : 0u;
+                    total += v;
+                }
+            }
+        }
+        // exclusive scans of the cluster's and of this CTA's digit counts
+        // (up to 2^16 and 2^12) in one word
+        const uint32_t both = total << 13 | mine;
+        uint32_t incl = both;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        if (lane == 31) sm.tmp[warp] = incl;
+        __syncthreads();
+        if (tid < S::kBins) {
+            uint32_t pre = incl - both;
+            for (uint32_t w = 0; w < warp; ++w) pre += sm.tmp[w];
+            uint32_t at = pre & 0x1FFFu;
+            sm.base[tid] = (pre >> 13) + before - at;
+#pragma unroll
+            for (int w = 0; w < kLocalWarps; ++w) {
+                sm.wh[w][tid] = (uint16_t)at;
+                at += x[w];
+            }
+        }
+        __syncthreads();
+        // into digit order in this CTA; one CTA: that is the pass
+        K* ok = ctas > 1 ? sm.out_key : sm.key;
+        uint32_t* ov = ctas > 1 ? sm.out_val : sm.val;
+#pragma unroll
+        for (int j = 0; j < KPT; ++j) {
+            if (first + own + 32 * j < count) {
+                const uint32_t k = wh[(uint32_t)(key[j] >> shift) & (S::kBins - 1u)] + rank[j];
+                ok[k] = key[j];
+                ov[k] = val[j];
+            }
+        }
+        __syncthreads();
+        if (ctas > 1) {
+            // runs of a digit go to consecutive places, mostly of one CTA
+#pragma unroll
+            for (int j = 0; j < KPT; ++j) {
+                const uint32_t k = tid + j * kLocalThreads;
+                if (first + k < count) {
+                    const K kk = sm.out_key[k];
+                    const uint32_t to = sm.base[(uint32_t)(kk >> shift) & (S::kBins - 1u)] + k;
+                    const uint32_t r = to / S::kTile, q = to % S::kTile;
+                    st_peer(peer_addr(&sm.key[q], r), kk);
+                    st_peer(peer_addr(&sm.val[q], r), sm.out_val[k]);
+                }
+            }
+            cluster_sync();
+        }
+    }
+}
+
+// One mesh: keys (in place) and the permutation.
+template <typename K, int RB, int KPT>
+__global__ __launch_bounds__(kLocalThreads) void sort_cluster_kernel(K* keys, uint32_t* vals, uint32_t n,
+                                                                     uint32_t shift, int passes) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    LocalSmem<K, RB, KPT>& sm = *reinterpret_cast<LocalSmem<K, RB, KPT>*>(smem);
+    constexpr uint32_t T = LocalSmem<K, RB, KPT>::kTile;
+    const uint32_t me = cluster_rank(), first = me * T;
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t k = threadIdx.x + j * kLocalThreads;
+        sm.key[k] = first + k < n ? __ldcg(keys + first + k) : (K)0;
+        sm.val[k] = first + k;
+    }
+    __syncthreads();
+    local_sort<K, RB, KPT>(sm, n, shift, passes, gridDim.x, me);
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t k = threadIdx.x + j * kLocalThreads;
+        if (first + k < n) {
+            keys[first + k] = sm.key[k];
+            vals[first + k] = sm.val[k];
+        }
+    }
+}
+
+// A batch: cluster m sorts mesh m's keys (mesh << 32 | code) by code.
+template <int RB, int KPT>
+__global__ __launch_bounds__(kLocalThreads) void sort_cluster_batch_kernel(uint64_t* keys, uint32_t* vals,
+                                                                           MeshBatch batch, uint32_t ctas,
+                                                                           uint32_t shift, int passes) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    LocalSmem<uint32_t, RB, KPT>& sm = *reinterpret_cast<LocalSmem<uint32_t, RB, KPT>*>(smem);
+    constexpr uint32_t T = LocalSmem<uint32_t, RB, KPT>::kTile;
+    const MeshSpan mesh = batch.span(blockIdx.x / ctas);
+    if (mesh.count == 0) return;  // the whole cluster
+    const uint32_t me = ctas > 1 ? cluster_rank() : 0u, first = me * T;
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t k = threadIdx.x + j * kLocalThreads;
+        sm.key[k] = first + k < mesh.count ? (uint32_t)__ldcg(keys + mesh.start + first + k) : 0u;
+        sm.val[k] = first + k;
+    }
+    __syncthreads();
+    local_sort<uint32_t, RB, KPT>(sm, mesh.count, shift, passes, ctas, me);
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t k = threadIdx.x + j * kLocalThreads;
+        if (first + k < mesh.count) {
+            keys[mesh.start + first + k] = ((uint64_t)mesh.m << 32) | sm.key[k];
+            vals[mesh.start + first + k] = sm.val[k];
+        }
+    }
+}
+
+// Digits of the pipeline's keys: codes of 30 bits are sorted on [2, 30) in
+// four 7-bit digits (bits 30 and 31 are zero), codes of 63 bits on [1, 64)
+// in seven 9-bit digits.
+constexpr int kLocalBits32 = 7, kLocalBits64 = 9;
+
+template <typename Kern>
+cudaError_t local_attributes(Kern* kernel, size_t smem) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (!e) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+cudaLaunchConfig_t local_config(uint32_t grid, uint32_t ctas, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(kLocalThreads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = ctas;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    c.attrs = attr;
+    c.numAttrs = ctas > 1 ? 1 : 0;
+    return c;
+}
+template <typename K, int RB, int KPT>
+cudaError_t launch_local(K* keys, uint32_t* vals, uint32_t n, uint32_t shift, int passes, cudaStream_t s) {
+    constexpr size_t smem = sizeof(LocalSmem<K, RB, KPT>);
+    cudaError_t e = once_per_device([] { return local_attributes(sort_cluster_kernel<K, RB, KPT>, smem); });
+    if (e) return e;
+    constexpr uint32_t T = LocalSmem<K, RB, KPT>::kTile;
+    const uint32_t ctas = (n + T - 1) / T;
+    cudaLaunchAttribute attr{};
+    cudaLaunchConfig_t c = local_config(ctas, ctas, smem, s, &attr);
+    return cudaLaunchKernelEx(&c, sort_cluster_kernel<K, RB, KPT>, keys, vals, n, shift, passes);
+}
+template <int RB, int KPT>
+cudaError_t launch_local_batch(uint64_t* keys, uint32_t* vals, const MeshBatch& batch, uint32_t max_mesh, uint32_t shift,
+                               int passes, cudaStream_t s) {
+    constexpr size_t smem = sizeof(LocalSmem<uint32_t, RB, KPT>);
+    cudaError_t e = once_per_device([] { return local_attributes(sort_cluster_batch_kernel<RB, KPT>, smem); });
+    if (e) return e;
+    constexpr uint32_t T = LocalSmem<uint32_t, RB, KPT>::kTile;
+    const uint32_t ctas = (max_mesh + T - 1) / T;
+    cudaLaunchAttribute attr{};
+    cudaLaunchConfig_t c = local_config(ctas * batch.meshes, ctas, smem, s, &attr);
+    return cudaLaunchKernelEx(&c, sort_cluster_batch_kernel<RB, KPT>, keys, vals, batch, ctas, shift, passes);
+}
+// Keys per thread: as few as the largest cluster (one mesh, where a pass is a
+// chain of steps) or one CTA (a batch, whose meshes share the SMs) can hold.
+// Measured: 4,000 30-bit keys 16 / 18 us at 2 / 8 keys per thread, 16,411
+// 63-bit keys 45 / 65; a batch of 200 meshes of up to 4,096 keys builds in
+// 268 us with four CTAs of 2 keys per thread for the largest, 256 with one of 8.
+template <typename F>
+cudaError_t by_keys_per_thread(uint32_t n, uint32_t ctas, F f) {
+    if (n <= ctas * kLocalThreads * 2) return f(std::integral_constant<int, 2>{});
+    if (n <= ctas * kLocalThreads * 4) return f(std::integral_constant<int, 4>{});
+    return f(std::integral_constant<int, 8>{});
+}
+
 }  // namespace
 
 // Bounded-wait check: one CTA claims tile 1 of a two-tile sort while tile 0
@@ -819,6 +1116,40 @@ cudaError_t run_sort_stall_probe(uint32_t* err_out) {
     if (!e) e = cudaMemcpy(err_out, err, 4, cudaMemcpyDeviceToHost);
     cudaFree(buf);
     return e;
+}
+
+// Up to 65,536 keys, if this device can hold a 16-CTA cluster of the largest
+// form (asked once per device).
+bool local_sort_takes(uint32_t n) {
+    if (n > kLocalMaxKeys) return false;
+    const cudaError_t e = once_per_device([] {
+        auto* kernel = sort_cluster_kernel<uint64_t, kLocalBits64, kLocalMaxKpt>;
+        constexpr size_t smem = sizeof(LocalSmem<uint64_t, kLocalBits64, kLocalMaxKpt>);
+        cudaError_t r = local_attributes(kernel, smem);
+        cudaLaunchAttribute attr{};
+        const cudaLaunchConfig_t c = local_config(kLocalMaxCtas, kLocalMaxCtas, smem, nullptr, &attr);
+        int clusters = 0;
+        if (!r) r = cudaOccupancyMaxActiveClusters(&clusters, kernel, &c);
+        if (!r && clusters < 1) r = cudaErrorNotSupported;
+        if (r) cudaGetLastError();
+        return r;
+    });
+    return e == cudaSuccess;
+}
+
+cudaError_t launch_local_sort(uint32_t key_bytes, void* keys, uint32_t* vals, uint32_t n, cudaStream_t s) {
+    return by_keys_per_thread(n, kLocalMaxCtas, [&](auto kpt) {
+        if (key_bytes == 4)
+            return launch_local<uint32_t, kLocalBits32, decltype(kpt)::value>((uint32_t*)keys, vals, n, 2, 4, s);
+        return launch_local<uint64_t, kLocalBits64, decltype(kpt)::value>((uint64_t*)keys, vals, n, 1, 7, s);
+    });
+}
+
+cudaError_t launch_local_sort_batch(uint64_t* keys, uint32_t* vals, const MeshBatch& batch, uint32_t max_mesh,
+                                    cudaStream_t s) {
+    return by_keys_per_thread(max_mesh, 1, [&](auto kpt) {
+        return launch_local_batch<kLocalBits32, decltype(kpt)::value>(keys, vals, batch, max_mesh, 2, 4, s);
+    });
 }
 
 SortPlan make_sort_plan(uint32_t begin_bit, uint32_t end_bit, uint32_t digit_bits) {
