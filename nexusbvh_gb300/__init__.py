@@ -292,6 +292,7 @@ class Builder:
     def __init__(self):
         load()
         self._ws = None
+        self._host_result = None  # pinned copy of the build result
 
     def sizes(self, n: int, config: BuildConfig) -> CSizes:
         s = CSizes()
@@ -321,9 +322,13 @@ class Builder:
         bvh2_nodes = torch.empty((s.bvh2_node_count, 32), dtype=torch.uint8, device="cuda")
         bvh8_nodes = torch.empty((s.bvh8_node_capacity, 80), dtype=torch.uint8, device="cuda") if wide else None
         prim_idx = torch.empty(n, dtype=torch.int32, device="cuda") if wide else None
-        result = torch.zeros(ctypes.sizeof(CResult), dtype=torch.uint8, device="cuda")
+        result = torch.empty(ctypes.sizeof(CResult), dtype=torch.uint8, device="cuda")  # the build writes all of it
         self.enqueue(prims, n, config, ws, bvh2_nodes, bvh8_nodes, prim_idx, result)
-        r = CResult.from_buffer_copy(result.cpu().numpy().tobytes())
+        if self._host_result is None:
+            self._host_result = torch.empty(ctypes.sizeof(CResult), dtype=torch.uint8, pin_memory=True)
+        self._host_result.copy_(result, non_blocking=True)
+        torch.cuda.current_stream().synchronize()
+        r = CResult.from_buffer_copy(self._host_result.numpy())
         if r.error_word:
             raise NxbError(7 if not (r.error_word & 3) else 6, f"device error word 0x{r.error_word:x}")
         bounds = (tuple(r.scene_bounds.bmin), tuple(r.scene_bounds.bmax))
@@ -358,8 +363,7 @@ def _build_plain(prims, config, metrics, wide):
                                  ctypes.byref(out), mp), "nxb_build_bvh8")
         nodes = torch.empty((out.node_count, 80), dtype=torch.uint8, device="cuda")
         prim_idx = torch.empty(n, dtype=torch.int32, device="cuda")
-        _copy_d2d(nodes.data_ptr(), out.nodes, out.node_count * 80)
-        _copy_d2d(prim_idx.data_ptr(), out.prim_idx, n * 4)
+        _copy_out((nodes, out.nodes), (prim_idx, out.prim_idx))
         bounds = (tuple(out.bounds.bmin), tuple(out.bounds.bmax))
         check(lib.nxb_free_device_bvh8(ctypes.byref(out)), "nxb_free_device_bvh8")
         res = BVH8(nodes, int(out.node_count), prim_idx, n, bounds)
@@ -368,7 +372,7 @@ def _build_plain(prims, config, metrics, wide):
         check(lib.nxb_build_bvh2(prims.data_ptr(), prim_type_of(prims), n, ctypes.byref(c), stream,
                                  ctypes.byref(out), mp), "nxb_build_bvh2")
         nodes = torch.empty((out.node_count, 32), dtype=torch.uint8, device="cuda")
-        _copy_d2d(nodes.data_ptr(), out.nodes, out.node_count * 32)
+        _copy_out((nodes, out.nodes))
         bounds = (tuple(out.bounds.bmin), tuple(out.bounds.bmax))
         check(lib.nxb_free_device_bvh2(ctypes.byref(out)), "nxb_free_device_bvh2")
         res = BVH2(nodes, int(out.node_count), n, bounds)
@@ -378,24 +382,27 @@ def _build_plain(prims, config, metrics, wide):
     return res
 
 
-def _copy_d2d(dst: int, src: int, nbytes: int) -> None:
+def _copy_out(*pairs) -> None:
+    """Copies library-owned device arrays into tensors of their sizes and waits
+    for the copies (the library's memory is freed next)."""
     import torch
-    if nbytes == 0:
-        return
-    # wrap the library-owned pointer without taking ownership
-    src_t = _borrow(src, nbytes)
-    dst_t = _borrow(dst, nbytes)
-    dst_t.copy_(src_t)
-    torch.cuda.synchronize()
+    for dst, src in pairs:
+        flat = dst.view(torch.uint8).view(-1)
+        flat.copy_(_borrow(src, flat.numel()), non_blocking=True)
+    torch.cuda.current_stream().synchronize()
+
+
+class _CudaArray:
+    """Device memory owned by someone else, for torch.as_tensor."""
+
+    def __init__(self, ptr: int, nbytes: int):
+        self.__cuda_array_interface__ = {"shape": (nbytes,), "typestr": "|u1", "data": (ptr, False), "version": 3,
+                                         "strides": None}
 
 
 def _borrow(ptr: int, nbytes: int):
     import torch
-    cls = type("_CudaArray", (), {})
-    obj = cls()
-    obj.__cuda_array_interface__ = {"shape": (nbytes,), "typestr": "|u1", "data": (ptr, False), "version": 3,
-                                    "strides": None}
-    return torch.as_tensor(obj, device="cuda")
+    return torch.as_tensor(_CudaArray(ptr, nbytes), device="cuda")
 
 
 class Batch:

@@ -79,7 +79,7 @@ Layout make_layout(uint32_t n, uint32_t key_bits) {
     };
     L.ctrl = seg(sizeof(Control));
     L.result = seg(sizeof(nxb_build_result));
-    L.cost = seg(2 * sizeof(float));
+    L.cost = seg(2 * sizeof(float));  // next to the result: both are read back in one copy
     L.keys_a = seg((size_t)L.key_bytes * n);
     L.keys_b = seg((size_t)L.key_bytes * n);
     L.vals_a = seg(4ull * n);
@@ -277,11 +277,18 @@ nxb_status build_plain(const void* prims, nxb_prim_type type, uint32_t n, const 
             if (e) status = cuda_fail(e);
         }
         if (status == NXB_OK) {
-            e = cudaMemcpyAsync(&res, d_res, sizeof(res), cudaMemcpyDeviceToHost, s);
+            unsigned char back[2 * kAlign];
+            static_assert(sizeof(res) <= kAlign, "the costs follow the result");
             float costs[2] = {0.f, 0.f};
-            if (!e && metrics) e = cudaMemcpyAsync(costs, d_cost, sizeof(costs), cudaMemcpyDeviceToHost, s);
+            const size_t bytes = metrics ? L.cost - L.result + sizeof(costs) : sizeof(res);
+            e = cudaMemcpyAsync(back, d_res, bytes, cudaMemcpyDeviceToHost, s);
             if (!e) e = cudaStreamSynchronize(s);
-            if (e) status = cuda_fail(e);
+            if (e) {
+                status = cuda_fail(e);
+            } else {
+                std::memcpy(&res, back, sizeof(res));
+                if (metrics) std::memcpy(costs, back + (L.cost - L.result), sizeof(costs));
+            }
             if (status == NXB_OK) status = status_from_error_word(res.error_word);
             if (status == NXB_OK && validate_of(cfg))
                 status = validate_built(prims, type, n, bvh2, wide ? bvh8 : nullptr, prim_idx, res.bvh8_node_count, s);
