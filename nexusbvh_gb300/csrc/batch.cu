@@ -6,10 +6,12 @@
 // small mesh's build time consists of.  A batch lays the meshes end to end
 // and runs each stage once over all of them:
 //   * scene bounds per mesh (warp-reduced into 6 ordered words per mesh);
-//   * 30-bit Morton codes from each mesh's own box, sorted as one 64-bit
-//     key mesh << 32 | code over bits [2, 32 + mesh bits): per mesh this is
-//     exactly the plain sort by code >> 2 (stable), and the meshes stay in
-//     order;
+//   * 30-bit Morton codes from each mesh's own box, sorted within every mesh
+//     by code >> 2 (stable), which is exactly the plain sort: in one cluster
+//     per mesh if no mesh is larger than that takes, else in segmented
+//     passes, else (many small meshes beside a large one) as one 64-bit key
+//     mesh << 32 | code over bits [2, 32 + mesh bits), which keeps the
+//     meshes in order;
 //   * H-PLOC and the BVH8 collapse with mesh-local indices (MeshBatch in
 //     common.cuh), so every mesh's BVH2 is the plain build's array;
 //   * nxb_batch_* capture the whole sequence once in a CUDA graph and
@@ -161,7 +163,10 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
     const MeshGroups& g = (groups && fork && groups->count > 1) ? *groups : one;
     const MeshBatch mb{a.off, a.off8, a.meshes};
     const bool local = local_sort_takes(a.max_mesh);
-    const SortPlan plan = local ? SortPlan{} : make_sort_plan(2, 32 + a.mesh_bits, t.digit_bits);
+    SegmentPlan segments{};
+    const bool seg = !local && segment_sort_takes(a.total, a.meshes, a.lookback,
+                                                  a.lookback_words_per_pass * kMaxSortPasses, &segments);
+    const SortPlan plan = local || seg ? SortPlan{} : make_sort_plan(2, 32 + a.mesh_bits, t.digit_bits);
     NXB_TRY(cudaMemsetAsync(a.zero_begin, 0, a.zero_bytes, s));
     if (a.total > 0) {
         NXB_TRY(launch_batch_tile_ranges(mb, a.total, t.block, a.tile_rng, s));
@@ -171,8 +176,18 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
         f.zero_words = align_up(4 * a.lookback_words_per_pass * plan.passes) / 4;
         f.ones_ptr = a.parent;
         f.ones_words = a.ones_words;
-        NXB_TRY(launch_batch_morton(a.bvh2, mb, a.total, a.scene_ord, a.keys_a, a.vals_a, plan, &a.ctrl->hist[0][0],
-                                    f, t.block, a.tile_rng, s));
+        if (seg) {
+            f.zero_ptr = segments.lookback;
+            f.zero_words = segments.lookback_words;
+            NXB_TRY(launch_segment_prepare(segments, mb, s));
+            NXB_TRY(launch_segment_morton(a.bvh2, mb, a.scene_ord, reinterpret_cast<uint32_t*>(a.keys_b), segments, f,
+                                          t.block, s));
+            NXB_TRY(launch_segment_sort(segments, mb, a.total, a.keys_a, a.keys_b, a.vals_a, a.vals_b,
+                                        a.ctrl->tile_ctr, &a.ctrl->error_word, s));
+        } else {
+            NXB_TRY(launch_batch_morton(a.bvh2, mb, a.total, a.scene_ord, a.keys_a, a.vals_a, plan,
+                                        &a.ctrl->hist[0][0], f, t.block, a.tile_rng, s));
+        }
         if (local) NXB_TRY(launch_local_sort_batch(a.keys_a, a.vals_a, mb, a.max_mesh, s));
         for (int p = 0; p < plan.passes; ++p) {
             const bool even = (p % 2) == 0;

@@ -180,6 +180,32 @@ bool local_sort_takes(uint32_t n);
 cudaError_t launch_local_sort(uint32_t key_bytes, void* keys, uint32_t* vals, uint32_t n, cudaStream_t s);
 cudaError_t launch_local_sort_batch(uint64_t* keys, uint32_t* vals, const MeshBatch& batch, uint32_t max_mesh,
                                     cudaStream_t s);
+// The sort of a batch whose meshes are larger than that: every mesh's codes
+// by themselves (a segment of its own in the buffers), bits [2, 30) in four
+// 7-bit passes.  A segment is cut into tiles of kSegmentTile keys.  Mesh m's
+// tiles have the numbers from off[m] / kSegmentTile + m on; that needs no
+// prefix sum over the meshes, and leaves at most one number per mesh without
+// keys.
+constexpr uint32_t kSegmentTile = 4096;
+constexpr uint32_t kSegmentBits = 7, kSegmentBins = 1u << kSegmentBits, kSegmentPasses = 4;
+struct SegmentPlan {
+    uint32_t tiles;      // tile numbers
+    uint32_t* hist;      // kSegmentPasses x kSegmentBins words per mesh
+    uint32_t* mesh_of;   // mesh of every tile number
+    uint32_t* lookback;  // kSegmentPasses x tiles x kSegmentBins words
+    size_t lookback_words;
+};
+// Whether the batch takes it; if so, *plan is laid out in the `words` words
+// (16-byte aligned) at `at`.
+bool segment_sort_takes(uint32_t total, uint32_t meshes, uint32_t* at, size_t words, SegmentPlan* plan);
+// Writes mesh_of and clears hist.
+cudaError_t launch_segment_prepare(const SegmentPlan& plan, const MeshBatch& batch, cudaStream_t s);
+// Sorts the codes in keys_b (32 bits each, from its start); the sorted keys
+// mesh << 32 | code and the mesh-local permutation end in keys_a and vals_a.
+// lookback and kSegmentPasses counters at tile_ctr are zero on entry.
+cudaError_t launch_segment_sort(const SegmentPlan& plan, const MeshBatch& batch, uint32_t total, uint64_t* keys_a,
+                                uint64_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t* tile_ctr,
+                                uint32_t* err, cudaStream_t s);
 // ---------------------------------------------------------------- stage 4
 // parent: n words holding INVALID on entry; parent_of_last: one word that
 // must hold INVALID on entry; tile_ctr: one word that must be zero on entry.
@@ -223,6 +249,11 @@ cudaError_t launch_batch_bounds(const void* prims, int prim_type, const MeshBatc
 cudaError_t launch_batch_morton(const Node2* nodes, const MeshBatch& batch, uint32_t total, const uint32_t* scene_ord,
                                 uint64_t* keys, uint32_t* vals, const SortPlan& plan, uint32_t* hist,
                                 const MortonFused& fill, uint32_t block, const uint2* tile_rng, cudaStream_t s);
+// For launch_segment_sort: the 32-bit codes alone, and the digit counts of
+// every mesh in plan.hist.
+cudaError_t launch_segment_morton(const Node2* nodes, const MeshBatch& batch, const uint32_t* scene_ord,
+                                  uint32_t* codes, const SegmentPlan& plan, const MortonFused& fill, uint32_t block,
+                                  cudaStream_t s);
 // H-PLOC over the sorted positions [begin, end), which must cover whole
 // meshes; leaf_ctr: a zeroed word of its own.  parent_of_last: one word per
 // mesh holding INVALID on entry; ctas_per_sm caps the persistent grid (0: as

@@ -1086,6 +1086,166 @@ cudaError_t by_keys_per_thread(uint32_t n, uint32_t ctas, F f) {
     return f(std::integral_constant<int, 8>{});
 }
 
+// ---- segmented passes: the meshes of a batch, each sorted by itself
+//
+// As one sort of mesh << 32 | code, a batch pays for the mesh bits, although
+// the meshes already lie in order, and moves 64-bit keys.  Here a pass sorts
+// 32-bit codes within every mesh: a tile belongs to one mesh, only looks
+// back over that mesh's tiles, and takes its digit starts from that mesh's
+// counts.  The passes cover bits [2, 30) in 7-bit digits; the first takes
+// the values from the positions, the last writes mesh << 32 | code, which
+// the climb reads.  Bound by ranking and its shared-memory traffic, not by
+// DRAM: 16 keys per thread and four CTAs per SM (five for the first pass,
+// which holds no values).  1,024 meshes of 36.5M triangles together: 193 +
+// 3 x 214 us, where five passes over 64-bit keys took 1,701; with five CTAs
+// throughout the later passes spill and take 223 each, with three 250.
+constexpr uint32_t kSegmentMinMean = 1536;
+
+__global__ __launch_bounds__(kThreads) void segment_prepare_kernel(SegmentPlan plan, MeshBatch batch) {
+    const uint32_t tid = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
+    for (uint32_t t = tid; t < plan.tiles; t += stride) {
+        uint32_t lo = 0, hi = batch.meshes - 1;  // the last mesh whose first tile is not after t
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo + 1) / 2;
+            if (__ldg(batch.off + mid) / kSegmentTile + mid <= t)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        plan.mesh_of[t] = lo;
+    }
+    const size_t vec4 = (size_t)batch.meshes * kSegmentPasses * kSegmentBins / 4;
+    for (size_t i = tid; i < vec4; i += stride) reinterpret_cast<uint4*>(plan.hist)[i] = make_uint4(0, 0, 0, 0);
+}
+
+template <bool FIRST, bool LAST>
+__global__ __launch_bounds__(kThreads, FIRST ? 5 : 4) void segment_pass_kernel(
+    const uint32_t* __restrict__ kin, void* __restrict__ kout, const uint32_t* __restrict__ vin,
+    uint32_t* __restrict__ vout, MeshBatch batch, SegmentPlan plan, uint32_t pass, uint32_t* tile_ctr, uint32_t* err) {
+    constexpr int KPT = kSegmentTile / kThreads;
+    constexpr uint32_t BINS = kSegmentBins;
+    static_assert(BINS <= kThreads, "a thread per digit");
+    __shared__ uint32_t s_keys[kSegmentTile], s_vals[kSegmentTile];
+    __shared__ uint32_t s_whist[kWarps * BINS];
+    __shared__ uint32_t s_local[BINS], s_delta[BINS], s_tmp[kWarps], s_tile;
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const uint32_t shift = 2 + pass * kSegmentBits;
+    if (tid == 0) s_tile = atomicAdd(tile_ctr + pass, 1u);
+    for (uint32_t i = tid; i < kWarps * BINS; i += kThreads) s_whist[i] = 0;
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    if (tile >= plan.tiles) return;
+    const MeshSpan mesh = batch.span(__ldg(plan.mesh_of + tile));
+    const uint32_t nth = tile - (mesh.start / kSegmentTile + mesh.m);  // of the mesh's tiles
+    const uint32_t base = nth * kSegmentTile, n = mesh.count;
+    if (base >= n) return;
+    kin += mesh.start;
+    if (!FIRST) vin += mesh.start;
+    vout += mesh.start;
+    const uint32_t* hist = plan.hist + ((size_t)mesh.m * kSegmentPasses + pass) * BINS;
+    uint32_t* lookback = plan.lookback + ((size_t)pass * plan.tiles + tile) * BINS;
+
+    uint32_t key[KPT], val[KPT], rank[KPT];
+    const uint32_t wbase = base + warp * 32u * KPT + lane;
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t i = wbase + 32u * j;
+        key[j] = i < n ? kin[i] : 0u;
+        val[j] = FIRST ? i : (i < n ? vin[i] : 0u);
+    }
+    uint32_t* wh = s_whist + warp * BINS;
+    const uint32_t lt_mask = lanemask_lt();
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const bool valid = wbase + 32u * j < n;
+        const uint32_t d = (key[j] >> shift) & (BINS - 1);
+        uint32_t peers = __ballot_sync(kFullMask, valid);
+#pragma unroll
+        for (uint32_t b = 0; b < kSegmentBits; ++b) {
+            const bool bit = (d >> b) & 1u;
+            const uint32_t bb = __ballot_sync(kFullMask, bit);
+            peers &= bit ? bb : ~bb;
+        }
+        const uint32_t below = __popc(peers & lt_mask);
+        const uint32_t leader = (uint32_t)(__ffs(peers) - 1) & 31u;
+        uint32_t start = 0;
+        if (valid && below == 0) {
+            start = wh[d];
+            wh[d] = start + __popc(peers);
+        }
+        start = __shfl_sync(kFullMask, start, leader);
+        rank[j] = start + below;
+        __syncwarp();
+    }
+    __syncthreads();
+
+    // ---- the tile's digit counts; publish and look back (thread = digit)
+    uint32_t count = 0, excl = 0;
+    if (tid < BINS) {
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t x = s_whist[w * BINS + tid];
+            s_whist[w * BINS + tid] = count;
+            count += x;
+        }
+        if (nth) atomicExch(lookback + tid, kFlagAgg | count);
+    }
+    if (nth == 0) {  // CTA-uniform
+        excl = cta_exclusive_scan(tid < BINS ? hist[tid] : 0u, s_tmp);
+    } else if (tid < BINS) {
+        const uint32_t* pred = lookback + tid;
+        uint32_t left = nth, polls = 0;
+        pred -= BINS;
+        while (left) {
+            const uint32_t v = ld_relaxed_u32(pred);
+            const uint32_t flag = v & ~kCountMask;
+            if (flag == 0) {
+                if (++polls > kSpinLimit) {
+                    set_error(err, NXB_DEVERR_SORT_LOOKBACK_TIMEOUT);
+                    break;
+                }
+                if (polls > 64) __nanosleep(64);
+                continue;
+            }
+            excl += v & kCountMask;
+            if (flag == kFlagInc) break;
+            --left;
+            pred -= BINS;
+        }
+    }
+    if (tid < BINS) atomicExch(lookback + tid, kFlagInc | (excl + count));
+    const uint32_t local = cta_exclusive_scan(count, s_tmp);
+    if (tid < BINS) {
+        s_local[tid] = local;
+        s_delta[tid] = excl - local;
+    }
+    __syncthreads();
+
+    // ---- reorder by digit in shared memory, then scatter runs of a digit
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        if (wbase + 32u * j < n) {
+            const uint32_t d = (key[j] >> shift) & (BINS - 1);
+            const uint32_t pos = s_local[d] + wh[d] + rank[j];
+            s_keys[pos] = key[j];
+            s_vals[pos] = val[j];
+        }
+    }
+    __syncthreads();
+    const uint32_t tile_n = min(kSegmentTile, n - base);
+    for (uint32_t i = tid; i < tile_n; i += kThreads) {
+        const uint32_t k = s_keys[i];
+        const uint32_t g = s_delta[(k >> shift) & (BINS - 1)] + i;
+        if (g < n) {  // always true unless a look-back wait expired
+            if (LAST)
+                reinterpret_cast<uint64_t*>(kout)[mesh.start + g] = ((uint64_t)mesh.m << 32) | k;
+            else
+                reinterpret_cast<uint32_t*>(kout)[mesh.start + g] = k;
+            vout[g] = s_vals[i];
+        }
+    }
+}
+
 }  // namespace
 
 // Bounded-wait check: one CTA claims tile 1 of a two-tile sort while tile 0
@@ -1150,6 +1310,58 @@ cudaError_t launch_local_sort_batch(uint64_t* keys, uint32_t* vals, const MeshBa
     return by_keys_per_thread(max_mesh, 1, [&](auto kpt) {
         return launch_local_batch<kLocalBits32, decltype(kpt)::value>(keys, vals, batch, max_mesh, 2, 4, s);
     });
+}
+
+// Batches whose meshes have 1,536 primitives or more on average: with more
+// meshes than that, their counts and look-back words don't fit the memory
+// that the passes over mesh and code need.  The line costs nothing: one mesh
+// of 70,000 and others of s on average, 6M primitives together, whole build,
+// this way against the passes over mesh and code: s = 30,000 1,851 against
+// 2,060 us, 8,192 1,656 / 1,851, 3,000 1,776 / 1,988, 1,500 1,899 / 2,020.
+bool segment_sort_takes(uint32_t total, uint32_t meshes, uint32_t* at, size_t words, SegmentPlan* plan) {
+    if ((uint64_t)meshes * kSegmentMinMean > total) return false;
+    const size_t tiles = (size_t)total / kSegmentTile + meshes;
+    const size_t hist = (size_t)meshes * kSegmentPasses * kSegmentBins;
+    const size_t lookback = tiles * kSegmentPasses * kSegmentBins;
+    if (hist + lookback + tiles > words) return false;
+    plan->tiles = (uint32_t)tiles;
+    plan->hist = at;
+    plan->lookback = at + hist;
+    plan->lookback_words = lookback;
+    plan->mesh_of = at + hist + lookback;
+    return true;
+}
+
+cudaError_t launch_segment_prepare(const SegmentPlan& plan, const MeshBatch& batch, cudaStream_t s) {
+    const uint32_t grid = std::min((plan.tiles + kThreads - 1) / kThreads, (uint32_t)device_info().sms * 4);
+    segment_prepare_kernel<<<grid, kThreads, 0, s>>>(plan, batch);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_segment_sort(const SegmentPlan& plan, const MeshBatch& batch, uint32_t total, uint64_t* keys_a,
+                                uint64_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t* tile_ctr,
+                                uint32_t* err, cudaStream_t s) {
+    const cudaError_t e = once_per_device([] {
+        cudaError_t r = cudaSuccess;
+        for (auto* kernel : {segment_pass_kernel<true, false>, segment_pass_kernel<false, false>,
+                             segment_pass_kernel<false, true>})
+            if (!r)
+                r = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         cudaSharedmemCarveoutMaxShared);
+        return r;
+    });
+    if (e) return e;
+    uint32_t* k0 = reinterpret_cast<uint32_t*>(keys_b);  // the passes go to and fro in the halves of keys_b
+    uint32_t* k1 = k0 + total;
+    segment_pass_kernel<true, false>
+        <<<plan.tiles, kThreads, 0, s>>>(k0, k1, nullptr, vals_b, batch, plan, 0, tile_ctr, err);
+    segment_pass_kernel<false, false>
+        <<<plan.tiles, kThreads, 0, s>>>(k1, k0, vals_b, vals_a, batch, plan, 1, tile_ctr, err);
+    segment_pass_kernel<false, false>
+        <<<plan.tiles, kThreads, 0, s>>>(k0, k1, vals_a, vals_b, batch, plan, 2, tile_ctr, err);
+    segment_pass_kernel<false, true>
+        <<<plan.tiles, kThreads, 0, s>>>(k1, keys_a, vals_b, vals_a, batch, plan, 3, tile_ctr, err);
+    return cudaGetLastError();
 }
 
 SortPlan make_sort_plan(uint32_t begin_bit, uint32_t end_bit, uint32_t digit_bits) {
