@@ -83,7 +83,11 @@ __device__ __forceinline__ T ld_data(const T* p) {
 // adjacent digits in the tile-wide steps (publish, look-back, scans).  L2:
 // every load of data written by other CTAs bypasses L1 (the persistent
 // fallback kernel reads buffers that other CTAs of the same launch wrote).
-template <typename K, bool HAS_VALS, int RB, bool L2>
+// FULL: the digits are as wide as the tables (bits == RB), so the ranking's
+// ballots and the tables' bounds are fixed when compiled: the four 9-bit
+// passes and the bucket sort of 12.58M 63-bit keys 660 -> 611 us, eight 8-bit
+// passes of 5.0M keys 532 -> 503.
+template <typename K, bool HAS_VALS, int RB, bool L2, bool FULL>
 __device__ __forceinline__ void sort_tile(uint32_t tile, const K* __restrict__ kin, K* __restrict__ kout,
                                           const uint32_t* __restrict__ vin, uint32_t* __restrict__ vout, uint32_t n,
                                           uint32_t shift, uint32_t bits, const uint32_t* __restrict__ hist,
@@ -98,6 +102,7 @@ __device__ __forceinline__ void sort_tile(uint32_t tile, const K* __restrict__ k
     uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + TILE);
     uint32_t* s_whist = s_vals + TILE;
 
+    if constexpr (FULL) bits = RB;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     const uint32_t mask = (1u << bits) - 1u;
     const uint32_t tile_base = tile * (uint32_t)TILE;
@@ -293,7 +298,7 @@ __device__ __forceinline__ void sort_tile(uint32_t tile, const K* __restrict__ k
     }
 }
 
-template <typename K, bool HAS_VALS, int RB>
+template <typename K, bool HAS_VALS, int RB, bool FULL>
 __global__ __launch_bounds__(kThreads, 4) void onesweep_kernel(const K* __restrict__ kin, K* __restrict__ kout,
                                                             const uint32_t* __restrict__ vin,
                                                             uint32_t* __restrict__ vout, uint32_t n, uint32_t shift,
@@ -308,8 +313,8 @@ __global__ __launch_bounds__(kThreads, 4) void onesweep_kernel(const K* __restri
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
     for (int i = threadIdx.x; i < kWarps * (1 << RB); i += kThreads) s_whist[i] = 0;
     __syncthreads();
-    sort_tile<K, HAS_VALS, RB, false>(s_tile, kin, kout, vin, vout, n, shift, bits, hist, lookback, err, smem, s_delta,
-                                      s_local, s_tmp);
+    sort_tile<K, HAS_VALS, RB, false, FULL>(s_tile, kin, kout, vin, vout, n, shift, bits, hist, lookback, err, smem,
+                                            s_delta, s_local, s_tmp);
 }
 
 // The same pass for 32-bit keys (8-bit digits, one digit per thread) as a
@@ -317,7 +322,7 @@ __global__ __launch_bounds__(kThreads, 4) void onesweep_kernel(const K* __restri
 // warp instructions (28.4 M against 22.8 M for a 4.19M-key pass) and takes
 // 11 % longer (0.478 against 0.428 ms for the four passes of 12.58M 30-bit
 // keys); for 64-bit keys sort_tile is not slower.
-template <bool HAS_VALS>
+template <bool HAS_VALS, bool FULL>
 __global__ __launch_bounds__(kThreads, 4) void onesweep32_kernel(const uint32_t* __restrict__ kin, uint32_t* __restrict__ kout,
                                                             const uint32_t* __restrict__ vin,
                                                             uint32_t* __restrict__ vout, uint32_t n, uint32_t shift,
@@ -335,6 +340,7 @@ __global__ __launch_bounds__(kThreads, 4) void onesweep32_kernel(const uint32_t*
     __shared__ uint32_t s_tmp[kWarps];
     __shared__ uint32_t s_tile;
 
+    if constexpr (FULL) bits = kRadixBits;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     const uint32_t mask = (1u << bits) - 1u;
     if (tid == 0) s_tile = atomicAdd(tile_ctr, 1u);
@@ -469,18 +475,25 @@ cudaError_t set_smem_attributes(Kern* kernel, size_t bytes) {
     return r;
 }
 
+// The kernel of a pass: FULL if its digits are as wide as the tables.
+template <typename K, int RB>
+auto* onesweep_of(bool has_vals, bool full) {
+    if constexpr (sizeof(K) == 4) {
+        static_assert(RB == kRadixBits, "32-bit keys take 8-bit digits");
+        return full ? (has_vals ? onesweep32_kernel<true, true> : onesweep32_kernel<false, true>)
+                    : (has_vals ? onesweep32_kernel<true, false> : onesweep32_kernel<false, false>);
+    } else {
+        return full ? (has_vals ? onesweep_kernel<K, true, RB, true> : onesweep_kernel<K, false, RB, true>)
+                    : (has_vals ? onesweep_kernel<K, true, RB, false> : onesweep_kernel<K, false, RB, false>);
+    }
+}
+
 template <typename K, int RB>
 cudaError_t configure_onesweep() {
     return once_per_device([] {
-        constexpr size_t smem = dyn_smem_bytes<K, RB>();
-        cudaError_t r;
-        if constexpr (sizeof(K) == 4) {
-            r = set_smem_attributes(onesweep32_kernel<true>, smem);
-            if (!r) r = set_smem_attributes(onesweep32_kernel<false>, smem);
-        } else {
-            r = set_smem_attributes(onesweep_kernel<K, true, RB>, smem);
-            if (!r) r = set_smem_attributes(onesweep_kernel<K, false, RB>, smem);
-        }
+        cudaError_t r = cudaSuccess;
+        for (int form = 0; form < 4 && !r; ++form)
+            r = set_smem_attributes(onesweep_of<K, RB>(form & 1, form & 2), dyn_smem_bytes<K, RB>());
         return r;
     });
 }
@@ -489,26 +502,12 @@ template <typename K, int RB>
 cudaError_t launch_pass_t(const K* kin, K* kout, const uint32_t* vin, uint32_t* vout, uint32_t n, uint32_t shift,
                           uint32_t bits, const uint32_t* hist, uint32_t* lookback, uint32_t* tile_ctr, uint32_t* err,
                           cudaStream_t s) {
-    constexpr size_t smem = dyn_smem_bytes<K, RB>();
     cudaError_t e = configure_onesweep<K, RB>();
     if (e != cudaSuccess) return e;
     const uint32_t tiles = (n + tile_keys<K>() - 1) / tile_keys<K>();
-    if constexpr (sizeof(K) == 4) {
-        static_assert(RB == kRadixBits, "32-bit keys take 8-bit digits");
-        if (vin)
-            onesweep32_kernel<true><<<tiles, kThreads, smem, s>>>(kin, kout, vin, vout, n, shift, bits, hist, lookback,
-                                                                  tile_ctr, err);
-        else
-            onesweep32_kernel<false><<<tiles, kThreads, smem, s>>>(kin, kout, vin, vout, n, shift, bits, hist,
-                                                                   lookback, tile_ctr, err);
-    } else {
-        if (vin)
-            onesweep_kernel<K, true, RB><<<tiles, kThreads, smem, s>>>(kin, kout, vin, vout, n, shift, bits, hist,
-                                                                      lookback, tile_ctr, err);
-        else
-            onesweep_kernel<K, false, RB><<<tiles, kThreads, smem, s>>>(kin, kout, vin, vout, n, shift, bits, hist,
-                                                                       lookback, tile_ctr, err);
-    }
+    auto* kernel = onesweep_of<K, RB>(vin != nullptr, bits == RB);
+    kernel<<<tiles, kThreads, (dyn_smem_bytes<K, RB>()), s>>>(kin, kout, vin, vout, n, shift, bits, hist, lookback,
+                                                              tile_ctr, err);
     return cudaGetLastError();
 }
 
@@ -779,7 +778,7 @@ __global__ __launch_bounds__(kThreads, 4) void sort_fallback_kernel(K* ka, K* kb
         } else {
             const uint32_t p = stage - 2;
             const bool even = (p & 1u) == 0;
-            sort_tile<K, true, kRadixBits, true>(local, even ? ka : kb, even ? kb : ka, even ? va : vb, even ? vb : va,
+            sort_tile<K, true, kRadixBits, true, false>(local, even ? ka : kb, even ? kb : ka, even ? va : vb, even ? vb : va,
                                                  n, f.plan.shift[p], f.plan.bits[p], f.hist + p * kRadixBins,
                                                  f.lookback + (size_t)p * f.lookback_per_pass, err, smem, s_delta,
                                                  s_local, s_tmp);
@@ -1270,7 +1269,7 @@ cudaError_t run_sort_stall_probe(uint32_t* err_out) {
     constexpr size_t smem = dyn_smem_bytes<uint32_t, kRadixBits>();
     if (!e) e = configure_onesweep<uint32_t, kRadixBits>();
     if (!e) {
-        onesweep32_kernel<false><<<1, kThreads, smem>>>(keys, kout, nullptr, vout, n, 0, 8, hist, lookback, ctr, err);
+        onesweep32_kernel<false, true><<<1, kThreads, smem>>>(keys, kout, nullptr, vout, n, 0, 8, hist, lookback, ctr, err);
         e = cudaGetLastError();
     }
     if (!e) e = cudaMemcpy(err_out, err, 4, cudaMemcpyDeviceToHost);
