@@ -314,6 +314,32 @@ __global__ void bvh8_batch_init_kernel(uint64_t* pairs, uint32_t slots, MeshBatc
     }
 }
 
+// A warp's account with the count of allocated-but-unfinished items: what it
+// allocates is added before the items are handed out, what it has finished
+// beyond that is kept as a credit for the items that it allocates next, and
+// subtracted only when it runs out of work.  The count is never too low, so
+// it reaches zero when no item is in flight and no warp holds a credit.
+// Added and subtracted after every pass of a warp instead, it was a third
+// atomic per pass on a line that every idle warp polls: 12.58M clustered
+// triangles 530 -> 512 us, 6.0M 340 -> 313, 4.19M sphere 245 -> 237.
+struct PendingCredit {
+    uint32_t* count;
+    uint32_t held = 0;
+    __device__ __forceinline__ void add(uint32_t allocated, uint32_t finished) {
+        held += finished;
+        if (allocated > held) {
+            if (lane_id() == 0) atomicAdd(count, allocated - held);
+            held = 0;
+        } else {
+            held -= allocated;
+        }
+    }
+    __device__ __forceinline__ void settle() {
+        if (held && lane_id() == 0) atomicAdd(count, 0u - held);
+        held = 0;
+    }
+};
+
 // Work items are the internal BVH8 nodes only: a parent writes the
 // primitive of each leaf child straight into primIdx (it holds the leaf's
 // node in its slot table), instead of queueing a work item per leaf as the
@@ -358,6 +384,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
     uint32_t slot = kInvalid;
     bool retired = false;
     uint32_t idle = 0;
+    PendingCredit credit{ctr + kBvh8Pending};
     for (;;) {
         // lanes without a slot claim the next ones, in increasing order; a
         // slot past the queue's end is never allocated and retires the lane
@@ -376,7 +403,10 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
                     retired = true;
             }
         }
-        if (__all_sync(kFullMask, retired)) return;
+        if (__all_sync(kFullMask, retired)) {
+            credit.settle();
+            return;
+        }
         uint64_t pr = 0;
         bool ready = false;
         if (slot != kInvalid) {
@@ -385,6 +415,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
         }
         if (!__any_sync(kFullMask, ready)) {
             // nothing ready: finished when no allocated item is outstanding
+            credit.settle();
             if (ld_relaxed_u32(ctr + kBvh8Pending) == 0) return;
             if (++idle > kQueueSpinLimit) {
                 if (lane == 0) set_error(err, NXB_DEVERR_BVH8_QUEUE_TIMEOUT);
@@ -546,6 +577,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
         }
         const uint32_t done = __popc(__ballot_sync(kFullMask, ready));
         // one 64-bit atomic: work slots (one mesh: = BVH8 nodes) low, leaves high
+        credit.add(__shfl_sync(kFullMask, incl >> 20, 31), done);
         uint64_t bases = 0;
         if (lane == 31) {
             const uint64_t tl = (incl >> 10) & 0x3FFu, tw = incl >> 20;
@@ -606,11 +638,6 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
                 reinterpret_cast<uint4*>(out + to)[part] = stage[u];
         }
         __syncwarp();
-        // pending += items allocated - items finished (one atomic, so it can
-        // only reach zero when no item is in flight)
-        __syncwarp();
-        const uint32_t new_items = __shfl_sync(kFullMask, incl >> 20, 31);
-        if (lane == 0 && new_items != done) atomicAdd(ctr + kBvh8Pending, new_items - done);
     }
 }
 
@@ -756,6 +783,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
     uint32_t slot = kInvalid;
     bool retired = false;
     uint32_t idle = 0;
+    PendingCredit credit{ctr + kBvh8Pending};
     for (;;) {
         // groups without a slot claim the next ones (see bvh8_kernel)
         const bool want = !retired && slot == kInvalid;
@@ -772,12 +800,16 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
                     retired = true;
             }
         }
-        if (__all_sync(kFullMask, retired)) return;
+        if (__all_sync(kFullMask, retired)) {
+            credit.settle();
+            return;
+        }
         uint64_t pr = ~0ull;
         if (slot != kInvalid) pr = ld_relaxed_u64(pairs + slot);
         pr = __shfl_sync(kFullMask, pr, 0, 8);  // one lane's view for the whole group
         const bool ready = (uint32_t)(pr >> 32) != kInvalid;
         if (!__any_sync(kFullMask, ready)) {
+            credit.settle();
             if (ld_relaxed_u32(ctr + kBvh8Pending) == 0) return;
             if (++idle > kQueueSpinLimit) {
                 if (lane == 0) set_error(err, NXB_DEVERR_BVH8_QUEUE_TIMEOUT);
@@ -906,6 +938,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
         const uint32_t done = __popc(__ballot_sync(kFullMask, ready && sub == 0));
         const uint32_t new_items = total & 0xFFFFu;
         const uint64_t tl = Seg::kBatch ? 0u : total >> 16;
+        credit.add(new_items, done);
         uint64_t bases = 0;
         if (lane == 0 && (tl | new_items))
             bases = atomicAdd(reinterpret_cast<unsigned long long*>(ctr + kBvh8Alloc),
@@ -938,9 +971,6 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
             }
         }
         if (internal) slot = kInvalid;
-        // pending += items allocated - items finished (see bvh8_kernel)
-        __syncwarp();
-        if (lane == 0 && new_items != done) atomicAdd(ctr + kBvh8Pending, new_items - done);
         // the node: lane s quantises slot s (write_node8)
         if (__any_sync(kFullMask, write)) {
             const uint8_t ex = (uint8_t)ceil_log2_biased((nb.mx.x - nb.mn.x) * kQuantStep);
