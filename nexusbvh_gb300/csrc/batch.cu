@@ -203,6 +203,10 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
         uint64_t* keys = in_a ? a.keys_a : a.keys_b;
         uint32_t* perm = in_a ? a.vals_a : a.vals_b;
         uint32_t* tokens = in_a ? a.vals_b : a.vals_a;
+        // a whole batch's collapse has the sort's buffers (24 bytes per
+        // primitive) for its lists; that of a group has not, as the climb of
+        // the next group still reads them
+        uint64_t* lists = g.count == 1 ? a.keys_a : nullptr;
         // H-PLOC group by group on s; the collapse of group k follows it on
         // the side stream (ordered by an event, no wait inside any kernel),
         // overlapping H-PLOC of group k+1
@@ -221,7 +225,7 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
             NXB_TRY(launch_bvh8_batch(a.bvh2, view, g.prim[k + 1] - g.prim[k], a.bvh8, g.slot[k + 1] - g.slot[k],
                                       a.prim_idx, a.pairs + g.slot[k], a.ctr8 + k * kBvh8CtrWords,
                                       a.mesh_nodes + m0, a.mesh_leaves + m0, &a.ctrl->error_word, t.auction, bs,
-                                      a.kids));
+                                      a.kids, lists));
         }
         if (g.count > 1) {
             NXB_TRY(cudaEventRecord(fork->join, fork->side));

@@ -209,9 +209,10 @@ nxb_status enqueue_build(const void* prims, nxb_prim_type type, uint32_t n, cons
                          bvh8 ? ctrl->bvh8_ctr : nullptr, kids));
     NXB_TRY(mark(4));
     if (bvh8) {
-        // the climb initialised the collapse's work queue
+        // the climb initialised the collapse's work queue, and is done with
+        // its cluster records
         NXB_TRY(launch_bvh8(bvh2, n, bvh8, (uint32_t)bvh8_capacity(n), prim_idx, pairs, ctrl->bvh8_ctr,
-                            &ctrl->error_word, auction_of(cfg), s, kids));
+                            &ctrl->error_word, auction_of(cfg), s, kids, reinterpret_cast<uint64_t*>(ws + L.records)));
     }
     NXB_TRY(mark(5));
     if (result) NXB_TRY(launch_finalize(ctrl, result, n, s));

@@ -229,9 +229,11 @@ cudaError_t launch_bvh8_init(uint64_t* pairs, uint32_t n, uint32_t* ctr, cudaStr
 // auction: the reference's USE_AUCTION slot assignment instead of the greedy one.
 // child_pairs (optional): the records launch_hploc wrote for this BVH2; the
 // collapse then opens nodes through them and reads no BVH2 node.
+// lists (optional, with child_pairs): 24 bytes of scratch per primitive, for
+// small collapses.
 cudaError_t launch_bvh8(const Node2* bvh2, uint32_t n, Node8* out, uint32_t cap, uint32_t* prim_idx, uint64_t* pairs,
                         uint32_t* ctr, uint32_t* err, bool auction, cudaStream_t s,
-                        const ChildPair* child_pairs = nullptr);
+                        const ChildPair* child_pairs = nullptr, uint64_t* lists = nullptr);
 // ---------------------------------------------------------------- batches
 // The same stages over independent meshes laid end to end (MeshBatch in
 // common.cuh): one launch per stage for the whole batch.
@@ -282,10 +284,11 @@ cudaError_t launch_bvh8_batch_init(uint64_t* pairs, uint32_t slots, const MeshBa
 // off, off8, mesh_nodes and mesh_leaves advanced to the group's first mesh,
 // pairs to its first slot, ctr to its counters).  child_pairs: as for
 // launch_bvh8, the records launch_hploc_batch wrote (mesh m's at off[m]).
+// lists: as for launch_bvh8, only for a whole batch.
 cudaError_t launch_bvh8_batch(const Node2* bvh2, const MeshBatch& batch, uint32_t total, Node8* out, uint32_t slots,
                               uint32_t* prim_idx, uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
                               uint32_t* mesh_leaves, uint32_t* err, bool auction, cudaStream_t s,
-                              const ChildPair* child_pairs = nullptr);
+                              const ChildPair* child_pairs = nullptr, uint64_t* lists = nullptr);
 cudaError_t launch_batch_finalize(const MeshBatch& batch, const uint32_t* scene_ord, const uint32_t* mesh_nodes,
                                   const uint32_t* mesh_leaves, nxb_batch_mesh* out, cudaStream_t s);
 // One batched build's device memory (a single allocation carved into

@@ -644,10 +644,10 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
 // ---------------------------------------------------------------- groups
 // The same collapse with eight lanes per work item: lane c of a group holds
 // child c while the node is opened, and slot c when slots are assigned,
-// quantised and written.  What bounds it is the chain of levels: per level
-// 2.3 us of dependent record loads (up to seven), 0.6 us of assignment (0.8
-// in one lane), 0.3 us each for the poll and the allocation; the 2 us that
-// one lane takes to quantise and write a node are 0.15.
+// quantised and written.  What bounds it is the chain of levels: without
+// lists, per level 3.3 us of dependent record loads (up to eight), 1.3 us of
+// assignment and allocation and 0.6 us until a child is seen; the write, 2 us
+// in one lane, is 0.45 and off that chain.
 constexpr uint32_t kGroupsPerCta = kThreads / 8;
 
 // Monotone key of a cost for comparing as uint32; 0 for one that the
@@ -760,12 +760,78 @@ __device__ __forceinline__ uint32_t group_auction(const Box& pb, const Box& cb, 
     return mine;
 }
 
-template <typename Seg, bool AUCTION>
+// ---------------------------------------------------------------- lists
+// What a BVH8 node made of BVH2 node X would hold, for every internal X: its
+// up to eight children, by slot, as one thread per X opens and assigns them.
+// It does not depend on X's place in the BVH8, so it needs no order, and it
+// leaves the collapse a shorter chain per level: a level of opening and
+// assigning takes 5.3 us (seven dependent record loads 2.9, the assignment
+// 1.3), one that reads its list 1.7.  Four nodes of five are never made, so
+// this pays as long as the chain is what a collapse takes (takes_lists).
+// A list is three words of three 21-bit child indices (kNoChild: none); their
+// top bits hold the number of children less one (0: the BVH2 is corrupt).
+constexpr uint32_t kNoChild = (1u << 21) - 1u;
+
+template <typename Seg>
+__global__ __launch_bounds__(kThreads) void bvh8_lists_kernel(Seg seg, uint32_t records,
+                                                              const ChildPair* __restrict__ kids, uint64_t* lists) {
+    extern __shared__ uint32_t s_slots[];
+    const SlotTable<true> tab{s_slots};
+    const uint32_t r = blockIdx.x * kThreads + threadIdx.x;
+    if (r >= records) return;
+    MeshSpan me{0, 0, 0};
+    if constexpr (Seg::kBatch)
+        me = seg.of_prim(r);
+    else
+        me.count = seg.n;
+    if (r - me.start + 1 >= me.count) return;  // a mesh has a record less than primitives
+    const uint32_t node_limit = 2 * me.count - 1;
+    ChildPair kp = load_child_pair(kids + r);
+    Box nb = kp.l;
+    grow(nb, kp.r);
+    uint32_t inner = 0, count = 0, msb = 0;
+    bool ok = true;
+    while (true) {
+        ok = kp.li < node_limit && kp.ri < node_limit;
+        if (!ok) break;
+        const bool in0 = kp.li >= me.count, in1 = kp.ri >= me.count;
+        const bool first = !(half_area(kp.l) < half_area(kp.r));
+        // the smaller-area child takes the re-opened position
+        tab.put(msb, first ? kp.ri : kp.li, first ? kp.r : kp.l);
+        tab.put(count + 1, first ? kp.li : kp.ri, first ? kp.l : kp.r);
+        if (first ? in1 : in0) inner |= 1u << msb;
+        if (first ? in0 : in1) inner |= 1u << (count + 1);
+        count += 2;
+        if (inner == 0 || count == 8) break;
+        msb = 31 - __clz(inner);
+        inner &= ~(1u << msb);
+        count--;
+        kp = load_child_pair(kids + me.start + (tab.idx(msb) - me.count));
+    }
+    uint64_t w[3] = {~0ull >> 1, ~0ull >> 1, ~0ull >> 1};
+    if (ok) {
+        const uint32_t asg = greedy_assign(
+            make_float3(nb.mn.x + nb.mx.x, nb.mn.y + nb.mx.y, nb.mn.z + nb.mx.z), tab, count);
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+            const uint32_t a = nib(asg, i), sh = 21 * (i % 3);
+            const uint32_t id = a == 0xFu ? kNoChild : tab.idx(a);
+            w[i / 3] = (w[i / 3] & ~((uint64_t)kNoChild << sh)) | ((uint64_t)id << sh);
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 3; ++k) w[k] |= (uint64_t)(((count - 1) >> k) & 1u) << 63;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 3; ++k) lists[3ull * r + k] = w[k];
+}
+
+template <typename Seg, bool AUCTION, bool LISTS>
 __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __restrict__ b2, Seg seg, Node8* out,
                                                               uint32_t cap, uint32_t slots, uint32_t* prim_idx,
                                                               uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
                                                               uint32_t* mesh_leaves, uint32_t* err,
-                                                              const ChildPair* __restrict__ kids) {
+                                                              const ChildPair* __restrict__ kids,
+                                                              const uint64_t* __restrict__ lists) {
     __shared__ __align__(8) uint8_t s_rows[kGroupsPerCta][64];  // meta and quantised bytes of a group's node
     const uint32_t lane = lane_id(), sub = lane & 7u, base = lane & 24u;
     uint8_t* rows = s_rows[threadIdx.x >> 3];
@@ -825,6 +891,8 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
         uint32_t base8 = 0, cap8 = cap;
         bool internal = false;
         ChildPair kp;
+        Box nb;  // the node's box
+        uint64_t list = 0;
         if (ready) {
             if constexpr (Seg::kBatch) {
                 me = seg.span(owner_of(seg.off8, 0, seg.meshes - 1, b8i));
@@ -843,86 +911,108 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
             } else if (b2i >= 2 * me.count - 1 || b8i - base8 >= cap8 || b2i < me.count) {
                 if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
             } else {
-                kp = load_child_pair(kids + me.start + (b2i - me.count));
-                if (kp.li >= 2 * me.count - 1 || kp.ri >= 2 * me.count - 1) {
-                    if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
-                } else {
+                const uint32_t record = me.start + (b2i - me.count);
+                if constexpr (LISTS) {
+                    list = __ldg(lists + 3ull * record + sub / 3);
+                    nb = load_box(mb2, b2i);
                     internal = true;
+                } else {
+                    kp = load_child_pair(kids + record);
+                    internal = kp.li < 2 * me.count - 1 && kp.ri < 2 * me.count - 1;
+                    if (!internal && sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
                 }
             }
             if (!internal) slot = kInvalid;  // done (or reported); the item counts as finished
         }
-        const uint32_t node_limit = 2 * me.count - 1;
-        Box nb, cb;  // the node's box, this lane's child's box
-        nb.mn = nb.mx = cb.mn = cb.mx = make_float3(0.f, 0.f, 0.f);
-        uint32_t idx = 0, inner = 0, count = 0, msb = 0;
-        if (internal) {
-            nb = kp.l;
-            grow(nb, kp.r);
-        }
-        // open BVH2 nodes top-down until 8 children or no inner child; every
-        // lane of the group has the record, the two lanes concerned keep a child
-        bool open = internal;
-        while (__any_sync(kFullMask, open)) {
-            if (open) {
-                const bool in0 = kp.li >= me.count, in1 = kp.ri >= me.count;
-                const bool first = !(half_area(kp.l) < half_area(kp.r));
-                // the smaller-area child takes the re-opened position
-                const bool low = sub == msb, high = sub == count + 1;
-                if (low || high) {
-                    const bool right = low == first;
-                    cb = right ? kp.r : kp.l;
-                    idx = right ? kp.ri : kp.li;
-                    if (idx >= me.count) prefetch_l2(kids + me.start + (idx - me.count));
-                }
-                if (first ? in1 : in0) inner |= 1u << msb;
-                if (first ? in0 : in1) inner |= 1u << (count + 1);
-                count += 2;
-                if (inner == 0 || count == 8) {
-                    open = false;
-                } else {
-                    msb = 31 - __clz(inner);
-                    inner &= ~(1u << msb);
-                    count--;
-                }
+        uint32_t count = 0, child;  // of the node; in slot `sub`
+        bool used, is_inner;
+        Box qb;  // the child's box
+        if (!internal) nb.mn = nb.mx = make_float3(0.f, 0.f, 0.f);
+        if constexpr (LISTS) {
+            const uint32_t bits = __ballot_sync(kFullMask, list >> 63) >> base;
+            count = 1u + ((bits & 1u) | (bits >> 2 & 2u) | (bits >> 4 & 4u));
+            if (internal && count == 1) {
+                if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
+                internal = false;
+                slot = kInvalid;
             }
-            const uint32_t next = __shfl_sync(kFullMask, idx, msb, 8);
-            if (open) {
-                kp = load_child_pair(kids + me.start + (next - me.count));
-                if (kp.li >= node_limit || kp.ri >= node_limit) {  // corrupt BVH2: report, stop expanding
-                    if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
-                    inner |= 1u << msb;
-                    count++;
-                    open = false;
-                }
-            }
-        }
-        const float3 pc = make_float3(nb.mn.x + nb.mx.x, nb.mn.y + nb.mx.y, nb.mn.z + nb.mx.z);
-        const float3 off = make_float3(pc.x - (cb.mx.x + cb.mn.x), pc.y - (cb.mx.y + cb.mn.y),
-                                       pc.z - (cb.mx.z + cb.mn.z));
-        uint32_t mine;  // the child of slot `sub`
-        if constexpr (AUCTION) {
-            mine = group_auction(nb, cb, max(count, 1u), internal, sub, base);
-            const bool failed = mine == kFallback;
-            if (__any_sync(kFullMask, failed)) {
-                const uint32_t g = group_greedy(off, count, sub);
-                if (failed) mine = g;
-            }
+            child = (uint32_t)(list >> (21 * (sub % 3))) & kNoChild;
+            used = internal && child != kNoChild;
+            is_inner = used && child >= me.count;
+            qb = nb;
+            if (used) qb = load_box(mb2, child);
         } else {
-            mine = group_greedy(off, count, sub);
+            const uint32_t node_limit = 2 * me.count - 1;
+            Box cb;  // this lane's child's box
+            cb.mn = cb.mx = make_float3(0.f, 0.f, 0.f);
+            uint32_t idx = 0, inner = 0, msb = 0;
+            if (internal) {
+                nb = kp.l;
+                grow(nb, kp.r);
+            }
+            // open BVH2 nodes top-down until 8 children or no inner child; every
+            // lane of the group has the record, the two lanes concerned keep a child
+            bool open = internal;
+            while (__any_sync(kFullMask, open)) {
+                if (open) {
+                    const bool in0 = kp.li >= me.count, in1 = kp.ri >= me.count;
+                    const bool first = !(half_area(kp.l) < half_area(kp.r));
+                    // the smaller-area child takes the re-opened position
+                    const bool low = sub == msb, high = sub == count + 1;
+                    if (low || high) {
+                        const bool right = low == first;
+                        cb = right ? kp.r : kp.l;
+                        idx = right ? kp.ri : kp.li;
+                        if (idx >= me.count) prefetch_l2(kids + me.start + (idx - me.count));
+                    }
+                    if (first ? in1 : in0) inner |= 1u << msb;
+                    if (first ? in0 : in1) inner |= 1u << (count + 1);
+                    count += 2;
+                    if (inner == 0 || count == 8) {
+                        open = false;
+                    } else {
+                        msb = 31 - __clz(inner);
+                        inner &= ~(1u << msb);
+                        count--;
+                    }
+                }
+                const uint32_t next = __shfl_sync(kFullMask, idx, msb, 8);
+                if (open) {
+                    kp = load_child_pair(kids + me.start + (next - me.count));
+                    if (kp.li >= node_limit || kp.ri >= node_limit) {  // corrupt BVH2: report, stop expanding
+                        if (sub == 0) set_error(err, NXB_DEVERR_BVH8_OVERFLOW);
+                        inner |= 1u << msb;
+                        count++;
+                        open = false;
+                    }
+                }
+            }
+            const float3 pc = make_float3(nb.mn.x + nb.mx.x, nb.mn.y + nb.mx.y, nb.mn.z + nb.mx.z);
+            const float3 off = make_float3(pc.x - (cb.mx.x + cb.mn.x), pc.y - (cb.mx.y + cb.mn.y),
+                                           pc.z - (cb.mx.z + cb.mn.z));
+            uint32_t mine;  // the child of slot `sub`
+            if constexpr (AUCTION) {
+                mine = group_auction(nb, cb, max(count, 1u), internal, sub, base);
+                const bool failed = mine == kFallback;
+                if (__any_sync(kFullMask, failed)) {
+                    const uint32_t g = group_greedy(off, count, sub);
+                    if (failed) mine = g;
+                }
+            } else {
+                mine = group_greedy(off, count, sub);
+            }
+            used = internal && mine != 0xFu;
+            is_inner = used && ((inner >> mine) & 1u);
+            child = __shfl_sync(kFullMask, idx, mine, 8);
+            qb.mn.x = __shfl_sync(kFullMask, cb.mn.x, mine, 8);
+            qb.mn.y = __shfl_sync(kFullMask, cb.mn.y, mine, 8);
+            qb.mn.z = __shfl_sync(kFullMask, cb.mn.z, mine, 8);
+            qb.mx.x = __shfl_sync(kFullMask, cb.mx.x, mine, 8);
+            qb.mx.y = __shfl_sync(kFullMask, cb.mx.y, mine, 8);
+            qb.mx.z = __shfl_sync(kFullMask, cb.mx.z, mine, 8);
         }
-        const bool used = internal && mine != 0xFu;
-        const bool is_inner = used && ((inner >> mine) & 1u);
         const uint32_t imask = __ballot_sync(kFullMask, is_inner) >> base & 0xFFu;
         const uint32_t lmask = __ballot_sync(kFullMask, used && !is_inner) >> base & 0xFFu;
-        const uint32_t child = __shfl_sync(kFullMask, idx, mine, 8);
-        Box qb;
-        qb.mn.x = __shfl_sync(kFullMask, cb.mn.x, mine, 8);
-        qb.mn.y = __shfl_sync(kFullMask, cb.mn.y, mine, 8);
-        qb.mn.z = __shfl_sync(kFullMask, cb.mn.z, mine, 8);
-        qb.mx.x = __shfl_sync(kFullMask, cb.mx.x, mine, 8);
-        qb.mx.y = __shfl_sync(kFullMask, cb.mx.y, mine, 8);
-        qb.mx.z = __shfl_sync(kFullMask, cb.mx.z, mine, 8);
         // allocation of work slots (one mesh: = BVH8 nodes) and leaves, one
         // atomic for the warp's four groups
         const uint32_t ic = internal ? (uint32_t)__popc(imask) : 0u;
@@ -999,35 +1089,54 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
     }
 }
 
-template <typename Seg, bool AUCTION>
+template <typename Seg, bool AUCTION, bool LISTS = false>
 cudaError_t launch_group(const Node2* bvh2, Seg seg, uint32_t items, Node8* out, uint32_t cap, uint32_t slots,
                          uint32_t* prim_idx, uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
-                         uint32_t* mesh_leaves, uint32_t* err, cudaStream_t s, const ChildPair* kids) {
+                         uint32_t* mesh_leaves, uint32_t* err, cudaStream_t s, const ChildPair* kids,
+                         uint64_t* lists = nullptr) {
+    if constexpr (LISTS) {
+        const cudaError_t e = once_per_device([] {
+            return cudaFuncSetAttribute(bvh8_lists_kernel<Seg>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                        cudaSharedmemCarveoutMaxShared);
+        });
+        if (e) return e;
+        bvh8_lists_kernel<Seg>
+            <<<(items + kThreads - 1) / kThreads, kThreads, (kSlotSmem<true>), s>>>(seg, items, kids, lists);
+    }
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bvh8_group_kernel<Seg, AUCTION>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bvh8_group_kernel<Seg, AUCTION, LISTS>, kThreads, 0);
     // Groups that wait poll the pending counter, and too many of them saturate
-    // its L2 line: 65,536 triangles take 104 us with a group per item, 70 with
-    // one per 16 primitives; 256,000 take 117 us at 8 CTAs per SM, 96 at 4.
-    // Auctions keep their groups busy: 1.05M triangles 631 us at 4, 512 at 8.
+    // its L2 line.  With lists, a group per 16 primitives and, above 4,096
+    // groups, per 32: 1,021 triangles 27 us (33 at 32), 65,536 39 (47 at 8),
+    // 128,000 49 (53 at 16), 256,000 68 (70); at 8 CTAs per SM instead of 4,
+    // 256,000 take 109 and 512,000 137 (98).  Auctions keep their groups
+    // busy: 1.05M triangles 631 us at 4, 512 at 8.
     if (!AUCTION) per_sm = std::min(per_sm, 4);
     if (per_sm < 1) per_sm = 1;
-    const uint32_t want = (items + 16 * kGroupsPerCta - 1) / (16 * kGroupsPerCta);
+    uint32_t groups = (items + 15) / 16;
+    if (LISTS) groups = std::max(std::min(groups, 4096u), (items + 31) / 32);
+    const uint32_t want = (groups + kGroupsPerCta - 1) / kGroupsPerCta;
     const uint32_t grid = std::max(1u, std::min(want, (uint32_t)(device_info().sms * per_sm)));
-    bvh8_group_kernel<Seg, AUCTION><<<grid, kThreads, 0, s>>>(bvh2, seg, out, cap, slots, prim_idx, pairs, ctr,
-                                                              mesh_nodes, mesh_leaves, err, kids);
+    bvh8_group_kernel<Seg, AUCTION, LISTS><<<grid, kThreads, 0, s>>>(bvh2, seg, out, cap, slots, prim_idx, pairs, ctr,
+                                                                     mesh_nodes, mesh_leaves, err, kids, lists);
     return cudaGetLastError();
 }
 
 // Which form of the collapse a build with child-pair records takes.  Small
-// greedy collapses are a chain of levels (12 at 65,536 triangles), where a
-// group gets an item done sooner and no item waits for the other 31 of its
-// warp; large ones are bound by random memory traffic, where one lane per
-// item keeps eight times the items in flight.  Measured (one lane / a group
-// per item): 16,411 clustered boxes 98 / 76 us, 65,536 soup triangles
-// 100 / 70, 256,000 129 / 96, 512,000 143 / 129, 1.0M 170 / 184, 4.19M sphere
-// 254 / 473.  An auction is a long sequential search per item, eight times
-// shorter in a group: 1.05M sphere 1042 / 512 us.
+// greedy collapses are a chain of levels (12 at 65,536 triangles), which
+// lists make shortest; large ones are bound by random memory traffic, where
+// one lane per item keeps eight times the items in flight, and where the
+// lists of nodes never made cost more than the chain.  Measured (one lane / a
+// group per item / a group with lists): 1,021 soup triangles - / 45 / 27 us,
+// 16,411 clustered boxes 98 / 76 / 37, 65,536 soup 100 / 70 / 39, 256,000
+// 129 / 100 / 72, 512,000 143 / 131 / 98, 1.0M 154 / 184 / 160, 1.0M
+// clustered 180 / - / 166, 4.19M sphere 237 / 473 / -.  Groups of a batch
+// that overlaps its stages have no room for lists.  An auction is a long
+// sequential search per item, eight times shorter in a group: 1.05M sphere
+// 1042 / 512 us; the lists would take it for every node.
+constexpr uint32_t kListMaxPrims = 800000;  // at most 2^20: a list holds 21-bit indices
 constexpr uint32_t kGroupMaxPrims = 600000;
+inline bool takes_lists(uint32_t prims, bool auction) { return !auction && prims <= kListMaxPrims; }
 inline bool takes_groups(uint32_t prims, bool auction) { return auction || prims <= kGroupMaxPrims; }
 
 template <typename Seg, bool AUCTION, bool KIDS>
@@ -1098,15 +1207,15 @@ cudaError_t launch_bvh8_init(uint64_t* pairs, uint32_t n, uint32_t* ctr, cudaStr
 }
 
 cudaError_t launch_bvh8(const Node2* bvh2, uint32_t n, Node8* out, uint32_t cap, uint32_t* prim_idx, uint64_t* pairs,
-                        uint32_t* ctr, uint32_t* err, bool auction, cudaStream_t s, const ChildPair* child_pairs) {
+                        uint32_t* ctr, uint32_t* err, bool auction, cudaStream_t s, const ChildPair* child_pairs,
+                        uint64_t* lists) {
     const SingleMesh seg{n};
-    if (child_pairs && takes_groups(n, auction)) {
-        if (auction)
-            return launch_group<SingleMesh, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr,
-                                                  err, s, child_pairs);
-        return launch_group<SingleMesh, false>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr, err,
-                                               s, child_pairs);
-    }
+    if (child_pairs && lists && takes_lists(n, auction))
+        return launch_group<SingleMesh, false, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr,
+                                                     nullptr, err, s, child_pairs, lists);
+    if (child_pairs && auction)
+        return launch_group<SingleMesh, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr, err,
+                                              s, child_pairs);
     if (child_pairs)
         return launch_wide<SingleMesh, false, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr,
                                                     nullptr, err, s, child_pairs);
@@ -1127,7 +1236,10 @@ cudaError_t launch_bvh8_batch_init(uint64_t* pairs, uint32_t slots, const MeshBa
 cudaError_t launch_bvh8_batch(const Node2* bvh2, const MeshBatch& batch, uint32_t total, Node8* out, uint32_t slots,
                               uint32_t* prim_idx, uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
                               uint32_t* mesh_leaves, uint32_t* err, bool auction, cudaStream_t s,
-                              const ChildPair* child_pairs) {
+                              const ChildPair* child_pairs, uint64_t* lists) {
+    if (child_pairs && lists && takes_lists(total, auction))
+        return launch_group<MeshBatch, false, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr,
+                                                    mesh_nodes, mesh_leaves, err, s, child_pairs, lists);
     if (child_pairs && takes_groups(total, auction)) {
         if (auction)
             return launch_group<MeshBatch, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
