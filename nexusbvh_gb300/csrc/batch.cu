@@ -167,9 +167,10 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
     const bool seg = !local && segment_sort_takes(a.total, a.meshes, a.lookback,
                                                   a.lookback_words_per_pass * kMaxSortPasses, &segments);
     const SortPlan plan = local || seg ? SortPlan{} : make_sort_plan(2, 32 + a.mesh_bits, t.digit_bits);
-    NXB_TRY(cudaMemsetAsync(a.zero_begin, 0, a.zero_bytes, s));
+    const BatchBegin begin{reinterpret_cast<uint4*>(a.zero_begin), a.zero_bytes / 16, a.tile_rng, t.block, a.total,
+                           a.pairs, a.slots, a.ctr8, a.mesh_nodes, a.mesh_leaves, g};
+    NXB_TRY(launch_batch_begin(begin, mb, s));
     if (a.total > 0) {
-        NXB_TRY(launch_batch_tile_ranges(mb, a.total, t.block, a.tile_rng, s));
         NXB_TRY(launch_batch_bounds(prims, type, mb, a.total, a.bvh2, a.scene_ord, t.block, a.tile_rng, s));
         MortonFused f{};
         f.zero_ptr = a.lookback;
@@ -197,7 +198,6 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
                                      a.ctrl->tile_ctr + p, &a.ctrl->error_word, s));
         }
     }
-    NXB_TRY(launch_bvh8_batch_init(a.pairs, a.slots, mb, a.ctr8, a.mesh_nodes, a.mesh_leaves, g, s));
     if (a.total > 0) {
         const bool in_a = (plan.passes % 2) == 0;
         uint64_t* keys = in_a ? a.keys_a : a.keys_b;

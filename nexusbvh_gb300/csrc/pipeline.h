@@ -5,6 +5,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <mutex>
 
 #include "../../include/nxb_gb300.h"
@@ -105,6 +106,23 @@ cudaError_t once_per_device(F set) {
     if (dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
     std::call_once(once[dev], [&] { result[dev] = set(); });
     return result[dev];
+}
+
+// CTAs of a kernel that an SM holds, at least 1 (asked once per device: the
+// question takes as long as a launch).
+template <auto* Kernel>
+int resident_ctas(int threads, size_t smem) {
+    constexpr int kMaxDev = 64;
+    static std::atomic<int> found[kMaxDev];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return 1;
+    int n = found[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, threads, smem);
+        n = n < 1 ? 1 : n;
+        found[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 struct DeviceInfo {
@@ -239,10 +257,7 @@ cudaError_t launch_bvh8(const Node2* bvh2, uint32_t n, Node8* out, uint32_t cap,
 // common.cuh): one launch per stage for the whole batch.
 // scene_ord: 6 words per mesh, zero on entry.
 // block: CTA size of the two tile kernels (128, 256 or 512).
-// tile_rng: the first and last mesh of every `block`-primitive tile
-// (launch_batch_tile_ranges with the same block).
-cudaError_t launch_batch_tile_ranges(const MeshBatch& batch, uint32_t total, uint32_t block, uint2* tile_rng,
-                                     cudaStream_t s);
+// tile_rng: the first and last mesh of every `block`-primitive tile.
 cudaError_t launch_batch_bounds(const void* prims, int prim_type, const MeshBatch& batch, uint32_t total,
                                 Node2* nodes, uint32_t* scene_ord, uint32_t block, const uint2* tile_rng,
                                 cudaStream_t s);
@@ -275,11 +290,21 @@ struct MeshGroups {
     uint32_t prim[kMaxMeshGroups + 1];
     uint32_t slot[kMaxMeshGroups + 1];
 };
-// pairs: `slots` = off8[meshes] uint64 slots; ctr: kBvh8CtrWords words per
-// group.  Seeds every group's queue with the root items of its meshes.
-cudaError_t launch_bvh8_batch_init(uint64_t* pairs, uint32_t slots, const MeshBatch& batch, uint32_t* ctr,
-                                   uint32_t* mesh_nodes, uint32_t* mesh_leaves, const MeshGroups& groups,
-                                   cudaStream_t s);
+// What a batched build begins with, in one launch: words cleared, tile_rng,
+// and the BVH8 work queue (pairs: `slots` = off8[meshes] slots; ctr:
+// kBvh8CtrWords words per group; every group's queue is seeded with the root
+// items of its meshes) with the per-mesh node and leaf counts.
+struct BatchBegin {
+    uint4* zero;
+    size_t zero_vec4;
+    uint2* tile_rng;
+    uint32_t block, total;
+    uint64_t* pairs;
+    uint32_t slots;
+    uint32_t *ctr, *mesh_nodes, *mesh_leaves;
+    MeshGroups groups;
+};
+cudaError_t launch_batch_begin(const BatchBegin& b, const MeshBatch& batch, cudaStream_t s);
 // The collapse of the meshes of `batch` (a whole batch, or one group's view:
 // off, off8, mesh_nodes and mesh_leaves advanced to the group's first mesh,
 // pairs to its first slot, ctr to its counters).  child_pairs: as for

@@ -307,14 +307,47 @@ __device__ __forceinline__ uint2 tile_meshes(const MeshBatch& b, uint32_t first,
     return make_uint2(lo, owner_of(b.off, lo, b.meshes - 1, last));
 }
 
-// The mesh range of every T-primitive tile, one thread per tile, so that the
-// tile kernels read it with one load instead of searching in one thread
-// while the others wait at a barrier.
-__global__ void batch_tile_ranges_kernel(MeshBatch batch, uint32_t total, uint32_t T, uint2* rng) {
-    const uint32_t tiles = (total + T - 1) / T;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < tiles; t += gridDim.x * blockDim.x) {
-        const uint32_t first = t * T;
-        rng[t] = tile_meshes(batch, first, min(first + T, total) - 1);
+// The mesh range of every tile (one thread per tile, so that the tile kernels
+// read it with one load instead of searching in one thread while the others
+// wait at a barrier), and everything else a batch needs at its start.  One
+// launch: a memset and two kernels took 8 us of a small batch, and as much of
+// the thread that launches them.
+__global__ void batch_begin_kernel(BatchBegin b, MeshBatch batch) {
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (size_t i = i0; i < b.zero_vec4; i += stride) b.zero[i] = make_uint4(0, 0, 0, 0);
+    const uint32_t tiles = (b.total + b.block - 1) / b.block;
+    for (uint32_t t = i0; t < tiles; t += stride) {
+        const uint32_t first = t * b.block;
+        b.tile_rng[t] = tile_meshes(batch, first, min(first + b.block, b.total) - 1);
+    }
+    for (uint32_t i = i0; i < b.slots; i += stride) {
+        // group g's queue is slots [slot[g], slot[g+1]); its first entries
+        // are the root items of the group's meshes (empty meshes too, they
+        // finish without output)
+        uint32_t g = 0;
+        while (g + 1 < b.groups.count && i >= b.groups.slot[g + 1]) ++g;
+        const uint32_t local = i - b.groups.slot[g];
+        uint64_t v = ~0ull;
+        if (local < b.groups.mesh[g + 1] - b.groups.mesh[g]) {
+            const uint32_t m = b.groups.mesh[g] + local;
+            const MeshSpan me = batch.span(m);
+            const uint32_t root = me.count ? 2 * me.count - 2 : 0u;
+            v = ((uint64_t)root << 32) | __ldg(batch.off8 + m);
+        }
+        if (i < batch.meshes) {
+            const MeshSpan me = batch.span(i);
+            b.mesh_nodes[i] = me.count ? 1u : 0u;
+            b.mesh_leaves[i] = 0;
+        }
+        b.pairs[i] = v;
+    }
+    if (i0 < b.groups.count) {
+        uint32_t* c = b.ctr + i0 * kBvh8CtrWords;
+        const uint32_t meshes = b.groups.mesh[i0 + 1] - b.groups.mesh[i0];
+        c[kBvh8Claim] = 0;
+        c[kBvh8Alloc] = meshes;  // a batch counts nodes and leaves per mesh
+        c[kBvh8Leaves] = 0;
+        c[kBvh8Pending] = meshes;
     }
 }
 
@@ -703,11 +736,9 @@ void bounds_t(const void* prims, int prim_type, const MeshBatch& batch, uint32_t
                                                                      scene_ord, aligned, tile_rng);
 }
 
-cudaError_t launch_batch_tile_ranges(const MeshBatch& batch, uint32_t total, uint32_t block, uint2* tile_rng,
-                                     cudaStream_t s) {
-    const uint32_t tiles = (total + block - 1) / block;
-    const uint32_t grid = std::max(1u, std::min<uint32_t>((tiles + 255) / 256, (uint32_t)device_info().sms * 4));
-    batch_tile_ranges_kernel<<<grid, 256, 0, s>>>(batch, total, block, tile_rng);
+cudaError_t launch_batch_begin(const BatchBegin& b, const MeshBatch& batch, cudaStream_t s) {
+    const uint32_t grid = std::max(1u, std::min<uint32_t>((b.slots + 255) / 256, (uint32_t)device_info().sms * 8));
+    batch_begin_kernel<<<grid, 256, 0, s>>>(b, batch);
     return cudaGetLastError();
 }
 

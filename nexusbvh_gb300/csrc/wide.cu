@@ -279,41 +279,6 @@ __global__ void bvh8_init_kernel(uint64_t* pairs, uint32_t n, uint32_t* ctr) {
     if (i0 == 0) bvh8_queue_counters(ctr);
 }
 
-// Batched form: slot m holds the root item of mesh m (empty meshes too,
-// they finish without output); per-mesh node and leaf counters.
-__global__ void bvh8_batch_init_kernel(uint64_t* pairs, uint32_t slots, MeshBatch batch, uint32_t* ctr,
-                                       uint32_t* mesh_nodes, uint32_t* mesh_leaves, MeshGroups groups) {
-    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    for (uint32_t i = i0; i < slots; i += gridDim.x * blockDim.x) {
-        // group g's queue is slots [slot[g], slot[g+1]); its first entries
-        // are the root items of the group's meshes
-        uint32_t g = 0;
-        while (g + 1 < groups.count && i >= groups.slot[g + 1]) ++g;
-        const uint32_t local = i - groups.slot[g];
-        uint64_t v = ~0ull;
-        if (local < groups.mesh[g + 1] - groups.mesh[g]) {
-            const uint32_t m = groups.mesh[g] + local;
-            const MeshSpan me = batch.span(m);
-            const uint32_t root = me.count ? 2 * me.count - 2 : 0u;
-            v = ((uint64_t)root << 32) | __ldg(batch.off8 + m);
-        }
-        if (i < batch.meshes) {
-            const MeshSpan me = batch.span(i);
-            mesh_nodes[i] = me.count ? 1u : 0u;
-            mesh_leaves[i] = 0;
-        }
-        pairs[i] = v;
-    }
-    if (i0 < groups.count) {
-        uint32_t* c = ctr + i0 * kBvh8CtrWords;
-        const uint32_t meshes = groups.mesh[i0 + 1] - groups.mesh[i0];
-        c[kBvh8Claim] = 0;
-        c[kBvh8Alloc] = meshes;  // a batch counts nodes and leaves per mesh
-        c[kBvh8Leaves] = 0;
-        c[kBvh8Pending] = meshes;
-    }
-}
-
 // A warp's account with the count of allocated-but-unfinished items: what it
 // allocates is added before the items are handed out, what it has finished
 // beyond that is kept as a credit for the items that it allocates next, and
@@ -1103,8 +1068,7 @@ cudaError_t launch_group(const Node2* bvh2, Seg seg, uint32_t items, Node8* out,
         bvh8_lists_kernel<Seg>
             <<<(items + kThreads - 1) / kThreads, kThreads, (kSlotSmem<true>), s>>>(seg, items, kids, lists);
     }
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bvh8_group_kernel<Seg, AUCTION, LISTS>, kThreads, 0);
+    int per_sm = resident_ctas<bvh8_group_kernel<Seg, AUCTION, LISTS>>(kThreads, 0);
     // Groups that wait poll the pending counter, and too many of them saturate
     // its L2 line.  With lists, a group per 16 primitives and, above 4,096
     // groups, per 32: 1,021 triangles 27 us (33 at 32), 65,536 39 (47 at 8),
@@ -1112,7 +1076,6 @@ cudaError_t launch_group(const Node2* bvh2, Seg seg, uint32_t items, Node8* out,
     // 256,000 take 109 and 512,000 137 (98).  Auctions keep their groups
     // busy: 1.05M triangles 631 us at 4, 512 at 8.
     if (!AUCTION) per_sm = std::min(per_sm, 4);
-    if (per_sm < 1) per_sm = 1;
     uint32_t groups = (items + 15) / 16;
     if (LISTS) groups = std::max(std::min(groups, 4096u), (items + 31) / 32);
     const uint32_t want = (groups + kGroupsPerCta - 1) / kGroupsPerCta;
@@ -1149,9 +1112,7 @@ cudaError_t configure_smem() {
 
 template <typename Seg, bool AUCTION, bool KIDS>
 uint32_t persistent_grid(uint32_t items) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bvh8_kernel<Seg, AUCTION, KIDS>, kThreads, kSlotSmem<KIDS>);
-    if (per_sm < 1) per_sm = 1;
+    const int per_sm = resident_ctas<bvh8_kernel<Seg, AUCTION, KIDS>>(kThreads, kSlotSmem<KIDS>);
     const uint32_t want = (items + kThreads - 1) / kThreads;
     return std::max(1u, std::min(want, (uint32_t)(device_info().sms * per_sm)));
 }
@@ -1223,14 +1184,6 @@ cudaError_t launch_bvh8(const Node2* bvh2, uint32_t n, Node8* out, uint32_t cap,
         return launch_wide<SingleMesh, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr, err,
                                              s);
     return launch_wide<SingleMesh, false>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr, err, s);
-}
-
-cudaError_t launch_bvh8_batch_init(uint64_t* pairs, uint32_t slots, const MeshBatch& batch, uint32_t* ctr,
-                                   uint32_t* mesh_nodes, uint32_t* mesh_leaves, const MeshGroups& groups,
-                                   cudaStream_t s) {
-    uint32_t grid = std::max(1u, std::min<uint32_t>((slots + 255) / 256, (uint32_t)device_info().sms * 8));
-    bvh8_batch_init_kernel<<<grid, 256, 0, s>>>(pairs, slots, batch, ctr, mesh_nodes, mesh_leaves, groups);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_bvh8_batch(const Node2* bvh2, const MeshBatch& batch, uint32_t total, Node8* out, uint32_t slots,
