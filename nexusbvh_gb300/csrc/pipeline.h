@@ -125,6 +125,19 @@ int resident_ctas(int threads, size_t smem) {
     return n;
 }
 
+// Loads kernels on the current device (the runtime loads each on first use).
+template <typename... K>
+cudaError_t load_kernels(K*... kernels) {
+    cudaFuncAttributes a;
+    cudaError_t e = cudaSuccess;
+    ((e = e ? e : cudaFuncGetAttributes(&a, kernels)), ...);
+    return e;
+}
+// Those that builds of a server's default radius take only at some sizes.
+cudaError_t load_setup_kernels();
+cudaError_t load_sort_kernels();
+cudaError_t load_collapse_kernels();
+
 struct DeviceInfo {
     int sms;
     int max_smem_optin;
@@ -390,6 +403,18 @@ void batch_groups(const uint32_t* h_off, const uint32_t* h_off8, uint32_t meshes
 nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type type, const BatchTuning& t,
                          uint32_t* h_err, cudaStream_t s, const MeshGroups* groups = nullptr,
                          const BatchFork* fork = nullptr);
+// Where the meshes of a batch come from and go to, one entry per mesh in
+// memory that the device can read: gather lays the primitives of the meshes
+// that have a source end to end at dst, scatter copies each mesh's BVH8 nodes
+// and primIdx out of a built arena.
+struct BatchPlaces {
+    const void* prims;  // null: not gathered
+    Node8* nodes;
+    uint32_t* prim_idx;
+};
+cudaError_t launch_batch_gather(const BatchArena& a, const BatchPlaces* places, nxb_prim_type type, void* dst,
+                                cudaStream_t s);
+cudaError_t launch_batch_scatter(const BatchArena& a, const BatchPlaces* places, cudaStream_t s);
 // ---------------------------------------------------------------- eval
 cudaError_t launch_bvh2_cost(const Node2* nodes, uint32_t count, const nxb_aabb* root, float* cost, cudaStream_t s);
 cudaError_t launch_bvh8_cost(const Node8* nodes, uint32_t count, const nxb_aabb* root, float* cost, cudaStream_t s);

@@ -1311,6 +1311,26 @@ cudaError_t launch_local_sort_batch(uint64_t* keys, uint32_t* vals, const MeshBa
     });
 }
 
+cudaError_t load_sort_kernels() {
+    cudaError_t e = load_kernels(bucket_sort_kernel, sort_fallback_kernel<uint64_t>, segment_prepare_kernel,
+                                 segment_pass_kernel<true, false>, segment_pass_kernel<false, false>,
+                                 segment_pass_kernel<false, true>);
+    for (int form = 0; form < 4 && !e; ++form)
+        e = load_kernels(onesweep_of<uint32_t, kRadixBits>(form & 1, form & 2),
+                         onesweep_of<uint64_t, kRadixBits>(form & 1, form & 2),
+                         onesweep_of<uint64_t, kMaxRadixBits>(form & 1, form & 2));
+    auto local = [&](auto kpt) {
+        constexpr int k = decltype(kpt)::value;
+        if (!e)
+            e = load_kernels(sort_cluster_kernel<uint32_t, kLocalBits32, k>, sort_cluster_kernel<uint64_t, kLocalBits64, k>,
+                             sort_cluster_batch_kernel<kLocalBits32, k>);
+    };
+    local(std::integral_constant<int, 2>());
+    local(std::integral_constant<int, 4>());
+    local(std::integral_constant<int, 8>());
+    return e;
+}
+
 // Batches whose meshes have 1,536 primitives or more on average: with more
 // meshes than that, their counts and look-back words don't fit the memory
 // that the passes over mesh and code need.  The line costs nothing: one mesh

@@ -626,6 +626,46 @@ __global__ void batch_finalize_kernel(MeshBatch batch, const uint32_t* scene_ord
     }
 }
 
+// Copies `count` elements with the threads of the CTAs of one grid row, four
+// loads in flight per thread.
+template <typename T>
+__device__ __forceinline__ void copy_row(T* __restrict__ dst, const T* __restrict__ src, uint32_t count) {
+    const uint32_t stride = gridDim.x * blockDim.x;
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + 3 * stride < count; i += 4 * stride) {
+        const T a = src[i], b = src[i + stride], c = src[i + 2 * stride], d = src[i + 3 * stride];
+        dst[i] = a;
+        dst[i + stride] = b;
+        dst[i + 2 * stride] = c;
+        dst[i + 3 * stride] = d;
+    }
+    for (; i < count; i += stride) dst[i] = src[i];
+}
+
+// A grid row per mesh (or several meshes in turn).
+__global__ void batch_gather_kernel(MeshBatch batch, const BatchPlaces* places, uint32_t words, uint32_t* dst) {
+    for (uint32_t m = blockIdx.y; m < batch.meshes; m += gridDim.y) {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(places[m].prims);
+        const MeshSpan me = batch.span(m);
+        if (src)  // aligned to words only
+            for (uint32_t k = 0; k < words; ++k)
+                copy_row(dst + (size_t)words * me.start + (size_t)k * me.count, src + (size_t)k * me.count, me.count);
+    }
+}
+
+__global__ void batch_scatter_kernel(MeshBatch batch, const BatchPlaces* places, const uint32_t* mesh_nodes,
+                                     const Node8* nodes, const uint32_t* prim_idx) {
+    for (uint32_t m = blockIdx.y; m < batch.meshes; m += gridDim.y) {
+        const BatchPlaces to = places[m];
+        const MeshSpan me = batch.span(m);
+        const uint32_t first = __ldg(batch.off8 + m), cap = __ldg(batch.off8 + m + 1) - first;
+        const uint32_t count = min(__ldg(mesh_nodes + m), cap);
+        copy_row(reinterpret_cast<uint4*>(to.nodes), reinterpret_cast<const uint4*>(nodes + first),
+                 count * (uint32_t)(sizeof(Node8) / sizeof(uint4)));
+        copy_row(to.prim_idx, prim_idx + me.start, me.count);
+    }
+}
+
 PassDigits to_digits(const SortPlan& plan) {
     PassDigits pd{};
     pd.passes = plan.passes;
@@ -742,6 +782,28 @@ cudaError_t launch_batch_begin(const BatchBegin& b, const MeshBatch& batch, cuda
     return cudaGetLastError();
 }
 
+// Grid rows for the meshes and enough CTAs in each to fill the SMs, or for the
+// largest mesh.
+dim3 rows_of(const BatchArena& a) {
+    const uint32_t rows = std::min(a.meshes, 4096u);
+    const uint32_t ctas = (uint32_t)device_info().sms * 8, most = (a.max_mesh + 1023) / 1024;
+    return dim3(std::max(1u, std::min((ctas + rows - 1) / rows, most)), rows);
+}
+
+cudaError_t launch_batch_gather(const BatchArena& a, const BatchPlaces* places, nxb_prim_type type, void* dst,
+                                cudaStream_t s) {
+    batch_gather_kernel<<<rows_of(a), 256, 0, s>>>(MeshBatch{a.off, a.off8, a.meshes}, places,
+                                                   type == NXB_PRIM_TRIANGLE ? 9u : 6u,
+                                                   reinterpret_cast<uint32_t*>(dst));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_batch_scatter(const BatchArena& a, const BatchPlaces* places, cudaStream_t s) {
+    batch_scatter_kernel<<<rows_of(a), 256, 0, s>>>(MeshBatch{a.off, a.off8, a.meshes}, places, a.mesh_nodes, a.bvh8,
+                                                    a.prim_idx);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_batch_bounds(const void* prims, int prim_type, const MeshBatch& batch, uint32_t total,
                                 Node2* nodes, uint32_t* scene_ord, uint32_t block, const uint2* tile_rng,
                                 cudaStream_t s) {
@@ -813,6 +875,12 @@ cudaError_t launch_batch_finalize(const MeshBatch& batch, const uint32_t* scene_
     const uint32_t grid = std::max(1u, std::min<uint32_t>((batch.meshes + 255) / 256, 1024u));
     batch_finalize_kernel<<<grid, 256, 0, s>>>(batch, scene_ord, mesh_nodes, mesh_leaves, out);
     return cudaGetLastError();
+}
+
+cudaError_t load_setup_kernels() {
+    return load_kernels(morton_kernel<uint32_t, true, 4>, morton_kernel<uint64_t, true, 4, 1 << kMaxRadixBits>,
+                        batch_morton_kernel<true, 256, 5>, batch_morton_kernel<true, 256>, segment_morton_kernel<256>,
+                        batch_gather_kernel, batch_scatter_kernel);
 }
 
 }  // namespace nxb

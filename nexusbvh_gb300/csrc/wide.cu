@@ -1210,4 +1210,8 @@ cudaError_t launch_bvh8_batch(const Node2* bvh2, const MeshBatch& batch, uint32_
                                          mesh_leaves, err, s);
 }
 
+cudaError_t load_collapse_kernels() {
+    return load_kernels(bvh8_kernel<SingleMesh, false, true>, bvh8_kernel<MeshBatch, false, true>);
+}
+
 }  // namespace nxb
