@@ -149,6 +149,14 @@ __device__ __forceinline__ uint32_t atom_exch_acq_rel(uint32_t* p, uint32_t v) {
 }
 
 // Box of a BVH2 node read through L2 (data written by other CTAs).
+// For kernels launched by launch_after (pipeline.h): waits for the kernel
+// before in the stream, which has then finished and whose writes are seen,
+// and lets the one after be set up meanwhile.  Nothing another kernel writes
+// or reads is touched before it.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ Box load_box_cg(const Node2* nodes, uint32_t i) {
     const float4* p = reinterpret_cast<const float4*>(nodes + i);
     float4 a = __ldcg(p);

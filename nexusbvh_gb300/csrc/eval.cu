@@ -82,6 +82,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_cost_kernel(const Node8* nodes,
 }
 
 __global__ void finalize_kernel(const Control* ctrl, nxb_build_result* r, uint32_t n) {
+    after_previous();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     for (int a = 0; a < 3; ++a) {
         r->scene_bounds.bmin[a] = ord2f(~ctrl->scene_ord[a]);
@@ -180,8 +181,7 @@ cudaError_t launch_bvh8_cost(const Node8* nodes, uint32_t count, const nxb_aabb*
 }
 
 cudaError_t launch_finalize(const Control* ctrl, nxb_build_result* result, uint32_t n, cudaStream_t s) {
-    finalize_kernel<<<1, 32, 0, s>>>(ctrl, result, n);
-    return cudaGetLastError();
+    return launch_after(n, finalize_kernel, 1, 32, 0, s, ctrl, result, n);
 }
 
 cudaError_t launch_ord_to_aabb(uint32_t* ord, cudaStream_t s) {

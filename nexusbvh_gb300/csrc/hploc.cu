@@ -797,6 +797,7 @@ __device__ __forceinline__ void climb_between(const Climb<K, Seg>& g, WarpTile<R
 template <typename K, int R, typename Seg>
 __global__ __launch_bounds__(32 * kTileWarps, kTileCtas) void hploc_kernel(Climb<K, Seg> g, uint32_t tiles, uint32_t* tile_ctr,
                                                             uint32_t* bvh8_ctr) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     WarpTile<R>& t = reinterpret_cast<WarpTile<R>*>(smem)[threadIdx.x >> 5];
     if (!Seg::kBatch && bvh8_ctr && blockIdx.x == 0 && threadIdx.x == 0) bvh8_queue_counters(bvh8_ctr);
@@ -833,8 +834,11 @@ cudaError_t launch_r(const Climb<K, Seg>& g, uint32_t* tile_ctr, uint32_t* bvh8_
     uint32_t per_sm = std::min((tiles + sms - 1) / sms, (uint32_t)(kTileWarps * kTileCtas));
     if (max_per_sm) per_sm = std::min(per_sm, 4 * max_per_sm);
     const uint32_t ctas = (per_sm + kTileWarps - 1) / kTileWarps, warps = (per_sm + ctas - 1) / ctas;
-    hploc_kernel<K, R, Seg><<<std::min(tiles, sms * ctas), 32 * warps, sizeof(WarpTile<R>) * warps, s>>>(
-        g, tiles, tile_ctr, bvh8_ctr);
+    const uint32_t grid = std::min(tiles, sms * ctas);
+    if constexpr (!Seg::kBatch)
+        return launch_after(g.end, hploc_kernel<K, R, Seg>, grid, 32 * warps, sizeof(WarpTile<R>) * warps, s, g, tiles, tile_ctr,
+                            bvh8_ctr);
+    hploc_kernel<K, R, Seg><<<grid, 32 * warps, sizeof(WarpTile<R>) * warps, s>>>(g, tiles, tile_ctr, bvh8_ctr);
     return cudaGetLastError();
 }
 

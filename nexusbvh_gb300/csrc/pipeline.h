@@ -138,6 +138,32 @@ cudaError_t load_setup_kernels();
 cudaError_t load_sort_kernels();
 cudaError_t load_collapse_kernels();
 
+// Launches a kernel that begins with after_previous(); if the build of n
+// primitives is small, its CTAs are set up while the kernel before it in the
+// stream still runs, otherwise as usual.  Whole builds, usual / early:
+// 1,021 triangles 80 / 72 us, 65,536 151 / 142, 200,000 216 / 205, 500,000
+// 310 / 300, 1.0M 454 / 449, 2.0M 628 / 630, 4.19M sphere 1,026 / 1,034
+// (there the early CTAs take room from the running kernel).  Replayed from a
+// graph, both are the same up to 1.0M; batches, which are, and the server's
+// are launched as usual (200 small meshes 237 / 245).
+constexpr uint32_t kAfterMaxPrims = 1000000;
+template <typename... P, typename... A>
+cudaError_t launch_after(uint32_t n, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &attr;
+    c.numAttrs = n <= kAfterMaxPrims ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+    if (e) cudaGetLastError();
+    return e;
+}
+
 struct DeviceInfo {
     int sms;
     int max_smem_optin;

@@ -975,6 +975,7 @@ __device__ __forceinline__ void local_sort(LocalSmem<K, RB, KPT>& sm, uint32_t c
 template <typename K, int RB, int KPT>
 __global__ __launch_bounds__(kLocalThreads) void sort_cluster_kernel(K* keys, uint32_t* vals, uint32_t n,
                                                                      uint32_t shift, int passes) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     LocalSmem<K, RB, KPT>& sm = *reinterpret_cast<LocalSmem<K, RB, KPT>*>(smem);
     constexpr uint32_t T = LocalSmem<K, RB, KPT>::kTile;
@@ -1037,17 +1038,25 @@ cudaError_t local_attributes(Kern* kernel, size_t smem) {
     if (!e) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
-cudaLaunchConfig_t local_config(uint32_t grid, uint32_t ctas, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr) {
+// Two attributes: launch_after's (if `after`), and the cluster.
+cudaLaunchConfig_t local_config(uint32_t grid, uint32_t ctas, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr,
+                                bool after) {
     cudaLaunchConfig_t c{};
     c.gridDim = dim3(grid);
     c.blockDim = dim3(kLocalThreads);
     c.dynamicSmemBytes = smem;
     c.stream = s;
-    attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = ctas;
-    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = ctas;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     c.attrs = attr;
-    c.numAttrs = ctas > 1 ? 1 : 0;
+    c.numAttrs = ctas > 1 ? 2 : 1;
+    if (!after) {
+        ++c.attrs;
+        --c.numAttrs;
+    }
     return c;
 }
 template <typename K, int RB, int KPT>
@@ -1057,8 +1066,8 @@ cudaError_t launch_local(K* keys, uint32_t* vals, uint32_t n, uint32_t shift, in
     if (e) return e;
     constexpr uint32_t T = LocalSmem<K, RB, KPT>::kTile;
     const uint32_t ctas = (n + T - 1) / T;
-    cudaLaunchAttribute attr{};
-    cudaLaunchConfig_t c = local_config(ctas, ctas, smem, s, &attr);
+    cudaLaunchAttribute attr[2]{};
+    cudaLaunchConfig_t c = local_config(ctas, ctas, smem, s, attr, true);
     return cudaLaunchKernelEx(&c, sort_cluster_kernel<K, RB, KPT>, keys, vals, n, shift, passes);
 }
 template <int RB, int KPT>
@@ -1069,8 +1078,8 @@ cudaError_t launch_local_batch(uint64_t* keys, uint32_t* vals, const MeshBatch& 
     if (e) return e;
     constexpr uint32_t T = LocalSmem<uint32_t, RB, KPT>::kTile;
     const uint32_t ctas = (max_mesh + T - 1) / T;
-    cudaLaunchAttribute attr{};
-    cudaLaunchConfig_t c = local_config(ctas * batch.meshes, ctas, smem, s, &attr);
+    cudaLaunchAttribute attr[2]{};
+    cudaLaunchConfig_t c = local_config(ctas * batch.meshes, ctas, smem, s, attr, false);
     return cudaLaunchKernelEx(&c, sort_cluster_batch_kernel<RB, KPT>, keys, vals, batch, ctas, shift, passes);
 }
 // Keys per thread: as few as the largest cluster (one mesh, where a pass is a
@@ -1285,8 +1294,8 @@ bool local_sort_takes(uint32_t n) {
         auto* kernel = sort_cluster_kernel<uint64_t, kLocalBits64, kLocalMaxKpt>;
         constexpr size_t smem = sizeof(LocalSmem<uint64_t, kLocalBits64, kLocalMaxKpt>);
         cudaError_t r = local_attributes(kernel, smem);
-        cudaLaunchAttribute attr{};
-        const cudaLaunchConfig_t c = local_config(kLocalMaxCtas, kLocalMaxCtas, smem, nullptr, &attr);
+        cudaLaunchAttribute attr[2]{};
+        const cudaLaunchConfig_t c = local_config(kLocalMaxCtas, kLocalMaxCtas, smem, nullptr, attr, true);
         int clusters = 0;
         if (!r) r = cudaOccupancyMaxActiveClusters(&clusters, kernel, &c);
         if (!r && clusters < 1) r = cudaErrorNotSupported;

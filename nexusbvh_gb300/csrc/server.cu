@@ -11,7 +11,7 @@
 //     built as one batch (batch.cu: one launch per stage for all of them),
 //     their inputs laid end to end and their results handed out by one
 //     kernel each (96 requests of 1,024 to 65,536 triangles in a burst: 3.20
-//     ms with three copies per request, 2.72 without); the others run the
+//     ms with three copies per request, 2.2 to 2.7 without); the others run the
 //     plain allocation-free pipeline (nxb_build_async);
 //   * memory comes from a server-owned stream-ordered pool whose release
 //     threshold is the budget, so steady-state requests reuse pool memory;

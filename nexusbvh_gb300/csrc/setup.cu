@@ -26,6 +26,7 @@ template <int FLOATS>
 __global__ __launch_bounds__(kThreads) void scene_bounds_kernel(const float* __restrict__ prims, uint32_t n,
                                                                 Node2* __restrict__ nodes, uint32_t* scene_ord,
                                                                 bool aligned16) {
+    after_previous();
     __shared__ __align__(16) float tile[kThreads * FLOATS];
     __shared__ float red[kThreads / 32][6];
     Box acc;
@@ -155,6 +156,7 @@ struct MortonArgs {
 template <typename K, bool HIST, int PASSES = 0, int BINS = kRadixBins>
 __global__ __launch_bounds__(kThreads) void morton_kernel(const Node2* __restrict__ nodes, uint32_t n, Control* ctrl,
                                                           K* __restrict__ keys, MortonArgs a) {
+    after_previous();
     static_assert(PASSES * BINS <= kMaxSortPasses * kRadixBins, "histograms fit the control block");
     __shared__ float s_scene[6];
     __shared__ uint32_t s_hist[HIST ? kMaxSortPasses * kRadixBins : 1];
@@ -712,25 +714,19 @@ cudaError_t launch_morton(const Node2* nodes, uint32_t n, Control* ctrl, int key
     // 14 us at 2 CTAs per SM, 23 at 8; 2.0M 25 at 3, 29 at 8; 12.58M 175 at 2,
     // 103 at 8
     uint32_t grid = grid_for(n, f.plan ? (int)std::min(2u + n / 1200000u, 8u) : 8);
+    auto go = [&](auto* kernel, auto* out) {
+        return launch_after(n, kernel, grid, kThreads, 0, s, nodes, n, ctrl, out, a);
+    };
     if (key_bits == 30) {
-        if (f.plan && a.pd.passes == 4)
-            morton_kernel<uint32_t, true, 4><<<grid, kThreads, 0, s>>>(nodes, n, ctrl, (uint32_t*)keys, a);
-        else if (f.plan)
-            morton_kernel<uint32_t, true><<<grid, kThreads, 0, s>>>(nodes, n, ctrl, (uint32_t*)keys, a);
-        else
-            morton_kernel<uint32_t, false><<<grid, kThreads, 0, s>>>(nodes, n, ctrl, (uint32_t*)keys, a);
-    } else {
-        if (f.plan && a.pd.passes == 4 && a.pd.mask[0] == (1u << kMaxRadixBits) - 1u)
-            morton_kernel<uint64_t, true, 4, 1 << kMaxRadixBits><<<grid, kThreads, 0, s>>>(nodes, n, ctrl,
-                                                                                           (uint64_t*)keys, a);
-        else if (f.plan && a.pd.passes == 8)
-            morton_kernel<uint64_t, true, 8><<<grid, kThreads, 0, s>>>(nodes, n, ctrl, (uint64_t*)keys, a);
-        else if (f.plan)
-            morton_kernel<uint64_t, true><<<grid, kThreads, 0, s>>>(nodes, n, ctrl, (uint64_t*)keys, a);
-        else
-            morton_kernel<uint64_t, false><<<grid, kThreads, 0, s>>>(nodes, n, ctrl, (uint64_t*)keys, a);
+        uint32_t* out = (uint32_t*)keys;
+        if (!f.plan) return go(morton_kernel<uint32_t, false>, out);
+        return a.pd.passes == 4 ? go(morton_kernel<uint32_t, true, 4>, out) : go(morton_kernel<uint32_t, true>, out);
     }
-    return cudaGetLastError();
+    uint64_t* out = (uint64_t*)keys;
+    if (!f.plan) return go(morton_kernel<uint64_t, false>, out);
+    if (a.pd.passes == 4 && a.pd.mask[0] == (1u << kMaxRadixBits) - 1u)
+        return go(morton_kernel<uint64_t, true, 4, 1 << kMaxRadixBits>, out);
+    return a.pd.passes == 8 ? go(morton_kernel<uint64_t, true, 8>, out) : go(morton_kernel<uint64_t, true>, out);
 }
 
 cudaError_t launch_morton_scene(const Node2* nodes, uint32_t n, const nxb_aabb* scene, int key_bits, void* keys,
@@ -766,14 +762,11 @@ uint32_t batch_grid(uint32_t total) {
 }
 
 template <int T>
-void bounds_t(const void* prims, int prim_type, const MeshBatch& batch, uint32_t total, Node2* nodes,
-              uint32_t* scene_ord, bool aligned, const uint2* tile_rng, cudaStream_t s) {
-    if (prim_type == NXB_PRIM_TRIANGLE)
-        batch_bounds_kernel<9, T><<<batch_grid<T>(total), T, 0, s>>>((const float*)prims, batch, total, nodes,
-                                                                     scene_ord, aligned, tile_rng);
-    else
-        batch_bounds_kernel<6, T><<<batch_grid<T>(total), T, 0, s>>>((const float*)prims, batch, total, nodes,
-                                                                     scene_ord, aligned, tile_rng);
+cudaError_t bounds_t(const void* prims, int prim_type, const MeshBatch& batch, uint32_t total, Node2* nodes,
+                     uint32_t* scene_ord, bool aligned, const uint2* tile_rng, cudaStream_t s) {
+    auto* kernel = prim_type == NXB_PRIM_TRIANGLE ? batch_bounds_kernel<9, T> : batch_bounds_kernel<6, T>;
+    kernel<<<batch_grid<T>(total), T, 0, s>>>((const float*)prims, batch, total, nodes, scene_ord, aligned, tile_rng);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_batch_begin(const BatchBegin& b, const MeshBatch& batch, cudaStream_t s) {
@@ -808,13 +801,9 @@ cudaError_t launch_batch_bounds(const void* prims, int prim_type, const MeshBatc
                                 Node2* nodes, uint32_t* scene_ord, uint32_t block, const uint2* tile_rng,
                                 cudaStream_t s) {
     const bool aligned = (reinterpret_cast<uintptr_t>(prims) & 15u) == 0;
-    if (block == 128)
-        bounds_t<128>(prims, prim_type, batch, total, nodes, scene_ord, aligned, tile_rng, s);
-    else if (block == 512)
-        bounds_t<512>(prims, prim_type, batch, total, nodes, scene_ord, aligned, tile_rng, s);
-    else
-        bounds_t<256>(prims, prim_type, batch, total, nodes, scene_ord, aligned, tile_rng, s);
-    return cudaGetLastError();
+    if (block == 128) return bounds_t<128>(prims, prim_type, batch, total, nodes, scene_ord, aligned, tile_rng, s);
+    if (block == 512) return bounds_t<512>(prims, prim_type, batch, total, nodes, scene_ord, aligned, tile_rng, s);
+    return bounds_t<256>(prims, prim_type, batch, total, nodes, scene_ord, aligned, tile_rng, s);
 }
 
 cudaError_t launch_batch_morton(const Node2* nodes, const MeshBatch& batch, uint32_t total, const uint32_t* scene_ord,
@@ -827,29 +816,15 @@ cudaError_t launch_batch_morton(const Node2* nodes, const MeshBatch& batch, uint
     a.ones_ptr = reinterpret_cast<uint4*>(f.ones_ptr);
     a.ones_vec4 = f.ones_words / 4;
     const bool five = a.pd.passes == 5;  // 8-bit digits over 40 bits: 1024 meshes
-    if (block == 128) {
-        if (five)
-            batch_morton_kernel<true, 128, 5><<<batch_grid<128>(total), 128, 0, s>>>(nodes, batch, total, scene_ord,
-                                                                                    keys, vals, hist, a, tile_rng);
-        else
-            batch_morton_kernel<true, 128><<<batch_grid<128>(total), 128, 0, s>>>(nodes, batch, total, scene_ord, keys,
-                                                                                  vals, hist, a, tile_rng);
-    } else if (block == 512) {
-        if (five)
-            batch_morton_kernel<true, 512, 5><<<batch_grid<512>(total), 512, 0, s>>>(nodes, batch, total, scene_ord,
-                                                                                    keys, vals, hist, a, tile_rng);
-        else
-            batch_morton_kernel<true, 512><<<batch_grid<512>(total), 512, 0, s>>>(nodes, batch, total, scene_ord, keys,
-                                                                                  vals, hist, a, tile_rng);
-    } else {
-        if (five)
-            batch_morton_kernel<true, 256, 5><<<batch_grid<256>(total), 256, 0, s>>>(nodes, batch, total, scene_ord,
-                                                                                    keys, vals, hist, a, tile_rng);
-        else
-            batch_morton_kernel<true, 256><<<batch_grid<256>(total), 256, 0, s>>>(nodes, batch, total, scene_ord, keys,
-                                                                                  vals, hist, a, tile_rng);
-    }
-    return cudaGetLastError();
+    auto go = [&](auto* kernel, uint32_t grid) {
+        kernel<<<grid, block, 0, s>>>(nodes, batch, total, scene_ord, keys, vals, hist, a, tile_rng);
+        return cudaGetLastError();
+    };
+    if (block == 128)
+        return go(five ? batch_morton_kernel<true, 128, 5> : batch_morton_kernel<true, 128>, batch_grid<128>(total));
+    if (block == 512)
+        return go(five ? batch_morton_kernel<true, 512, 5> : batch_morton_kernel<true, 512>, batch_grid<512>(total));
+    return go(five ? batch_morton_kernel<true, 256, 5> : batch_morton_kernel<true, 256>, batch_grid<256>(total));
 }
 
 cudaError_t launch_segment_morton(const Node2* nodes, const MeshBatch& batch, const uint32_t* scene_ord,

@@ -740,6 +740,7 @@ constexpr uint32_t kNoChild = (1u << 21) - 1u;
 template <typename Seg>
 __global__ __launch_bounds__(kThreads) void bvh8_lists_kernel(Seg seg, uint32_t records,
                                                               const ChildPair* __restrict__ kids, uint64_t* lists) {
+    after_previous();
     extern __shared__ uint32_t s_slots[];
     const SlotTable<true> tab{s_slots};
     const uint32_t r = blockIdx.x * kThreads + threadIdx.x;
@@ -797,6 +798,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
                                                               uint32_t* mesh_leaves, uint32_t* err,
                                                               const ChildPair* __restrict__ kids,
                                                               const uint64_t* __restrict__ lists) {
+    after_previous();
     __shared__ __align__(8) uint8_t s_rows[kGroupsPerCta][64];  // meta and quantised bytes of a group's node
     const uint32_t lane = lane_id(), sub = lane & 7u, base = lane & 24u;
     uint8_t* rows = s_rows[threadIdx.x >> 3];
@@ -1065,8 +1067,14 @@ cudaError_t launch_group(const Node2* bvh2, Seg seg, uint32_t items, Node8* out,
                                         cudaSharedmemCarveoutMaxShared);
         });
         if (e) return e;
-        bvh8_lists_kernel<Seg>
-            <<<(items + kThreads - 1) / kThreads, kThreads, (kSlotSmem<true>), s>>>(seg, items, kids, lists);
+        const uint32_t ctas = (items + kThreads - 1) / kThreads;
+        if constexpr (Seg::kBatch) {
+            bvh8_lists_kernel<Seg><<<ctas, kThreads, (kSlotSmem<true>), s>>>(seg, items, kids, lists);
+        } else {
+            const cudaError_t le =
+                launch_after(items, bvh8_lists_kernel<Seg>, ctas, kThreads, kSlotSmem<true>, s, seg, items, kids, lists);
+            if (le) return le;
+        }
     }
     int per_sm = resident_ctas<bvh8_group_kernel<Seg, AUCTION, LISTS>>(kThreads, 0);
     // Groups that wait poll the pending counter, and too many of them saturate
@@ -1080,6 +1088,9 @@ cudaError_t launch_group(const Node2* bvh2, Seg seg, uint32_t items, Node8* out,
     if (LISTS) groups = std::max(std::min(groups, 4096u), (items + 31) / 32);
     const uint32_t want = (groups + kGroupsPerCta - 1) / kGroupsPerCta;
     const uint32_t grid = std::max(1u, std::min(want, (uint32_t)(device_info().sms * per_sm)));
+    if constexpr (LISTS && !Seg::kBatch)
+        return launch_after(items, bvh8_group_kernel<Seg, AUCTION, LISTS>, grid, kThreads, 0, s, bvh2, seg, out, cap, slots,
+                            prim_idx, pairs, ctr, mesh_nodes, mesh_leaves, err, kids, lists);
     bvh8_group_kernel<Seg, AUCTION, LISTS><<<grid, kThreads, 0, s>>>(bvh2, seg, out, cap, slots, prim_idx, pairs, ctr,
                                                                      mesh_nodes, mesh_leaves, err, kids, lists);
     return cudaGetLastError();
