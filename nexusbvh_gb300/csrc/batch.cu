@@ -202,7 +202,6 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
         const bool in_a = (plan.passes % 2) == 0;
         uint64_t* keys = in_a ? a.keys_a : a.keys_b;
         uint32_t* perm = in_a ? a.vals_a : a.vals_b;
-        uint32_t* tokens = in_a ? a.vals_b : a.vals_a;
         // a whole batch's collapse has the sort's buffers (24 bytes per
         // primitive) for its lists; that of a group has not, as the climb of
         // the next group still reads them
@@ -211,7 +210,11 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
         // the side stream (ordered by an event, no wait inside any kernel),
         // overlapping H-PLOC of group k+1
         for (uint32_t k = 0; k < g.count; ++k) {
-            NXB_TRY(launch_hploc_batch(keys, perm, a.parent, a.bvh2, mb, g.prim[k], g.prim[k + 1], t.radius, tokens,
+            // its records lie where the group's BVH8 nodes will: 32 bytes for
+            // each of a mesh's n primitives in 80 for each of its slots, of
+            // which there are at least (4n - 1) / 7 and one
+            Node2* records = reinterpret_cast<Node2*>(a.bvh8 + g.slot[k]) - g.prim[k];
+            NXB_TRY(launch_hploc_batch(keys, perm, a.parent, a.bvh2, mb, g.prim[k], g.prim[k + 1], t.radius, records,
                                        a.pol, a.ctrl->hploc_tile_ctr + k, &a.ctrl->error_word, t.hploc_ctas_per_sm, s,
                                        a.kids));
             const uint32_t m0 = g.mesh[k];

@@ -336,28 +336,15 @@ __device__ __forceinline__ uint32_t merge_window(const MergeCtx& m, uint32_t num
     return num;
 }
 
-// Where subtrees that leave their tile keep their clusters.  A plain build
-// stores them as {box, id, token} records at the window's positions, so the
-// next merge reads 16 consecutive records in one round trip; a batch, which
-// has no room for records, stores id and token and reads the box from the
-// node array.
-struct Published {
-    Node2* rec;         // plain builds
-    uint32_t* cluster;  // batches
-    uint32_t* tok;
-    template <typename Seg>
-    __device__ __forceinline__ void store(uint32_t pos, const Box& b, uint32_t cid, uint32_t ctok) const {
-        if constexpr (Seg::kBatch) {
-            __stcg(cluster + pos, cid);
-            __stcg(tok + pos, ctok);
-        } else {
-            uint4* p = reinterpret_cast<uint4*>(rec + pos);
-            __stcg(p, make_uint4(__float_as_uint(b.mn.x), __float_as_uint(b.mn.y), __float_as_uint(b.mn.z),
-                                 __float_as_uint(b.mx.x)));
-            __stcg(p + 1, make_uint4(__float_as_uint(b.mx.y), __float_as_uint(b.mx.z), cid, ctok));
-        }
-    }
-};
+// Subtrees that leave their tile store their clusters as {box, id, token}
+// records at the window's positions, so that the next merge reads 16
+// consecutive records in one round trip.
+__device__ __forceinline__ void publish(Node2* rec, uint32_t pos, const Box& b, uint32_t cid, uint32_t ctok) {
+    uint4* p = reinterpret_cast<uint4*>(rec + pos);
+    __stcg(p, make_uint4(__float_as_uint(b.mn.x), __float_as_uint(b.mn.y), __float_as_uint(b.mn.z),
+                         __float_as_uint(b.mx.x)));
+    __stcg(p + 1, make_uint4(__float_as_uint(b.mx.y), __float_as_uint(b.mx.z), cid, ctok));
+}
 
 // ---------------------------------------------------------------- tiles
 // A tile is a run of consecutive sorted leaves held in shared memory by one
@@ -388,11 +375,11 @@ struct __align__(16) WarpTile {
 template <typename K, typename Seg>
 struct Climb {
     const K* keys;
-    uint32_t* cluster;
+    const uint32_t* cluster;
     uint32_t* parent;
     Seg seg;
     Outputs out;
-    Published pub;
+    Node2* rec;
     uint32_t begin, end, tile;  // tile: leaves per tile
     uint64_t* bvh8_pairs;
 };
@@ -400,24 +387,18 @@ struct Climb {
 // LoadIndices (BinaryBuilder.cu:42-57): one lane's entry k of a published
 // window of `size` leaves at `pos`.
 template <typename K, typename Seg>
-__device__ __forceinline__ void load_entry(const Climb<K, Seg>& g, const MergeCtx& m, uint32_t pos, uint32_t k,
-                                           uint32_t size, uint32_t& v, uint32_t& t, Box& b) {
+__device__ __forceinline__ void load_entry(const Climb<K, Seg>& g, uint32_t pos, uint32_t k, uint32_t size, uint32_t& v,
+                                           uint32_t& t, Box& b) {
     v = kInvalid;
     t = 0;
     b.mn = b.mx = make_float3(0.f, 0.f, 0.f);
     if (k >= min(size, kMergeThreshold)) return;
-    if constexpr (Seg::kBatch) {
-        v = __ldcg(g.pub.cluster + pos + k);
-        t = __ldcg(g.pub.tok + pos + k);
-        if (v < m.limit()) b = load_box_cg(m.node(v), 0);
-    } else {
-        const uint4* p = reinterpret_cast<const uint4*>(g.pub.rec + pos + k);
-        const uint4 lo = __ldcg(p), hi = __ldcg(p + 1);
-        b.mn = make_float3(__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z));
-        b.mx = make_float3(__uint_as_float(lo.w), __uint_as_float(hi.x), __uint_as_float(hi.y));
-        v = hi.z;
-        t = hi.w;
-    }
+    const uint4* p = reinterpret_cast<const uint4*>(g.rec + pos + k);
+    const uint4 lo = __ldcg(p), hi = __ldcg(p + 1);
+    b.mn = make_float3(__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z));
+    b.mx = make_float3(__uint_as_float(lo.w), __uint_as_float(hi.x), __uint_as_float(hi.y));
+    v = hi.z;
+    t = hi.w;
 }
 
 // FindParentId (BinaryBuilder.cu:30-40): whether the range [l, r] of the mesh
@@ -448,7 +429,7 @@ __device__ __forceinline__ bool merge_between(const Climb<K, Seg>& g, uint32_t o
     bool bad;  // a window's valid ids must be a prefix of it, and in range
     {
         const bool lo = lane < 16;
-        load_entry(g, m, lo ? l : mid, lane & 15u, lo ? mid - l : r + 1 - mid, cid, ctok, cb);
+        load_entry(g, lo ? l : mid, lane & 15u, lo ? mid - l : r + 1 - mid, cid, ctok, cb);
         const uint32_t vb = __ballot_sync(kFullMask, cid != kInvalid);
         first = __popc(vb & 0xFFFFu);
         num = __popc(vb);
@@ -482,7 +463,7 @@ __device__ __forceinline__ bool merge_between(const Climb<K, Seg>& g, uint32_t o
         __syncwarp();  // acquired by all
         uint32_t v, t;
         Box b;
-        load_entry(g, m, go_right ? r + 1 : other, lane, go_right ? other - r : l - other, v, t, b);
+        load_entry(g, go_right ? r + 1 : other, lane, go_right ? other - r : l - other, v, t, b);
         const uint32_t vb = __ballot_sync(kFullMask, v != kInvalid);
         const uint32_t ns = __popc(vb);
         bad = (vb & (vb + 1)) != 0;
@@ -495,7 +476,7 @@ __device__ __forceinline__ bool merge_between(const Climb<K, Seg>& g, uint32_t o
         else
             l = other;
     }
-    if (!fin && lane < min(r - l + 1, kMergeThreshold)) g.pub.template store<Seg>(l + lane, cb, lane < num ? cid : kInvalid, ctok);
+    if (!fin && lane < min(r - l + 1, kMergeThreshold)) publish(g.rec, l + lane, cb, lane < num ? cid : kInvalid, ctok);
     if (lane == owner) {
         left = l;
         right = r;
@@ -698,7 +679,7 @@ __device__ __forceinline__ uint32_t leave_tile(const Climb<K, Seg>& g, WarpTile<
         const uint32_t num = (uint32_t)(e >> 32) & 0xFFu, k = lane & 15u;
         if (k < min(size, kMergeThreshold)) {
             const uint2 it = rows.ids(l + k);
-            g.pub.template store<Seg>(base + l + k, rows.box(l + k), k < num ? it.x : kInvalid, it.y);
+            publish(g.rec, base + l + k, rows.box(l + k), k < num ? it.x : kInvalid, it.y);
         }
     }
     __syncwarp();
@@ -725,6 +706,7 @@ __device__ __forceinline__ void climb_between(const Climb<K, Seg>& g, WarpTile<R
     uint32_t item = lane;
     uint32_t left = 0, right = 0, split = 0;
     bool active = false, peek = false;
+    MeshSpan me = Seg::kBatch ? MeshSpan{0, 0, 0} : g.seg.of_prim(0);
     bool release_due = true;  // warp-uniform: stores or acquired clusters since the last release fence
     for (;;) {
         bool fresh = false, go_right = false;
@@ -738,8 +720,7 @@ __device__ __forceinline__ void climb_between(const Climb<K, Seg>& g, WarpTile<R
             peek = false;
         }
         if (!__any_sync(kFullMask, active)) break;
-        MeshSpan me = Seg::kBatch ? MeshSpan{0, 0, 0} : g.seg.of_prim(0);
-        if (Seg::kBatch && active) me = span_at(g.keys, g.seg, left);
+        if (Seg::kBatch && fresh) me = span_at(g.keys, g.seg, left);
         if (active && !fresh) go_right = hands_right(g.keys, left, right, me.start, me.count);
         uint32_t* slot = g.parent + (go_right ? right : left - 1);
         uint32_t sib = kInvalid;  // the sibling's other end
@@ -843,17 +824,16 @@ cudaError_t launch_r(const Climb<K, Seg>& g, uint32_t* tile_ctr, uint32_t* bvh8_
 }
 
 template <typename K, typename Seg>
-cudaError_t launch_t(const K* keys, uint32_t* cluster, uint32_t* parent, Node2* nodes, Seg seg, uint32_t begin,
-                     uint32_t end, uint32_t radius, uint32_t* tok, uint32_t* pol, uint32_t* tile_ctr, uint32_t* err,
-                     uint32_t max_per_sm, cudaStream_t s, Node2* rec = nullptr, uint64_t* pairs = nullptr,
-                     uint32_t* ctr = nullptr, ChildPair* kids = nullptr) {
+cudaError_t launch_t(const K* keys, const uint32_t* cluster, uint32_t* parent, Node2* nodes, Seg seg, uint32_t begin,
+                     uint32_t end, uint32_t radius, uint32_t* pol, uint32_t* tile_ctr, uint32_t* err,
+                     uint32_t max_per_sm, cudaStream_t s, Node2* rec, uint64_t* pairs, uint32_t* ctr,
+                     ChildPair* kids) {
     // one tile per resident warp while that is at most kTile leaves, so that
     // small builds use every SM: 65,536 triangles take 71 us with 32 leaves
     // per tile, 88 with 144; below 32 leaves (two windows) a tile has no merge
     const uint32_t warps = (uint32_t)device_info().sms * kTileWarps * kTileCtas;
     const uint32_t tile = std::max(32u, std::min((end - begin + warps - 1) / warps, (uint32_t)kTile));
-    const Climb<K, Seg> g{keys, cluster, parent, seg,  {nodes, kids, pol, err}, {rec, cluster, tok},
-                          begin, end,   tile,   pairs};
+    const Climb<K, Seg> g{keys, cluster, parent, seg, {nodes, kids, pol, err}, rec, begin, end, tile, pairs};
     switch (radius) {
         case 4: return launch_r<K, 4, Seg>(g, tile_ctr, ctr, max_per_sm, s);
         case 16: return launch_r<K, 16, Seg>(g, tile_ctr, ctr, max_per_sm, s);
@@ -870,19 +850,18 @@ cudaError_t launch_hploc(uint32_t key_bytes, const void* keys, uint32_t* cluster
     const SingleMesh seg{n};
     if (!bvh8_pairs != !bvh8_ctr) return cudaErrorInvalidValue;
     if (key_bytes == 4)
-        return launch_t((const uint32_t*)keys, cluster_idx, parent, nodes, seg, 0u, n, radius, nullptr,
-                        parent_of_last, ctr, err, 0u, s, records, bvh8_pairs, bvh8_ctr,
-                        child_pairs);
-    return launch_t((const uint64_t*)keys, cluster_idx, parent, nodes, seg, 0u, n, radius, nullptr, parent_of_last,
-                    ctr, err, 0u, s, records, bvh8_pairs, bvh8_ctr, child_pairs);
+        return launch_t((const uint32_t*)keys, cluster_idx, parent, nodes, seg, 0u, n, radius, parent_of_last, ctr,
+                        err, 0u, s, records, bvh8_pairs, bvh8_ctr, child_pairs);
+    return launch_t((const uint64_t*)keys, cluster_idx, parent, nodes, seg, 0u, n, radius, parent_of_last, ctr,
+                    err, 0u, s, records, bvh8_pairs, bvh8_ctr, child_pairs);
 }
 
 cudaError_t launch_hploc_batch(const uint64_t* keys, uint32_t* cluster_idx, uint32_t* parent, Node2* nodes,
                                const MeshBatch& batch, uint32_t begin, uint32_t end, uint32_t radius,
-                               uint32_t* tokens, uint32_t* parent_of_last, uint32_t* ctr, uint32_t* err,
+                               Node2* records, uint32_t* parent_of_last, uint32_t* ctr, uint32_t* err,
                                uint32_t ctas_per_sm, cudaStream_t s, ChildPair* child_pairs) {
     return launch_t(reinterpret_cast<const MeshKey*>(keys), cluster_idx, parent, nodes, batch, begin, end, radius,
-                    tokens, parent_of_last, ctr, err, ctas_per_sm, s, nullptr, nullptr, nullptr, child_pairs);
+                    parent_of_last, ctr, err, ctas_per_sm, s, records, nullptr, nullptr, child_pairs);
 }
 
 }  // namespace nxb

@@ -311,13 +311,13 @@ cudaError_t launch_segment_morton(const Node2* nodes, const MeshBatch& batch, co
                                   uint32_t* codes, const SegmentPlan& plan, const MortonFused& fill, uint32_t block,
                                   cudaStream_t s);
 // H-PLOC over the sorted positions [begin, end), which must cover whole
-// meshes; leaf_ctr: a zeroed word of its own.  parent_of_last: one word per
+// meshes; records: as for launch_hploc, by position; tile_ctr: a zeroed word of its own.  parent_of_last: one word per
 // mesh holding INVALID on entry; ctas_per_sm caps the persistent grid (0: as
 // many CTAs as fit).  child_pairs (optional): one 64-byte record per
 // primitive of the batch; mesh m's internal node X gets record off[m] + X - n_m.
 cudaError_t launch_hploc_batch(const uint64_t* keys, uint32_t* cluster_idx, uint32_t* parent, Node2* nodes,
                                const MeshBatch& batch, uint32_t begin, uint32_t end, uint32_t radius,
-                               uint32_t* tokens, uint32_t* parent_of_last, uint32_t* tile_ctr, uint32_t* err,
+                               Node2* records, uint32_t* parent_of_last, uint32_t* tile_ctr, uint32_t* err,
                                uint32_t ctas_per_sm, cudaStream_t s, ChildPair* child_pairs = nullptr);
 // Meshes cut into consecutive groups whose BVH8 collapses are separate
 // launches: group g holds meshes [mesh[g], mesh[g+1]), primitives
