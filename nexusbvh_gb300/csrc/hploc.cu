@@ -366,6 +366,7 @@ struct __align__(16) WarpTile {
     uint2 c[kRows];
     uint64_t gap[kTile + 2];   // deltas; then the list of subtrees that leave the tile
     uint32_t hand[kTile + 4];  // hand-over slots: the range's other end | clusters << 16
+    uint4 mesh;                // batches: the mesh, its start and count if the tile lies in one, else count 0
     __device__ __forceinline__ Row rows() {
         return {(uint32_t)__cvta_generic_to_shared(a + kRowFront), (uint32_t)__cvta_generic_to_shared(b + kRowFront),
                 (uint32_t)__cvta_generic_to_shared(c + kRowFront)};
@@ -374,6 +375,18 @@ struct __align__(16) WarpTile {
 
 template <typename K, typename Seg>
 struct Climb {
+    // the mesh of the leaf at position p, which lies in the tile (or in a
+    // range that reaches into it)
+    template <int R>
+    __device__ __forceinline__ MeshSpan span(const WarpTile<R>& t, uint32_t p) const {
+        if constexpr (Seg::kBatch) {
+            const uint4 m = t.mesh;
+            if (m.z) return {m.x, m.y, m.z};
+            return span_at(keys, seg, p);
+        } else {
+            return seg.of_prim(p);
+        }
+    }
     const K* keys;
     const uint32_t* cluster;
     uint32_t* parent;
@@ -416,12 +429,12 @@ __device__ __forceinline__ bool hands_right(const K* keys, uint32_t l, uint32_t 
 // to load.  Returns the range reached and whether it is a whole mesh; the
 // clusters of a range that is not are stored (StoreIndices, :59-69).
 template <int R, typename K, typename Seg>
-__device__ __forceinline__ bool merge_between(const Climb<K, Seg>& g, uint32_t owner, uint32_t& left, uint32_t& right,
-                                              uint32_t split, const Row& row) {
+__device__ __forceinline__ bool merge_between(const Climb<K, Seg>& g, const WarpTile<R>& t, uint32_t owner,
+                                              uint32_t& left, uint32_t& right, uint32_t split, const Row& row) {
     const uint32_t lane = lane_id();
     uint32_t l = __shfl_sync(kFullMask, left, owner), r = __shfl_sync(kFullMask, right, owner);
     const uint32_t mid = __shfl_sync(kFullMask, split, owner);
-    const MeshSpan me = span_at(g.keys, g.seg, l);
+    const MeshSpan me = g.span(t, l);
     const uint32_t start = me.start;
     const MergeCtx m{g.out, me.m, start, me.count};
     uint32_t cid, ctok, num, first;
@@ -461,15 +474,15 @@ __device__ __forceinline__ bool merge_between(const Climb<K, Seg>& g, uint32_t o
         const uint32_t other = __shfl_sync(kFullMask, ld_acquire_u32(g.parent + (go_right ? r : l - 1)), 0);
         if (other == kInvalid) break;
         __syncwarp();  // acquired by all
-        uint32_t v, t;
+        uint32_t v, vt;
         Box b;
-        load_entry(g, go_right ? r + 1 : other, lane, go_right ? other - r : l - other, v, t, b);
+        load_entry(g, go_right ? r + 1 : other, lane, go_right ? other - r : l - other, v, vt, b);
         const uint32_t vb = __ballot_sync(kFullMask, v != kInvalid);
         const uint32_t ns = __popc(vb);
         bad = (vb & (vb + 1)) != 0;
         __syncwarp();
         if (!go_right && lane < num) row.put(ns + lane, cb, cid, ctok);
-        if (v != kInvalid) row.put((go_right ? num : 0u) + lane, b, v, t);
+        if (v != kInvalid) row.put((go_right ? num : 0u) + lane, b, v, vt);
         num += ns;
         if (go_right)
             r = other;
@@ -494,6 +507,7 @@ __device__ __forceinline__ void load_tile(const Climb<K, Seg>& g, WarpTile<R>& t
     // most tiles of a batch lie inside one mesh
     MeshSpan first = span_at(g.keys, g.seg, base);
     const bool one = !Seg::kBatch || base + cnt <= first.start + first.count;
+    if (Seg::kBatch && lane == 0) t.mesh = make_uint4(first.m, first.start, one ? first.count : 0u, 0u);
     uint32_t id[kPer];
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
@@ -602,7 +616,7 @@ __device__ __forceinline__ void climb_tile(const Climb<K, Seg>& g, WarpTile<R>& 
             const uint32_t lr = __shfl_sync(kFullMask, range, owner), ps = __shfl_sync(kFullMask, parts, owner);
             uint32_t l = lr & 0xFFFFu, r = lr >> 16, mid = ps & 0xFFFFu, cl = ps >> 16 & 0xFFu, num = cl + (ps >> 24);
             bool fin = t.gap[l] == kEdge && t.gap[r + 1] == kEdge;
-            const MeshSpan me = span_at(g.keys, g.seg, base + l);
+            const MeshSpan me = g.span(t, base + l);
             const MergeCtx m{g.out, me.m, me.start, me.count};
             uint32_t cid, ctok = 0;
             Box cb;
@@ -720,7 +734,7 @@ __device__ __forceinline__ void climb_between(const Climb<K, Seg>& g, WarpTile<R
             peek = false;
         }
         if (!__any_sync(kFullMask, active)) break;
-        if (Seg::kBatch && fresh) me = span_at(g.keys, g.seg, left);
+        if (Seg::kBatch && fresh) me = g.span(t, left);
         if (active && !fresh) go_right = hands_right(g.keys, left, right, me.start, me.count);
         uint32_t* slot = g.parent + (go_right ? right : left - 1);
         uint32_t sib = kInvalid;  // the sibling's other end
@@ -752,7 +766,7 @@ __device__ __forceinline__ void climb_between(const Climb<K, Seg>& g, WarpTile<R
         while (todo) {
             const uint32_t owner = __ffs(todo) - 1;
             todo &= todo - 1;
-            if (merge_between<R>(g, owner, left, right, split, row) && lane == owner) active = false;
+            if (merge_between<R>(g, t, owner, left, right, split, row) && lane == owner) active = false;
         }
     }
     __syncwarp();
