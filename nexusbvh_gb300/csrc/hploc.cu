@@ -844,9 +844,12 @@ cudaError_t launch_t(const K* keys, const uint32_t* cluster, uint32_t* parent, N
                      ChildPair* kids) {
     // one tile per resident warp while that is at most kTile leaves, so that
     // small builds use every SM: 65,536 triangles take 71 us with 32 leaves
-    // per tile, 88 with 144; below 32 leaves (two windows) a tile has no merge
+    // per tile, 88 with 144.  The smallest tile is a window and a little: whole
+    // builds of 1,021 / 8,000 / 16,411 / 32,000 / 65,536 primitives with 16
+    // leaves 68 / 96 / 161 / 124 / 143 us, 20: 68 / 92 / 159 / 120 / 143, 24:
+    // 69 / 93 / 158 / 120 / 145, 32: 72 / 94 / 163 / 119 / 146
     const uint32_t warps = (uint32_t)device_info().sms * kTileWarps * kTileCtas;
-    const uint32_t tile = std::max(32u, std::min((end - begin + warps - 1) / warps, (uint32_t)kTile));
+    const uint32_t tile = std::max(20u, std::min((end - begin + warps - 1) / warps, (uint32_t)kTile));
     const Climb<K, Seg> g{keys, cluster, parent, seg, {nodes, kids, pol, err}, rec, begin, end, tile, pairs};
     switch (radius) {
         case 4: return launch_r<K, 4, Seg>(g, tile_ctr, ctr, max_per_sm, s);
