@@ -429,18 +429,25 @@ void batch_groups(const uint32_t* h_off, const uint32_t* h_off8, uint32_t meshes
 nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type type, const BatchTuning& t,
                          uint32_t* h_err, cudaStream_t s, const MeshGroups* groups = nullptr,
                          const BatchFork* fork = nullptr);
-// Where the meshes of a batch come from and go to, one entry per mesh in
-// memory that the device can read: gather lays the primitives of the meshes
-// that have a source end to end at dst, scatter copies each mesh's BVH8 nodes
-// and primIdx out of a built arena.
+// Where the meshes of a batch come from and go to, one entry per mesh.
 struct BatchPlaces {
     const void* prims;  // null: not gathered
     Node8* nodes;
     uint32_t* prim_idx;
 };
-cudaError_t launch_batch_gather(const BatchArena& a, const BatchPlaces* places, nxb_prim_type type, void* dst,
+// What a batched job shares with the host, in pinned memory: gather writes
+// the arena's offsets and lays the primitives of the meshes that have a
+// source end to end at dst; scatter copies each mesh's BVH8 nodes and primIdx
+// out of the built arena, and the results and the error word to the host.
+struct BatchHost {
+    const uint32_t *off, *off8;  // meshes + 1
+    const BatchPlaces* places;
+    nxb_batch_mesh* meshes;
+    uint32_t* err;
+};
+cudaError_t launch_batch_gather(const BatchArena& a, const BatchHost& h, nxb_prim_type type, void* dst,
                                 cudaStream_t s);
-cudaError_t launch_batch_scatter(const BatchArena& a, const BatchPlaces* places, cudaStream_t s);
+cudaError_t launch_batch_scatter(const BatchArena& a, const BatchHost& h, cudaStream_t s);
 // ---------------------------------------------------------------- eval
 cudaError_t launch_bvh2_cost(const Node2* nodes, uint32_t count, const nxb_aabb* root, float* cost, cudaStream_t s);
 cudaError_t launch_bvh8_cost(const Node8* nodes, uint32_t count, const nxb_aabb* root, float* cost, cudaStream_t s);

@@ -74,7 +74,8 @@ struct Job {
     std::condition_variable* wake = nullptr;
 };
 
-// Pinned per-slot staging: a slot runs one job at a time.
+// Pinned per-slot staging, which the device reads and writes: a slot runs one
+// job at a time.
 struct Slot {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_start = nullptr, ev_end = nullptr;  // the running job's device interval
@@ -84,7 +85,7 @@ struct Slot {
     uint32_t* h_off = nullptr;             // batch_max_meshes + 1
     uint32_t* h_off8 = nullptr;            // batch_max_meshes + 1
     nxb_batch_mesh* h_meshes = nullptr;    // batch_max_meshes
-    BatchPlaces* h_places = nullptr;       // batch_max_meshes; read by the device
+    BatchPlaces* h_places = nullptr;       // batch_max_meshes
 };
 
 }  // namespace
@@ -220,36 +221,32 @@ nxb_status launch_batch(nxb_server* s, Job* j) {
     e = cudaEventRecord(sl->ev_start, st);
     // the meshes end to end: those in this device's memory by one kernel, the
     // others by copies
-    bool gather = false;
     for (uint32_t m = 0; m < M && !e; ++m) {
         const Request* r = j->reqs[m];
         const size_t cap = batch_bvh8_capacity(r->n);
         const bool here = r->on_device && readable(s, r->prims);
         sl->h_places[m] = {here ? r->prims : nullptr, reinterpret_cast<Node8*>(r->result),
                            reinterpret_cast<uint32_t*>(r->result + align_up(sizeof(nxb_bvh8_node) * cap))};
-        gather |= here;
         if (!here)
             e = cudaMemcpyAsync(scratch + prim_bytes(type) * sl->h_off[m], r->prims, prim_bytes(type) * r->n,
                                 r->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st);
     }
-    if (!e) e = cudaMemcpyAsync(a.off, sl->h_off, 4ull * (M + 1), cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemcpyAsync(a.off8, sl->h_off8, 4ull * (M + 1), cudaMemcpyHostToDevice, st);
-    if (!e && gather) e = launch_batch_gather(a, sl->h_places, type, scratch, st);
+    const BatchHost host{sl->h_off, sl->h_off8, sl->h_places, sl->h_meshes, sl->h_err};
+    if (!e) e = launch_batch_gather(a, host, type, scratch, st);
     if (e) return record_cuda_error(e);
     BatchTuning t;
     t.radius = j->reqs[0]->cfg.search_radius ? j->reqs[0]->cfg.search_radius : 8u;
     t.auction = (j->reqs[0]->cfg.flags & NXB_BUILD_AUCTION) != 0;
-    nxb_status stt = batch_enqueue(a, scratch, type, t, sl->h_err, st);
+    nxb_status stt = batch_enqueue(a, scratch, type, t, nullptr, st);
     if (stt != NXB_OK) return stt;
     // each mesh's BVH8 into its request's own result memory
-    e = launch_batch_scatter(a, sl->h_places, st);
+    e = launch_batch_scatter(a, host, st);
     for (uint32_t m = 0; m < M && !e; ++m) {
         Request* r = j->reqs[m];
         r->bvh8.nodes = reinterpret_cast<nxb_bvh8_node*>(sl->h_places[m].nodes);
         r->bvh8.prim_idx = sl->h_places[m].prim_idx;
         r->bvh8.prim_count = r->n;
     }
-    if (!e) e = cudaMemcpyAsync(sl->h_meshes, a.results, sizeof(nxb_batch_mesh) * M, cudaMemcpyDeviceToHost, st);
     if (!e) e = cudaEventRecord(sl->ev_end, st);
     if (!e) e = cudaFreeAsync(scratch, st);
     if (!e) j->scratch = nullptr;

@@ -662,27 +662,36 @@ __device__ __forceinline__ void copy_row(T* __restrict__ dst, const T* __restric
     for (; i < count; i += stride) dst[i] = src[i];
 }
 
-// A grid row per mesh (or several meshes in turn).
-__global__ void batch_gather_kernel(MeshBatch batch, const BatchPlaces* places, uint32_t words, uint32_t* dst) {
-    for (uint32_t m = blockIdx.y; m < batch.meshes; m += gridDim.y) {
+// A grid row per mesh (or several meshes in turn).  Both kernels work on
+// memory of the host too, so that a job needs no copies of its few words.
+__global__ void batch_gather_kernel(MeshBatch host, const BatchPlaces* places, uint32_t words, uint32_t* dst,
+                                    uint32_t* off, uint32_t* off8) {
+    if (blockIdx.x == 0 && blockIdx.y == 0)
+        for (uint32_t m = threadIdx.x; m <= host.meshes; m += blockDim.x) {
+            off[m] = host.off[m];
+            off8[m] = host.off8[m];
+        }
+    for (uint32_t m = blockIdx.y; m < host.meshes; m += gridDim.y) {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(places[m].prims);
-        const MeshSpan me = batch.span(m);
+        const MeshSpan me = host.span(m);
         if (src)  // aligned to words only
             for (uint32_t k = 0; k < words; ++k)
                 copy_row(dst + (size_t)words * me.start + (size_t)k * me.count, src + (size_t)k * me.count, me.count);
     }
 }
 
-__global__ void batch_scatter_kernel(MeshBatch batch, const BatchPlaces* places, const uint32_t* mesh_nodes,
-                                     const Node8* nodes, const uint32_t* prim_idx) {
+__global__ void batch_scatter_kernel(MeshBatch batch, BatchHost h, const uint32_t* mesh_nodes, const Node8* nodes,
+                                     const uint32_t* prim_idx, const nxb_batch_mesh* results, const uint32_t* err) {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *h.err = *err;
     for (uint32_t m = blockIdx.y; m < batch.meshes; m += gridDim.y) {
-        const BatchPlaces to = places[m];
+        const BatchPlaces to = h.places[m];
         const MeshSpan me = batch.span(m);
         const uint32_t first = __ldg(batch.off8 + m), cap = __ldg(batch.off8 + m + 1) - first;
         const uint32_t count = min(__ldg(mesh_nodes + m), cap);
         copy_row(reinterpret_cast<uint4*>(to.nodes), reinterpret_cast<const uint4*>(nodes + first),
                  count * (uint32_t)(sizeof(Node8) / sizeof(uint4)));
         copy_row(to.prim_idx, prim_idx + me.start, me.count);
+        if (blockIdx.x == 0 && threadIdx.x == 0) h.meshes[m] = results[m];
     }
 }
 
@@ -801,17 +810,17 @@ dim3 rows_of(const BatchArena& a) {
     return dim3(std::max(1u, std::min((ctas + rows - 1) / rows, most)), rows);
 }
 
-cudaError_t launch_batch_gather(const BatchArena& a, const BatchPlaces* places, nxb_prim_type type, void* dst,
+cudaError_t launch_batch_gather(const BatchArena& a, const BatchHost& h, nxb_prim_type type, void* dst,
                                 cudaStream_t s) {
-    batch_gather_kernel<<<rows_of(a), 256, 0, s>>>(MeshBatch{a.off, a.off8, a.meshes}, places,
+    batch_gather_kernel<<<rows_of(a), 256, 0, s>>>(MeshBatch{h.off, h.off8, a.meshes}, h.places,
                                                    type == NXB_PRIM_TRIANGLE ? 9u : 6u,
-                                                   reinterpret_cast<uint32_t*>(dst));
+                                                   reinterpret_cast<uint32_t*>(dst), a.off, a.off8);
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_scatter(const BatchArena& a, const BatchPlaces* places, cudaStream_t s) {
-    batch_scatter_kernel<<<rows_of(a), 256, 0, s>>>(MeshBatch{a.off, a.off8, a.meshes}, places, a.mesh_nodes, a.bvh8,
-                                                    a.prim_idx);
+cudaError_t launch_batch_scatter(const BatchArena& a, const BatchHost& h, cudaStream_t s) {
+    batch_scatter_kernel<<<rows_of(a), 256, 0, s>>>(MeshBatch{a.off, a.off8, a.meshes}, h, a.mesh_nodes, a.bvh8,
+                                                    a.prim_idx, a.results, &a.ctrl->error_word);
     return cudaGetLastError();
 }
 
