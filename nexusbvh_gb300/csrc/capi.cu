@@ -64,11 +64,11 @@ Layout make_layout(uint32_t n, uint32_t key_bits) {
     Layout L;
     L.n = n;
     L.key_bytes = key_bits == 30 ? 4 : 8;
-    // 30-bit keys: four 8-bit passes over [2,32); 63-bit keys: the hybrid
+    // 30-bit keys: four 7-bit passes over [2,30), the bits of a code; 63-bit keys: the hybrid
     // sort (launch_sort63_hybrid), whose Morton-fused histograms are those of
     // its four 9-bit top passes and whose look-back storage also serves its
     // eight-pass fallback (the same number of words)
-    L.plan = key_bits == 30 ? make_sort_plan(2, 32) : hybrid63_top_plan();
+    L.plan = key_bits == 30 ? sort30_plan() : hybrid63_top_plan();
     L.tiles_words = key_bits == 30 ? sort_lookback_words(n, L.key_bytes, L.plan.passes)
                                    : sort_lookback_words(n, L.key_bytes, kMaxSortPasses);
     size_t off = 0;
@@ -184,14 +184,8 @@ nxb_status enqueue_build(const void* prims, nxb_prim_type type, uint32_t n, cons
     if (local) {
         NXB_TRY(launch_local_sort(L.key_bytes, keys_a, vals_a, n, s));
     } else if (key_bits == 30) {
-        const size_t tiles_per_pass = L.tiles_words / L.plan.passes;
-        for (int p = 0; p < L.plan.passes; ++p) {
-            const bool even = (p % 2) == 0;
-            NXB_TRY(launch_sort_pass(L.key_bytes, even ? keys_a : keys_b, even ? keys_b : keys_a,
-                                     p == 0 ? nullptr : (even ? vals_a : vals_b), even ? vals_b : vals_a, n,
-                                     L.plan.shift[p], L.plan.bits[p], ctrl->hist[p], lookback + p * tiles_per_pass,
-                                     ctrl->tile_ctr + p, &ctrl->error_word, s));
-        }
+        NXB_TRY(launch_sort30(reinterpret_cast<uint32_t*>(keys_a), reinterpret_cast<uint32_t*>(keys_b), vals_a, vals_b,
+                              n, &ctrl->hist[0][0], lookback, ctrl->tile_ctr, &ctrl->error_word, s));
     } else {
         NXB_TRY(launch_sort63_hybrid(nullptr, nullptr, reinterpret_cast<uint64_t*>(keys_a),
                                      reinterpret_cast<uint64_t*>(keys_b), vals_a, vals_b, n, &ctrl->hist[0][0], lookback,

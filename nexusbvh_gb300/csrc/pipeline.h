@@ -263,6 +263,12 @@ cudaError_t launch_segment_prepare(const SegmentPlan& plan, const MeshBatch& bat
 cudaError_t launch_segment_sort(const SegmentPlan& plan, const MeshBatch& batch, uint32_t total, uint64_t* keys_a,
                                 uint64_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t* tile_ctr,
                                 uint32_t* err, cudaStream_t s);
+// The pipeline's 30-bit codes (bits [2, 30); plan: sort30_plan) in the same
+// passes; keys and the permutation end in keys_a and vals_a.  hist: kRadixBins
+// words per pass; look-back words and counters zero on entry.
+inline SortPlan sort30_plan() { return make_sort_plan(2, 30, kSegmentBits); }
+cudaError_t launch_sort30(uint32_t* keys_a, uint32_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t n,
+                          uint32_t* hist, uint32_t* lookback, uint32_t* tile_ctr, uint32_t* err, cudaStream_t s);
 // ---------------------------------------------------------------- stage 4
 // parent: n words holding INVALID on entry; parent_of_last: one word that
 // must hold INVALID on entry; tile_ctr: one word that must be zero on entry.

@@ -1126,10 +1126,14 @@ __global__ __launch_bounds__(kThreads) void segment_prepare_kernel(SegmentPlan p
     for (size_t i = tid; i < vec4; i += stride) reinterpret_cast<uint4*>(plan.hist)[i] = make_uint4(0, 0, 0, 0);
 }
 
-template <bool FIRST, bool LAST>
+// A plain build's 30-bit codes take the same passes as one segment (its
+// histograms are kRadixBins apart): 12.58M codes 363 us and Morton 88, 6.0M
+// 201 and 43, 1.0M 76 and 14, where onesweep32_kernel's passes over bits
+// [2, 32) take 389 and 93, 219 and 48, 76 and 16.
+template <typename Seg, bool FIRST, bool LAST>
 __global__ __launch_bounds__(kThreads, FIRST ? 5 : 4) void segment_pass_kernel(
     const uint32_t* __restrict__ kin, void* __restrict__ kout, const uint32_t* __restrict__ vin,
-    uint32_t* __restrict__ vout, MeshBatch batch, SegmentPlan plan, uint32_t pass, uint32_t* tile_ctr, uint32_t* err) {
+    uint32_t* __restrict__ vout, Seg seg, SegmentPlan plan, uint32_t pass, uint32_t* tile_ctr, uint32_t* err) {
     constexpr int KPT = kSegmentTile / kThreads;
     constexpr uint32_t BINS = kSegmentBins;
     static_assert(BINS <= kThreads, "a thread per digit");
@@ -1143,14 +1147,21 @@ __global__ __launch_bounds__(kThreads, FIRST ? 5 : 4) void segment_pass_kernel(
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= plan.tiles) return;
-    const MeshSpan mesh = batch.span(__ldg(plan.mesh_of + tile));
-    const uint32_t nth = tile - (mesh.start / kSegmentTile + mesh.m);  // of the mesh's tiles
+    MeshSpan mesh;
+    uint32_t nth;  // of the mesh's tiles
+    if constexpr (Seg::kBatch) {
+        mesh = seg.span(__ldg(plan.mesh_of + tile));
+        nth = tile - (mesh.start / kSegmentTile + mesh.m);
+    } else {
+        mesh = seg.of_prim(0);
+        nth = tile;
+    }
     const uint32_t base = nth * kSegmentTile, n = mesh.count;
     if (base >= n) return;
     kin += mesh.start;
     if (!FIRST) vin += mesh.start;
     vout += mesh.start;
-    const uint32_t* hist = plan.hist + ((size_t)mesh.m * kSegmentPasses + pass) * BINS;
+    const uint32_t* hist = plan.hist + (Seg::kBatch ? ((size_t)mesh.m * kSegmentPasses + pass) * BINS : pass * kRadixBins);
     uint32_t* lookback = plan.lookback + ((size_t)pass * plan.tiles + tile) * BINS;
 
     uint32_t key[KPT], val[KPT], rank[KPT];
@@ -1245,7 +1256,7 @@ __global__ __launch_bounds__(kThreads, FIRST ? 5 : 4) void segment_pass_kernel(
         const uint32_t k = s_keys[i];
         const uint32_t g = s_delta[(k >> shift) & (BINS - 1)] + i;
         if (g < n) {  // always true unless a look-back wait expired
-            if (LAST)
+            if (LAST && Seg::kBatch)
                 reinterpret_cast<uint64_t*>(kout)[mesh.start + g] = ((uint64_t)mesh.m << 32) | k;
             else
                 reinterpret_cast<uint32_t*>(kout)[mesh.start + g] = k;
@@ -1322,8 +1333,9 @@ cudaError_t launch_local_sort_batch(uint64_t* keys, uint32_t* vals, const MeshBa
 
 cudaError_t load_sort_kernels() {
     cudaError_t e = load_kernels(bucket_sort_kernel, sort_fallback_kernel<uint64_t>, segment_prepare_kernel,
-                                 segment_pass_kernel<true, false>, segment_pass_kernel<false, false>,
-                                 segment_pass_kernel<false, true>);
+                                 segment_pass_kernel<MeshBatch, true, false>, segment_pass_kernel<MeshBatch, false, false>,
+                                 segment_pass_kernel<MeshBatch, false, true>, segment_pass_kernel<SingleMesh, true, false>,
+                                 segment_pass_kernel<SingleMesh, false, false>);
     for (int form = 0; form < 4 && !e; ++form)
         e = load_kernels(onesweep_of<uint32_t, kRadixBits>(form & 1, form & 2),
                          onesweep_of<uint64_t, kRadixBits>(form & 1, form & 2),
@@ -1371,8 +1383,8 @@ cudaError_t launch_segment_sort(const SegmentPlan& plan, const MeshBatch& batch,
                                 uint32_t* err, cudaStream_t s) {
     const cudaError_t e = once_per_device([] {
         cudaError_t r = cudaSuccess;
-        for (auto* kernel : {segment_pass_kernel<true, false>, segment_pass_kernel<false, false>,
-                             segment_pass_kernel<false, true>})
+        for (auto* kernel : {segment_pass_kernel<MeshBatch, true, false>, segment_pass_kernel<MeshBatch, false, false>,
+                             segment_pass_kernel<MeshBatch, false, true>})
             if (!r)
                 r = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared);
@@ -1381,14 +1393,39 @@ cudaError_t launch_segment_sort(const SegmentPlan& plan, const MeshBatch& batch,
     if (e) return e;
     uint32_t* k0 = reinterpret_cast<uint32_t*>(keys_b);  // the passes go to and fro in the halves of keys_b
     uint32_t* k1 = k0 + total;
-    segment_pass_kernel<true, false>
+    segment_pass_kernel<MeshBatch, true, false>
         <<<plan.tiles, kThreads, 0, s>>>(k0, k1, nullptr, vals_b, batch, plan, 0, tile_ctr, err);
-    segment_pass_kernel<false, false>
+    segment_pass_kernel<MeshBatch, false, false>
         <<<plan.tiles, kThreads, 0, s>>>(k1, k0, vals_b, vals_a, batch, plan, 1, tile_ctr, err);
-    segment_pass_kernel<false, false>
+    segment_pass_kernel<MeshBatch, false, false>
         <<<plan.tiles, kThreads, 0, s>>>(k0, k1, vals_a, vals_b, batch, plan, 2, tile_ctr, err);
-    segment_pass_kernel<false, true>
+    segment_pass_kernel<MeshBatch, false, true>
         <<<plan.tiles, kThreads, 0, s>>>(k1, keys_a, vals_b, vals_a, batch, plan, 3, tile_ctr, err);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sort30(uint32_t* keys_a, uint32_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t n,
+                          uint32_t* hist, uint32_t* lookback, uint32_t* tile_ctr, uint32_t* err, cudaStream_t s) {
+    const cudaError_t e = once_per_device([] {
+        cudaError_t r = cudaSuccess;
+        for (auto* kernel : {segment_pass_kernel<SingleMesh, true, false>, segment_pass_kernel<SingleMesh, false, false>})
+            if (!r)
+                r = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         cudaSharedmemCarveoutMaxShared);
+        return r;
+    });
+    if (e) return e;
+    SegmentPlan plan{};
+    plan.tiles = (n + kSegmentTile - 1) / kSegmentTile;
+    plan.hist = hist;
+    plan.lookback = lookback;
+    const SingleMesh seg{n};
+    for (uint32_t p = 0; p < kSegmentPasses; ++p) {
+        const bool even = p % 2 == 0;
+        auto* kernel = p == 0 ? segment_pass_kernel<SingleMesh, true, false> : segment_pass_kernel<SingleMesh, false, false>;
+        kernel<<<plan.tiles, kThreads, 0, s>>>(even ? keys_a : keys_b, even ? keys_b : keys_a, even ? vals_a : vals_b,
+                                               even ? vals_b : vals_a, seg, plan, p, tile_ctr, err);
+    }
     return cudaGetLastError();
 }
 

@@ -39,3 +39,20 @@ def test_meshes(gpu, case, kind):
         if n:
             out = S.build_async(np.ascontiguousarray(prims[off[m]:off[m + 1]]), 30)
             assert batch.mesh_bvh2_host(m, meshes).tobytes() == S.nodes2(out.bvh2.nodes.view(-1)).tobytes()
+
+
+@pytest.mark.parametrize("kind", ["spread", "equal", "few"])
+@pytest.mark.parametrize("n", [65_537, 69_632, 69_633, 131_071, 1_000_001])
+def test_plain_30_bit_builds(gpu, n, kind):
+    """The same passes with the whole build as one segment, against the stage
+    chain, whose sort takes the onesweep passes over bits [2, 32)."""
+    prims = scenes.uniform_soup(n, seed=n)
+    if kind == "equal":
+        prims[:] = prims[0]
+    elif kind == "few":
+        prims = prims[np.random.default_rng(n).integers(0, 37, n)]
+    prims = np.ascontiguousarray(prims)
+    d_nodes, d_scene = S.stage_bounds(prims)
+    d_sk, d_perm = S.stage_sort(S.stage_morton(d_nodes, d_scene, n, 30), n, 30)
+    want = S.host(S.stage_hploc(d_sk, d_perm, d_nodes, n, 30))
+    assert S.host(S.build_async(prims, 30).bvh2.nodes.view(-1)).tobytes() == want.tobytes()
