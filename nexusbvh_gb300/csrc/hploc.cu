@@ -5,7 +5,7 @@
 // identical; how they are computed on the GPU differs:
 //   * the bottom-up LBVH climb (Apetrei 2014; FindParentId/Delta,
 //     BinaryBuilder.cu:14-40) is cut into tiles of consecutive sorted leaves.
-//     One CTA loads a tile's key deltas, ids and leaf boxes into shared
+//     A warp loads a tile's key deltas, ids and leaf boxes into shared
 //     memory once, and every LBVH node whose range lies inside the tile is
 //     climbed to, merged and handed over there; only subtrees that touch the
 //     tile's edge publish their clusters and climb on through global

@@ -5,7 +5,7 @@
 // [1,64) of 64-bit keys, carrying the full keys.  Written from the published
 // onesweep algorithm (Adinets & Merrill 2022): the digit histograms of all
 // passes come from one up-front read (fused into the Morton kernel), then
-// one kernel per 8-bit digit:
+// one kernel per digit:
 //   * tiles are claimed in order through an atomic counter, so a tile only
 //     ever waits on tiles that are already running;
 //   * each warp ranks its keys stably with ballots over the digit bits;
@@ -14,6 +14,9 @@
 //     on expiry the error word is set and the kernel finishes);
 //   * keys are reordered in shared memory so that the global scatter writes
 //     runs of consecutive addresses.
+// Three forms: onesweep kernels (63-bit keys, callers' keys), segmented passes
+// (30-bit codes, of one mesh or of each mesh of a batch), and one launch of
+// thread-block clusters (up to 65,536 keys of a mesh).
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -1337,8 +1340,7 @@ cudaError_t load_sort_kernels() {
                                  segment_pass_kernel<MeshBatch, false, true>, segment_pass_kernel<SingleMesh, true, false>,
                                  segment_pass_kernel<SingleMesh, false, false>);
     for (int form = 0; form < 4 && !e; ++form)
-        e = load_kernels(onesweep_of<uint32_t, kRadixBits>(form & 1, form & 2),
-                         onesweep_of<uint64_t, kRadixBits>(form & 1, form & 2),
+        e = load_kernels(onesweep_of<uint64_t, kRadixBits>(form & 1, form & 2),
                          onesweep_of<uint64_t, kMaxRadixBits>(form & 1, form & 2));
     auto local = [&](auto kpt) {
         constexpr int k = decltype(kpt)::value;

@@ -23,7 +23,10 @@
 //     Measured on GB300 at 12.58M clustered triangles: BVH8 0.833 ->
 //     0.553 ms, H-PLOC 2.16 -> 2.34 ms (the records' stores), build 3.91 ->
 //     3.81 ms; the BVH8 kernel's time hardly depends on its occupancy (3 / 6
-//     CTAs per SM: 0.898 / 0.833 ms), it follows the random node traffic.
+//     CTAs per SM: 0.898 / 0.833 ms), it follows the random node traffic;
+//   * small greedy collapses, which are chains of levels, read every node's
+//     children and slots from lists made beforehand, and auctions take eight
+//     lanes per item (takes_lists, takes_groups).
 // The decisions are the reference's:
 //   * expansion always re-opens the highest-indexed inner child, the child
 //     with the smaller area going to the re-opened position (:284-330);
