@@ -803,23 +803,43 @@ __global__ __launch_bounds__(kThreads, 4) void sort_fallback_kernel(K* ka, K* kb
 //
 // What bounds it: the chain of steps of a pass (2 us in one CTA, 6 to 8 in a
 // cluster), not bandwidth.  The sort stage on GB300, onesweep passes -> this:
-// 1,021 30-bit keys 35.5 -> 9.9 us, 32,000 44 -> 24, 65,536 47.7 -> 32.4;
-// 16,411 63-bit keys 60 -> 45.  Stores to peers straight from the ranking
-// order, without sorting the CTA's keys by digit first, took 46.7 us at
-// 65,536 keys: one request per lane instead of runs.
+// 1,021 30-bit keys 35.5 -> 9.9 us, 32,000 44 -> 22, 65,536 47.7 -> 30.5;
+// 16,411 63-bit keys 60 -> 42.6, 32,000 47.5.  Stores to peers straight from
+// the ranking order, without sorting the CTA's keys by digit first, took 46.7
+// us at 65,536 keys: one request per lane instead of runs.  Keys and values
+// stored apart, two requests per key: 65,536 32.4, 16,411 45, 32,000 53.  Of a
+// pass at 65,536 keys (7.6 us then) the ranking took 1.7, the counts and
+// their barrier 1.5, the stores and theirs 3.3.
 constexpr int kLocalThreads = 512;
 constexpr int kLocalWarps = kLocalThreads / 32;
 constexpr uint32_t kLocalMaxCtas = 16;
 constexpr int kLocalMaxKpt = 8;
-constexpr uint32_t kLocalMaxKeys = kLocalMaxCtas * kLocalThreads * kLocalMaxKpt;  // 65,536
+constexpr uint32_t kLocalMaxKeys = kLocalMaxCtas * kLocalThreads * kLocalMaxKpt;  // 65,536 (16-bit positions)
 
-template <typename K, int RB, int KPT>
+// A key with its position as one element, so that a pass has one store per
+// key to another CTA, not two: a 30-bit code above a position below 2^16, or
+// a 64-bit key beside one.
+constexpr uint32_t kPackBits = 16;
+struct __align__(16) KeyPos {
+    uint64_t key;
+    uint32_t pos, unused;
+};
+__device__ __forceinline__ void make_element(uint64_t& e, uint32_t code, uint32_t pos) {
+    e = (uint64_t)code << kPackBits | pos;
+}
+__device__ __forceinline__ void make_element(KeyPos& e, uint64_t key, uint32_t pos) { e = {key, pos, 0u}; }
+__device__ __forceinline__ uint64_t key_bits_of(uint64_t e) { return e >> kPackBits; }
+__device__ __forceinline__ uint64_t key_bits_of(const KeyPos& e) { return e.key; }
+__device__ __forceinline__ uint32_t pos_of(uint64_t e) { return (uint32_t)e & ((1u << kPackBits) - 1u); }
+__device__ __forceinline__ uint32_t pos_of(const KeyPos& e) { return e.pos; }
+template <typename K>
+using Element = std::conditional_t<sizeof(K) == 4, uint64_t, KeyPos>;
+
+template <typename E, int RB, int KPT>
 struct __align__(16) LocalSmem {
     static constexpr int kTile = kLocalThreads * KPT, kBins = 1 << RB;
-    K key[kTile];
-    K out_key[kTile];  // a pass's keys in digit order, on their way to other CTAs
-    uint32_t val[kTile];
-    uint32_t out_val[kTile];
+    E key[kTile];
+    E out_key[kTile];  // a pass's keys in digit order, on their way to other CTAs
     uint16_t wh[kLocalWarps][kBins];  // per-warp digit counts, then offsets
     uint32_t cnt[kBins];              // this CTA's digit counts, read by the cluster
     uint32_t base[kBins];             // first position of this CTA's keys of a digit
@@ -848,20 +868,19 @@ __device__ __forceinline__ uint32_t ld_peer(uint32_t a) {
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_peer(uint32_t a, uint32_t v) {
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
 __device__ __forceinline__ void st_peer(uint32_t a, uint64_t v) {
     asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
+__device__ __forceinline__ void st_peer(uint32_t a, const KeyPos& v) {
+    asm volatile("st.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(a), "l"(v.key), "l"((uint64_t)v.pos) : "memory");
+}
 
-// Sorts `count` keys, loaded by the caller into key/val of the cluster's
-// CTAs in order, stably on `passes` digits of RB bits from bit `shift` on.
+// Sorts `count` keys, loaded by the caller into the cluster's CTAs in order, stably on `passes` digits of RB bits from bit `shift` on.
 // ctas: CTAs of the cluster (uniform); me: this CTA's rank in it.
-template <typename K, int RB, int KPT>
-__device__ __forceinline__ void local_sort(LocalSmem<K, RB, KPT>& sm, uint32_t count, uint32_t shift, int passes,
+template <typename E, int RB, int KPT>
+__device__ __forceinline__ void local_sort(LocalSmem<E, RB, KPT>& sm, uint32_t count, uint32_t shift, int passes,
                                            uint32_t ctas, uint32_t me) {
-    using S = LocalSmem<K, RB, KPT>;
+    using S = LocalSmem<E, RB, KPT>;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     const uint32_t first = me * S::kTile;
     const uint32_t own = warp * 32u * KPT + lane;
@@ -869,18 +888,17 @@ __device__ __forceinline__ void local_sort(LocalSmem<K, RB, KPT>& sm, uint32_t c
     const uint32_t lt_mask = lanemask_lt();
     for (int p = 0; p < passes; ++p, shift += RB) {
         for (uint32_t i = lane; i < S::kBins / 2; i += 32) reinterpret_cast<uint32_t*>(wh)[i] = 0;
-        K key[KPT];
-        uint32_t val[KPT], rank[KPT];
+        E key[KPT];
+        uint32_t rank[KPT];
 #pragma unroll
         for (int j = 0; j < KPT; ++j) {
             key[j] = sm.key[own + 32 * j];
-            val[j] = sm.val[own + 32 * j];
         }
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < KPT; ++j) {
             const bool valid = first + own + 32 * j < count;
-            const uint32_t d = (uint32_t)(key[j] >> shift) & (S::kBins - 1u);
+            const uint32_t d = (uint32_t)(key_bits_of(key[j]) >> shift) & (S::kBins - 1u);
             uint32_t peers = __ballot_sync(kFullMask, valid);
 #pragma unroll
             for (int b = 0; b < RB; ++b) {
@@ -945,14 +963,12 @@ __device__ __forceinline__ void local_sort(LocalSmem<K, RB, KPT>& sm, uint32_t c
         }
         __syncthreads();
         // into digit order in this CTA; one CTA: that is the pass
-        K* ok = ctas > 1 ? sm.out_key : sm.key;
-        uint32_t* ov = ctas > 1 ? sm.out_val : sm.val;
+        E* ok = ctas > 1 ? sm.out_key : sm.key;
 #pragma unroll
         for (int j = 0; j < KPT; ++j) {
             if (first + own + 32 * j < count) {
-                const uint32_t k = wh[(uint32_t)(key[j] >> shift) & (S::kBins - 1u)] + rank[j];
+                const uint32_t k = wh[(uint32_t)(key_bits_of(key[j]) >> shift) & (S::kBins - 1u)] + rank[j];
                 ok[k] = key[j];
-                ov[k] = val[j];
             }
         }
         __syncthreads();
@@ -962,11 +978,10 @@ __device__ __forceinline__ void local_sort(LocalSmem<K, RB, KPT>& sm, uint32_t c
             for (int j = 0; j < KPT; ++j) {
                 const uint32_t k = tid + j * kLocalThreads;
                 if (first + k < count) {
-                    const K kk = sm.out_key[k];
-                    const uint32_t to = sm.base[(uint32_t)(kk >> shift) & (S::kBins - 1u)] + k;
+                    const E kk = sm.out_key[k];
+                    const uint32_t to = sm.base[(uint32_t)(key_bits_of(kk) >> shift) & (S::kBins - 1u)] + k;
                     const uint32_t r = to / S::kTile, q = to % S::kTile;
                     st_peer(peer_addr(&sm.key[q], r), kk);
-                    st_peer(peer_addr(&sm.val[q], r), sm.out_val[k]);
                 }
             }
             cluster_sync();
@@ -980,23 +995,22 @@ __global__ __launch_bounds__(kLocalThreads) void sort_cluster_kernel(K* keys, ui
                                                                      uint32_t shift, int passes) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
-    LocalSmem<K, RB, KPT>& sm = *reinterpret_cast<LocalSmem<K, RB, KPT>*>(smem);
-    constexpr uint32_t T = LocalSmem<K, RB, KPT>::kTile;
-    const uint32_t me = cluster_rank(), first = me * T;
+    using S = LocalSmem<Element<K>, RB, KPT>;
+    S& sm = *reinterpret_cast<S*>(smem);
+    const uint32_t me = cluster_rank(), first = me * S::kTile;
 #pragma unroll
     for (int j = 0; j < KPT; ++j) {
         const uint32_t k = threadIdx.x + j * kLocalThreads;
-        sm.key[k] = first + k < n ? __ldcg(keys + first + k) : (K)0;
-        sm.val[k] = first + k;
+        make_element(sm.key[k], first + k < n ? __ldcg(keys + first + k) : (K)0, first + k);
     }
     __syncthreads();
-    local_sort<K, RB, KPT>(sm, n, shift, passes, gridDim.x, me);
+    local_sort<Element<K>, RB, KPT>(sm, n, shift, passes, gridDim.x, me);
 #pragma unroll
     for (int j = 0; j < KPT; ++j) {
         const uint32_t k = threadIdx.x + j * kLocalThreads;
         if (first + k < n) {
-            keys[first + k] = sm.key[k];
-            vals[first + k] = sm.val[k];
+            keys[first + k] = (K)key_bits_of(sm.key[k]);
+            vals[first + k] = pos_of(sm.key[k]);
         }
     }
 }
@@ -1007,25 +1021,24 @@ __global__ __launch_bounds__(kLocalThreads) void sort_cluster_batch_kernel(uint6
                                                                            MeshBatch batch, uint32_t ctas,
                                                                            uint32_t shift, int passes) {
     extern __shared__ __align__(16) unsigned char smem[];
-    LocalSmem<uint32_t, RB, KPT>& sm = *reinterpret_cast<LocalSmem<uint32_t, RB, KPT>*>(smem);
-    constexpr uint32_t T = LocalSmem<uint32_t, RB, KPT>::kTile;
+    using S = LocalSmem<uint64_t, RB, KPT>;
+    S& sm = *reinterpret_cast<S*>(smem);
     const MeshSpan mesh = batch.span(blockIdx.x / ctas);
     if (mesh.count == 0) return;  // the whole cluster
-    const uint32_t me = ctas > 1 ? cluster_rank() : 0u, first = me * T;
+    const uint32_t me = ctas > 1 ? cluster_rank() : 0u, first = me * S::kTile;
 #pragma unroll
     for (int j = 0; j < KPT; ++j) {
         const uint32_t k = threadIdx.x + j * kLocalThreads;
-        sm.key[k] = first + k < mesh.count ? (uint32_t)__ldcg(keys + mesh.start + first + k) : 0u;
-        sm.val[k] = first + k;
+        make_element(sm.key[k], first + k < mesh.count ? (uint32_t)__ldcg(keys + mesh.start + first + k) : 0u, first + k);
     }
     __syncthreads();
-    local_sort<uint32_t, RB, KPT>(sm, mesh.count, shift, passes, ctas, me);
+    local_sort<uint64_t, RB, KPT>(sm, mesh.count, shift, passes, ctas, me);
 #pragma unroll
     for (int j = 0; j < KPT; ++j) {
         const uint32_t k = threadIdx.x + j * kLocalThreads;
         if (first + k < mesh.count) {
-            keys[mesh.start + first + k] = ((uint64_t)mesh.m << 32) | sm.key[k];
-            vals[mesh.start + first + k] = sm.val[k];
+            keys[mesh.start + first + k] = ((uint64_t)mesh.m << 32) | key_bits_of(sm.key[k]);
+            vals[mesh.start + first + k] = pos_of(sm.key[k]);
         }
     }
 }
@@ -1064,10 +1077,10 @@ cudaLaunchConfig_t local_config(uint32_t grid, uint32_t ctas, size_t smem, cudaS
 }
 template <typename K, int RB, int KPT>
 cudaError_t launch_local(K* keys, uint32_t* vals, uint32_t n, uint32_t shift, int passes, cudaStream_t s) {
-    constexpr size_t smem = sizeof(LocalSmem<K, RB, KPT>);
+    constexpr size_t smem = sizeof(LocalSmem<Element<K>, RB, KPT>);
     cudaError_t e = once_per_device([] { return local_attributes(sort_cluster_kernel<K, RB, KPT>, smem); });
     if (e) return e;
-    constexpr uint32_t T = LocalSmem<K, RB, KPT>::kTile;
+    constexpr uint32_t T = kLocalThreads * KPT;
     const uint32_t ctas = (n + T - 1) / T;
     cudaLaunchAttribute attr[2]{};
     cudaLaunchConfig_t c = local_config(ctas, ctas, smem, s, attr, true);
@@ -1076,10 +1089,10 @@ cudaError_t launch_local(K* keys, uint32_t* vals, uint32_t n, uint32_t shift, in
 template <int RB, int KPT>
 cudaError_t launch_local_batch(uint64_t* keys, uint32_t* vals, const MeshBatch& batch, uint32_t max_mesh, uint32_t shift,
                                int passes, cudaStream_t s) {
-    constexpr size_t smem = sizeof(LocalSmem<uint32_t, RB, KPT>);
+    constexpr size_t smem = sizeof(LocalSmem<uint64_t, RB, KPT>);
     cudaError_t e = once_per_device([] { return local_attributes(sort_cluster_batch_kernel<RB, KPT>, smem); });
     if (e) return e;
-    constexpr uint32_t T = LocalSmem<uint32_t, RB, KPT>::kTile;
+    constexpr uint32_t T = kLocalThreads * KPT;
     const uint32_t ctas = (max_mesh + T - 1) / T;
     cudaLaunchAttribute attr[2]{};
     cudaLaunchConfig_t c = local_config(ctas * batch.meshes, ctas, smem, s, attr, false);
@@ -1306,7 +1319,7 @@ bool local_sort_takes(uint32_t n) {
     if (n > kLocalMaxKeys) return false;
     const cudaError_t e = once_per_device([] {
         auto* kernel = sort_cluster_kernel<uint64_t, kLocalBits64, kLocalMaxKpt>;
-        constexpr size_t smem = sizeof(LocalSmem<uint64_t, kLocalBits64, kLocalMaxKpt>);
+        constexpr size_t smem = sizeof(LocalSmem<KeyPos, kLocalBits64, kLocalMaxKpt>);
         cudaError_t r = local_attributes(kernel, smem);
         cudaLaunchAttribute attr[2]{};
         const cudaLaunchConfig_t c = local_config(kLocalMaxCtas, kLocalMaxCtas, smem, nullptr, attr, true);
