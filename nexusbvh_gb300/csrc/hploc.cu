@@ -842,6 +842,7 @@ cudaError_t launch_t(const K* keys, const uint32_t* cluster, uint32_t* parent, N
                      uint32_t end, uint32_t radius, uint32_t* pol, uint32_t* tile_ctr, uint32_t* err,
                      uint32_t max_per_sm, cudaStream_t s, Node2* rec, uint64_t* pairs, uint32_t* ctr,
                      ChildPair* kids) {
+    if (begin == end) return cudaSuccess;  // a batch's group of empty meshes has nothing to climb
     // one tile per resident warp while that is at most kTile leaves, so that
     // small builds use every SM: 65,536 triangles take 71 us with 32 leaves
     // per tile, 88 with 144.  The smallest tile is a window and a little: whole
