@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import threading
 from pathlib import Path
 
 import numpy as np
@@ -282,6 +283,18 @@ class BVH8:
     bvh2: BVH2 | None = None
 
 
+_pinned = threading.local()
+
+
+def _host_result():
+    """The calling thread's pinned copy of a build result (threads may share a
+    ``Builder``, and each reads its result after its own wait)."""
+    import torch
+    if not hasattr(_pinned, "result"):
+        _pinned.result = torch.empty(ctypes.sizeof(CResult), dtype=torch.uint8, pin_memory=True)
+    return _pinned.result
+
+
 class Builder:
     """Keeps a workspace resident across builds and drives ``nxb_build_async``.
 
@@ -292,7 +305,6 @@ class Builder:
     def __init__(self):
         load()
         self._ws = None
-        self._host_result = None  # pinned copy of the build result
 
     def sizes(self, n: int, config: BuildConfig) -> CSizes:
         s = CSizes()
@@ -324,11 +336,10 @@ class Builder:
         prim_idx = torch.empty(n, dtype=torch.int32, device="cuda") if wide else None
         result = torch.empty(ctypes.sizeof(CResult), dtype=torch.uint8, device="cuda")  # the build writes all of it
         self.enqueue(prims, n, config, ws, bvh2_nodes, bvh8_nodes, prim_idx, result)
-        if self._host_result is None:
-            self._host_result = torch.empty(ctypes.sizeof(CResult), dtype=torch.uint8, pin_memory=True)
-        self._host_result.copy_(result, non_blocking=True)
+        host = _host_result()
+        host.copy_(result, non_blocking=True)
         torch.cuda.current_stream().synchronize()
-        r = CResult.from_buffer_copy(self._host_result.numpy())
+        r = CResult.from_buffer_copy(host.numpy())
         if r.error_word:
             raise NxbError(7 if not (r.error_word & 3) else 6, f"device error word 0x{r.error_word:x}")
         bounds = (tuple(r.scene_bounds.bmin), tuple(r.scene_bounds.bmax))
