@@ -148,14 +148,33 @@ __device__ __forceinline__ uint32_t atom_exch_acq_rel(uint32_t* p, uint32_t v) {
     return old;
 }
 
-// Box of a BVH2 node read through L2 (data written by other CTAs).
 // For kernels launched by launch_after (pipeline.h): waits for the kernel
 // before in the stream, which has then finished and whose writes are seen,
 // and lets the one after be set up meanwhile.  Nothing another kernel writes
-// or reads is touched before it.
+// or reads is touched before it.  What the kernel before wrote, it wrote
+// while this one's grid was already there, so it is read by ordinary loads:
+// the read-only path (ld.global.nc, which the compiler also takes for
+// `const __restrict__` parameters) is only defined for memory that nobody
+// writes as long as the grid exists, and may be moved above the wait.
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Streaming loads (evicted first) that stay behind after_previous().
+__device__ __forceinline__ float ld_stream(const float* p) {
+    float v;
+    asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_stream(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.cs.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
 }
 __device__ __forceinline__ Box load_box_cg(const Node2* nodes, uint32_t i) {
     const float4* p = reinterpret_cast<const float4*>(nodes + i);
@@ -168,8 +187,8 @@ __device__ __forceinline__ Box load_box_cg(const Node2* nodes, uint32_t i) {
 }
 __device__ __forceinline__ Box load_box(const Node2* nodes, uint32_t i) {
     const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    float4 a = __ldg(p);
-    float2 b = __ldg(reinterpret_cast<const float2*>(p + 1));
+    const float4 a = *p;
+    const float2 b = *reinterpret_cast<const float2*>(p + 1);
     Box r;
     r.mn = make_float3(a.x, a.y, a.z);
     r.mx = make_float3(a.w, b.x, b.y);
@@ -204,10 +223,9 @@ __device__ __forceinline__ void store_child_pair(ChildPair* p, const Box& l, con
                              __float_as_uint(r.mx.z)));
     __stcg(q + 3, make_uint4(li, ri, 0u, 0u));
 }
-// Through the read-only path: the records are finished by an earlier kernel.
 __device__ __forceinline__ ChildPair load_child_pair(const ChildPair* p) {
     const uint4* q = reinterpret_cast<const uint4*>(p);
-    const uint4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3);
+    const uint4 a = q[0], b = q[1], c = q[2], d = q[3];
     ChildPair r;
     r.l.mn = make_float3(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z));
     r.l.mx = make_float3(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y));

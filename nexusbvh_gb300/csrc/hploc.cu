@@ -40,20 +40,20 @@ constexpr uint32_t kMergeThreshold = 16;  // MERGING_THRESHOLD, BinaryBuilder.cu
 // Delta (BinaryBuilder.cu:16-28) of sorted positions a and b of the mesh
 // whose first position is s; the index tie-break uses mesh-local positions.
 __device__ __forceinline__ uint64_t delta(const uint32_t* k, uint32_t a, uint32_t b, uint32_t s) {
-    return (((uint64_t)__ldg(k + a) << 32) | (a - s)) ^ (((uint64_t)__ldg(k + b) << 32) | (b - s));
+    return (((uint64_t)k[a] << 32) | (a - s)) ^ (((uint64_t)k[b] << 32) | (b - s));
 }
 __device__ __forceinline__ uint64_t delta(const uint64_t* k, uint32_t a, uint32_t b, uint32_t s) {
-    const uint64_t d = __ldg(k + a) ^ __ldg(k + b);
+    const uint64_t d = k[a] ^ k[b];
     return d ? d : (uint64_t)((a - s) ^ (b - s));
 }
 // Batched 30-bit keys: mesh << 32 | code, sorted as one key; the delta is
 // the 32-bit one of the code.
 __device__ __forceinline__ uint64_t delta(const MeshKey* k, uint32_t a, uint32_t b, uint32_t s) {
-    const uint32_t ka = (uint32_t)__ldg(&k[a].v), kb = (uint32_t)__ldg(&k[b].v);
+    const uint32_t ka = (uint32_t)k[a].v, kb = (uint32_t)k[b].v;
     return (((uint64_t)ka << 32) | (a - s)) ^ (((uint64_t)kb << 32) | (b - s));
 }
 // The mesh of sorted position p (the high half of its key).
-__device__ __forceinline__ uint32_t mesh_of(const MeshKey* k, uint32_t p) { return (uint32_t)(__ldg(&k[p].v) >> 32); }
+__device__ __forceinline__ uint32_t mesh_of(const MeshKey* k, uint32_t p) { return (uint32_t)(k[p].v >> 32); }
 template <typename K>
 __device__ __forceinline__ uint32_t mesh_of(const K*, uint32_t) {
     return 0;
@@ -512,7 +512,7 @@ __device__ __forceinline__ void load_tile(const Climb<K, Seg>& g, WarpTile<R>& t
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
         const uint32_t j = lane + 32 * q;
-        id[q] = j < cnt ? __ldcg(g.cluster + base + j) : kInvalid;
+        id[q] = j < cnt ? g.cluster[base + j] : kInvalid;
     }
 #pragma unroll
     for (int q = 0; q <= kPer; ++q) {

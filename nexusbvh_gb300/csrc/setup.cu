@@ -23,8 +23,8 @@ namespace {
 constexpr int kThreads = 256;
 
 template <int FLOATS>
-__global__ __launch_bounds__(kThreads) void scene_bounds_kernel(const float* __restrict__ prims, uint32_t n,
-                                                                Node2* __restrict__ nodes, uint32_t* scene_ord,
+__global__ __launch_bounds__(kThreads) void scene_bounds_kernel(const float* prims, uint32_t n,
+                                                                Node2* nodes, uint32_t* scene_ord,
                                                                 bool aligned16) {
     after_previous();
     __shared__ __align__(16) float tile[kThreads * FLOATS];
@@ -43,9 +43,9 @@ __global__ __launch_bounds__(kThreads) void scene_bounds_kernel(const float* __r
             const float4* s4 = reinterpret_cast<const float4*>(src);
             float4* d4 = reinterpret_cast<float4*>(tile);
 #pragma unroll
-            for (int v = threadIdx.x; v < V; v += kThreads) d4[v] = __ldcs(s4 + v);
+            for (int v = threadIdx.x; v < V; v += kThreads) d4[v] = ld_stream(s4 + v);
         } else {
-            for (uint32_t v = threadIdx.x; v < cnt * FLOATS; v += kThreads) tile[v] = __ldcs(src + v);
+            for (uint32_t v = threadIdx.x; v < cnt * FLOATS; v += kThreads) tile[v] = ld_stream(src + v);
         }
         __syncthreads();
         if (threadIdx.x < cnt) {
@@ -154,8 +154,8 @@ struct MortonArgs {
 // loop unrolls.  BINS: digits per pass (256, or 512 for 9-bit digits); the
 // histograms are laid out pass after pass, BINS words each.
 template <typename K, bool HIST, int PASSES = 0, int BINS = kRadixBins>
-__global__ __launch_bounds__(kThreads) void morton_kernel(const Node2* __restrict__ nodes, uint32_t n, Control* ctrl,
-                                                          K* __restrict__ keys, MortonArgs a) {
+__global__ __launch_bounds__(kThreads) void morton_kernel(const Node2* nodes, uint32_t n, Control* ctrl,
+                                                          K* keys, MortonArgs a) {
     after_previous();
     static_assert(PASSES * BINS <= kMaxSortPasses * kRadixBins, "histograms fit the control block");
     __shared__ float s_scene[6];
@@ -191,8 +191,8 @@ __global__ __launch_bounds__(kThreads) void morton_kernel(const Node2* __restric
         K key = 0;
         if (valid) {
             const float4* p = reinterpret_cast<const float4*>(nodes + i);
-            float4 lo = __ldcs(p);
-            float2 hi = __ldcs(reinterpret_cast<const float2*>(p + 1));
+            float4 lo = ld_stream(p);
+            float2 hi = ld_stream(reinterpret_cast<const float2*>(p + 1));
             Box b;
             b.mn = make_float3(lo.x, lo.y, lo.z);
             b.mx = make_float3(lo.w, hi.x, hi.y);

@@ -746,7 +746,7 @@ constexpr uint32_t kNoChild = (1u << 21) - 1u;
 
 template <typename Seg>
 __global__ __launch_bounds__(kThreads) void bvh8_lists_kernel(Seg seg, uint32_t records,
-                                                              const ChildPair* __restrict__ kids, uint64_t* lists) {
+                                                              const ChildPair* kids, uint64_t* lists) {
     after_previous();
     extern __shared__ uint32_t s_slots[];
     const SlotTable<true> tab{s_slots};
@@ -799,12 +799,12 @@ __global__ __launch_bounds__(kThreads) void bvh8_lists_kernel(Seg seg, uint32_t 
 }
 
 template <typename Seg, bool AUCTION, bool LISTS>
-__global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __restrict__ b2, Seg seg, Node8* out,
+__global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* b2, Seg seg, Node8* out,
                                                               uint32_t cap, uint32_t slots, uint32_t* prim_idx,
                                                               uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
                                                               uint32_t* mesh_leaves, uint32_t* err,
-                                                              const ChildPair* __restrict__ kids,
-                                                              const uint64_t* __restrict__ lists) {
+                                                              const ChildPair* kids,
+                                                              const uint64_t* lists) {
     after_previous();
     __shared__ __align__(8) uint8_t s_rows[kGroupsPerCta][64];  // meta and quantised bytes of a group's node
     __shared__ __align__(16) float s_costs[AUCTION ? kGroupsPerCta : 1][8][8];  // by child and slot
@@ -888,7 +888,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* __res
             } else {
                 const uint32_t record = me.start + (b2i - me.count);
                 if constexpr (LISTS) {
-                    list = __ldg(lists + 3ull * record + sub / 3);
+                    list = lists[3ull * record + sub / 3];
                     nb = load_box(mb2, b2i);
                     internal = true;
                 } else {
