@@ -21,10 +21,10 @@ constexpr int kMaxSortPasses = 10;
 // next slot to claim; one 64-bit word of work slots allocated (low half)
 // and leaves (high half), bumped with one atomic, where one mesh's BVH8
 // nodes are its slots (every internal node is one work item, root
-// included); work items allocated but not finished.  Each counter has its
+// included); work items finished.  Each counter has its
 // own 128-byte line.
 constexpr int kBvh8Claim = 0, kBvh8Alloc = 32, kBvh8Nodes = kBvh8Alloc, kBvh8Leaves = kBvh8Alloc + 1,
-              kBvh8Pending = 64;
+              kBvh8Finished = 64;
 constexpr int kBvh8CtrWords = 160;
 
 // The BVH8 work queue of an n-primitive build before the collapse: slot 0
@@ -37,7 +37,7 @@ __device__ __forceinline__ void bvh8_queue_counters(uint32_t* ctr) {
     ctr[kBvh8Claim] = 0;
     ctr[kBvh8Alloc] = 1;  // = kBvh8Nodes: the root
     ctr[kBvh8Leaves] = 0;
-    ctr[kBvh8Pending] = 1;
+    ctr[kBvh8Finished] = 0;
 }
 constexpr int kRadixBits = 8;
 constexpr int kRadixBins = 1 << kRadixBits;

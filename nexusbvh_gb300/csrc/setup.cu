@@ -349,7 +349,7 @@ __global__ void batch_begin_kernel(BatchBegin b, MeshBatch batch) {
         c[kBvh8Claim] = 0;
         c[kBvh8Alloc] = meshes;  // a batch counts nodes and leaves per mesh
         c[kBvh8Leaves] = 0;
-        c[kBvh8Pending] = meshes;
+        c[kBvh8Finished] = 0;
     }
 }
 

@@ -282,29 +282,38 @@ __global__ void bvh8_init_kernel(uint64_t* pairs, uint32_t n, uint32_t* ctr) {
     if (i0 == 0) bvh8_queue_counters(ctr);
 }
 
-// A warp's account with the count of allocated-but-unfinished items: what it
-// allocates is added before the items are handed out, what it has finished
-// beyond that is kept as a credit for the items that it allocates next, and
-// subtracted only when it runs out of work.  The count is never too low, so
-// it reaches zero when no item is in flight and no warp holds a credit.
-// Added and subtracted after every pass of a warp instead, it was a third
-// atomic per pass on a line that every idle warp polls: 12.58M clustered
-// triangles 530 -> 512 us, 6.0M 340 -> 313, 4.19M sphere 245 -> 237.
-struct PendingCredit {
-    uint32_t* count;
-    uint32_t held = 0;
-    __device__ __forceinline__ void add(uint32_t allocated, uint32_t finished) {
-        held += finished;
-        if (allocated > held) {
-            if (lane_id() == 0) atomicAdd(count, allocated - held);
-            held = 0;
-        } else {
-            held -= allocated;
-        }
-    }
+// When the collapse is over: as many items have been finished as allocated.
+// A warp counts what it finishes and adds it to the queue's count when it has
+// nothing ready.  The two counts are never found equal early: an item's
+// children are allocated by an atomic whose result the warp waits for (their
+// slots follow from it), so that atomic has been performed before the item is
+// counted; a warp that looks waits for the finished count before it reads the
+// allocated one.  Fences in both places say the same in the memory model's
+// words; they take 2 us of a small build's 35 to 50 (they wait for the nodes
+// just written).  Counting allocated-but-unfinished items instead, in one
+// word, either lets a child be finished before the word knows of it, or has
+// every pass wait for a second atomic, on a line that idle warps poll
+// (65,536 triangles 39 us instead of 37, 4.19M sphere 242 instead of 236).
+constexpr uint32_t kEndCheck = 2;  // idle passes per look: 256,000 triangles 65.5 / 61.4 / 59.4 us at 1 / 2 / 4,
+                                   // 16,411 boxes 34.8 / 34.8 / 36.8, 12.58M 517 / 512 / 516
+struct FinishedItems {
+    uint32_t* ctr;
+    uint32_t held = 0, seen = 0;
+    __device__ __forceinline__ void add(uint32_t finished) { held += finished; }
     __device__ __forceinline__ void settle() {
-        if (held && lane_id() == 0) atomicAdd(count, 0u - held);
+        if (held && lane_id() == 0) atomicAdd(ctr + kBvh8Finished, held);
         held = 0;
+    }
+    // Whether every item is finished.  The allocated count, which every pass
+    // bumps, is only read again once as many items have been finished as had
+    // been allocated at its last reading (reading it at every look: 12.58M
+    // 512 -> 527 us).  Its address depends on the finished count, which is
+    // below 2^31.
+    __device__ __forceinline__ bool all() {
+        const uint32_t finished = ld_relaxed_u32(ctr + kBvh8Finished);
+        if (finished < seen) return false;
+        seen = ld_relaxed_u32(ctr + kBvh8Alloc + (finished >> 31));
+        return finished == seen;
     }
 };
 
@@ -344,7 +353,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
                 write_node8(out, load_box(b2, 0), LeafZero{b2}, 0, 0, 0xFFFFFFF0u, 0u, 1u);
                 prim_idx[0] = 0;
                 ctr[kBvh8Leaves] = 1;
-                ctr[kBvh8Pending] = 0;
+                ctr[kBvh8Finished] = 1;
             }
             return;
         }
@@ -352,7 +361,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
     uint32_t slot = kInvalid;
     bool retired = false;
     uint32_t idle = 0;
-    PendingCredit credit{ctr + kBvh8Pending};
+    FinishedItems items{ctr};
     for (;;) {
         // lanes without a slot claim the next ones, in increasing order; a
         // slot past the queue's end is never allocated and retires the lane
@@ -372,7 +381,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
             }
         }
         if (__all_sync(kFullMask, retired)) {
-            credit.settle();
+            items.settle();
             return;
         }
         uint64_t pr = 0;
@@ -382,10 +391,9 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
             ready = (uint32_t)(pr >> 32) != kInvalid;
         }
         if (!__any_sync(kFullMask, ready)) {
-            // nothing ready: finished when no allocated item is outstanding
-            credit.settle();
-            if (ld_relaxed_u32(ctr + kBvh8Pending) == 0) return;
-            if (++idle > kQueueSpinLimit) {
+            items.settle();
+            if (++idle % kEndCheck == 0 && items.all()) return;
+            if (idle > kQueueSpinLimit) {
                 if (lane == 0) set_error(err, NXB_DEVERR_BVH8_QUEUE_TIMEOUT);
                 return;
             }
@@ -545,7 +553,6 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
         }
         const uint32_t done = __popc(__ballot_sync(kFullMask, ready));
         // one 64-bit atomic: work slots (one mesh: = BVH8 nodes) low, leaves high
-        credit.add(__shfl_sync(kFullMask, incl >> 20, 31), done);
         uint64_t bases = 0;
         if (lane == 31) {
             const uint64_t tl = (incl >> 10) & 0x3FFu, tw = incl >> 20;
@@ -554,6 +561,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_kernel(const Node2* __restrict_
                                   (unsigned long long)((tl << 32) | tw));
         }
         bases = __shfl_sync(kFullMask, bases, 31);
+        items.add(done);
         const uint32_t wb = (uint32_t)bases, nb = wb, lb = (uint32_t)(bases >> 32);
         bool wrote = false;
         __syncwarp();
@@ -816,7 +824,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* b2, S
                 write_node8(out, load_box(b2, 0), LeafZero{b2}, 0, 0, 0xFFFFFFF0u, 0u, 1u);
                 prim_idx[0] = 0;
                 ctr[kBvh8Leaves] = 1;
-                ctr[kBvh8Pending] = 0;
+                ctr[kBvh8Finished] = 1;
             }
             return;
         }
@@ -824,7 +832,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* b2, S
     uint32_t slot = kInvalid;
     bool retired = false;
     uint32_t idle = 0;
-    PendingCredit credit{ctr + kBvh8Pending};
+    FinishedItems items{ctr};
     for (;;) {
         // groups without a slot claim the next ones (see bvh8_kernel)
         const bool want = !retired && slot == kInvalid;
@@ -842,7 +850,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* b2, S
             }
         }
         if (__all_sync(kFullMask, retired)) {
-            credit.settle();
+            items.settle();
             return;
         }
         uint64_t pr = ~0ull;
@@ -850,9 +858,9 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* b2, S
         pr = __shfl_sync(kFullMask, pr, 0, 8);  // one lane's view for the whole group
         const bool ready = (uint32_t)(pr >> 32) != kInvalid;
         if (!__any_sync(kFullMask, ready)) {
-            credit.settle();
-            if (ld_relaxed_u32(ctr + kBvh8Pending) == 0) return;
-            if (++idle > kQueueSpinLimit) {
+            items.settle();
+            if (++idle % kEndCheck == 0 && items.all()) return;
+            if (idle > kQueueSpinLimit) {
                 if (lane == 0) set_error(err, NXB_DEVERR_BVH8_QUEUE_TIMEOUT);
                 return;
             }
@@ -1003,7 +1011,6 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* b2, S
         const uint32_t done = __popc(__ballot_sync(kFullMask, ready && sub == 0));
         const uint32_t new_items = total & 0xFFFFu;
         const uint64_t tl = Seg::kBatch ? 0u : total >> 16;
-        credit.add(new_items, done);
         uint64_t bases = 0;
         if (lane == 0 && (tl | new_items))
             bases = atomicAdd(reinterpret_cast<unsigned long long*>(ctr + kBvh8Alloc),
@@ -1014,6 +1021,7 @@ __global__ __launch_bounds__(kThreads) void bvh8_group_kernel(const Node2* b2, S
             prim_base = lc ? atomicAdd(mesh_leaves + me.m, lc) : 0u;
         }
         bases = __shfl_sync(kFullMask, bases, 0);
+        items.add(done);
         const uint32_t work_base = (uint32_t)bases + (excl & 0xFFFFu);
         if constexpr (Seg::kBatch) {
             child_base = __shfl_sync(kFullMask, child_base, 0, 8);
@@ -1085,7 +1093,7 @@ cudaError_t launch_group(const Node2* bvh2, Seg seg, uint32_t items, Node8* out,
         }
     }
     int per_sm = resident_ctas<bvh8_group_kernel<Seg, AUCTION, LISTS>>(kThreads, 0);
-    // Groups that wait poll the pending counter, and too many of them saturate
+    // Groups that wait poll the finished count, and too many of them saturate
     // its L2 line.  With lists, a group per 16 primitives and, above 4,096
     // groups, per 32: 1,021 triangles 27 us (33 at 32), 65,536 39 (47 at 8),
     // 128,000 49 (53 at 16), 256,000 68 (70); at 8 CTAs per SM instead of 4,
@@ -1167,8 +1175,7 @@ cudaError_t run_bvh8_stall_probe(uint32_t* err_out) {
     e = cudaMemset(buf, 0, bytes);
     if (!e) e = cudaMemset(pairs, 0xFF, 8 * n);
     uint32_t c[kBvh8CtrWords] = {};
-    c[kBvh8Alloc] = 1;    // slot 0 is allocated ...
-    c[kBvh8Pending] = 1;  // ... but its pair is never written
+    c[kBvh8Alloc] = 1;  // slot 0 is allocated, but its pair is never written
     if (!e) e = cudaMemcpy(ctr, c, sizeof(c), cudaMemcpyHostToDevice);
     if (!e) {
         bvh8_kernel<SingleMesh, false, false><<<1, kThreads, (kSlotSmem<false>)>>>(b2, SingleMesh{n}, out, 2, n, prim, pairs,
