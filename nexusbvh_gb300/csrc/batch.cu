@@ -8,10 +8,9 @@
 //   * scene bounds per mesh (warp-reduced into 6 ordered words per mesh);
 //   * 30-bit Morton codes from each mesh's own box, sorted within every mesh
 //     by code >> 2 (stable), which is exactly the plain sort: in one cluster
-//     per mesh if no mesh is larger than that takes, else in segmented
-//     passes, else (many small meshes beside a large one) as one 64-bit key
-//     mesh << 32 | code over bits [2, 32 + mesh bits), which keeps the
-//     meshes in order;
+//     per mesh where the clusters are few enough, else in segmented passes,
+//     else (many small meshes) as one 64-bit key mesh << 32 | code over bits
+//     [2, 32 + mesh bits), which keeps the meshes in order;
 //   * H-PLOC and the BVH8 collapse with mesh-local indices (MeshBatch in
 //     common.cuh), so every mesh's BVH2 is the plain build's array;
 //   * nxb_batch_* capture the whole sequence once in a CUDA graph and
@@ -162,10 +161,11 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
     one.slot[1] = a.slots;
     const MeshGroups& g = (groups && fork && groups->count > 1) ? *groups : one;
     const MeshBatch mb{a.off, a.off8, a.meshes};
-    const bool local = local_sort_takes(a.max_mesh);
     SegmentPlan segments{};
-    const bool seg = !local && segment_sort_takes(a.total, a.meshes, a.lookback,
-                                                  a.lookback_words_per_pass * kMaxSortPasses, &segments);
+    const bool fits = segment_sort_takes(a.total, a.meshes, a.lookback, a.lookback_words_per_pass * kMaxSortPasses,
+                                         &segments);
+    const bool local = local_sort_takes_batch(a.max_mesh, a.meshes, a.total, fits);
+    const bool seg = fits && !local;
     const SortPlan plan = local || seg ? SortPlan{} : make_sort_plan(2, 32 + a.mesh_bits, t.digit_bits);
     const BatchBegin begin{reinterpret_cast<uint4*>(a.zero_begin), a.zero_bytes / 16, a.tile_rng, t.block, a.total,
                            a.pairs, a.slots, a.ctr8, a.mesh_nodes, a.mesh_leaves, g};

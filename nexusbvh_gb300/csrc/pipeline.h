@@ -229,11 +229,12 @@ cudaError_t launch_sort63_hybrid(const uint64_t* keys_in, const uint32_t* vals_i
                                  uint32_t* lookback, uint32_t* tile_ctr, uint32_t* overflow, uint32_t* fb_hist,
                                  uint32_t* fb_ticket, uint32_t* fb_done, uint32_t* err, cudaStream_t s);
 // The pipeline's small sorts in one launch (a thread-block cluster per mesh):
-// whether n keys (of one mesh, or of a batch's largest mesh) are sorted that
-// way; Morton keys in place with the permutation in vals; a batch's keys
-// (mesh << 32 | code) with the mesh-local permutation.  Neither needs
-// histograms, look-back words or counters.
+// whether n keys of one mesh, or a batch (segments: instead of segmented
+// passes), are sorted that way; Morton keys in place with the permutation in
+// vals; a batch's keys (mesh << 32 | code) with the mesh-local permutation.
+// Neither needs histograms, look-back words or counters.
 bool local_sort_takes(uint32_t n);
+bool local_sort_takes_batch(uint32_t max_mesh, uint32_t meshes, uint32_t total, bool segments);
 cudaError_t launch_local_sort(uint32_t key_bytes, void* keys, uint32_t* vals, uint32_t n, cudaStream_t s);
 cudaError_t launch_local_sort_batch(uint64_t* keys, uint32_t* vals, const MeshBatch& batch, uint32_t max_mesh,
                                     cudaStream_t s);

@@ -1338,6 +1338,28 @@ bool local_sort_takes(uint32_t n) {
     return e == cudaSuccess;
 }
 
+// A batch gives every mesh the cluster that its largest mesh needs, so the time
+// goes with the CTAs, full or not, and few of the large clusters run at once
+// (a CTA of 8 keys per thread has an SM to itself).  The other passes cost
+// their launches and the keys.  The line, in CTAs of 8 keys per thread, is
+// where whole builds cross (us, clusters / other passes; m meshes, all of one
+// size, or one of them so large and the others of 16 primitives):
+//   1,024 primitives: 8,000 full 1,589 / 1,921; 2,000 sparse 140 / 149, 4,000 197 / 172
+//   4,096: 1,200 full 1,000 / 1,016, 1,800 1,443 / 1,446; 300 sparse 125 / 147, 600 149 / 148, 900 174 / 150
+//   8,192: 300 full 688 / 689, 400 831 / 812; 150 sparse 135 / 147, 200 149 / 147
+//   16,384: 100 full 568 / 570, 140 701 / 691; 70 sparse 138 / 149, 100 154 / 151
+//   32,768: 19 full 347 / 349, 40 568 / 558; 30 sparse 153 / 162, 40 161 / 160
+//   65,536: 8 full 322 / 321, 16 516 / 493; 10 sparse 160 / 172, 16 175 / 172
+// Taken for every batch it cost 20,000 meshes of 30 beside one of 60,000
+// 50,157 us (459 by the other passes) and 900 of 16 to 60,000 3,792 (1,430).
+bool local_sort_takes_batch(uint32_t max_mesh, uint32_t meshes, uint32_t total, bool segments) {
+    if (!local_sort_takes(max_mesh)) return false;
+    const double ctas = (max_mesh + kLocalThreads * kLocalMaxKpt - 1) / (kLocalThreads * kLocalMaxKpt);
+    const double cta = max_mesh <= kLocalThreads * 2 ? 0.25 : max_mesh <= kLocalThreads * 4 ? 0.375 : 1.0;
+    const double full = (double)total / (kLocalThreads * kLocalMaxKpt);
+    return meshes * cta * ctas * (3.0 + ctas) / 4.0 <= 4.0 * device_info().sms + (segments ? 0.57 : 2.1) * full;
+}
+
 cudaError_t launch_local_sort(uint32_t key_bytes, void* keys, uint32_t* vals, uint32_t n, cudaStream_t s) {
     return by_keys_per_thread(n, kLocalMaxCtas, [&](auto kpt) {
         if (key_bytes == 4)
