@@ -25,8 +25,9 @@
 //     3.81 ms; the BVH8 kernel's time hardly depends on its occupancy (3 / 6
 //     CTAs per SM: 0.898 / 0.833 ms), it follows the random node traffic;
 //   * small greedy collapses, which are chains of levels, read every node's
-//     children and slots from lists made beforehand, and auctions take eight
-//     lanes per item (takes_lists, takes_groups).
+//     children and slots from lists made beforehand, and auctions up to
+//     2,000,000 primitives take eight lanes per item (takes_lists,
+//     takes_groups).
 // The decisions are the reference's:
 //   * expansion always re-opens the highest-indexed inner child, the child
 //     with the smaller area going to the re-opened position (:284-330);
@@ -1122,12 +1123,18 @@ cudaError_t launch_group(const Node2* bvh2, Seg seg, uint32_t items, Node8* out,
 // 129 / 100 / 72, 512,000 143 / 131 / 98, 1.0M 154 / 184 / 160, 1.0M
 // clustered 180 / - / 166, 4.19M sphere 237 / 473 / -.  Groups of a batch
 // that overlaps its stages have no room for lists.  An auction is a long
-// sequential search per item, eight times shorter in a group: 1.05M sphere
-// 1042 / 512 us; the lists would take it for every node.
+// sequential search per item, eight times shorter in a group, so it takes the
+// groups further, up to where the items in flight count (group / one lane):
+// 100,000 soup triangles 256 / 457 us, 1.0M 510 / 674, 2.0M 756 / 748, 3.0M
+// 1,026 / 817, 12.58M 3,565 / 1,655; 2.0M clustered 746 / 776.  The lists would
+// take it for every node.
 constexpr uint32_t kListMaxPrims = 800000;  // at most 2^20: a list holds 21-bit indices
 constexpr uint32_t kGroupMaxPrims = 600000;
+constexpr uint32_t kAuctionGroupMaxPrims = 2000000;
 inline bool takes_lists(uint32_t prims, bool auction) { return !auction && prims <= kListMaxPrims; }
-inline bool takes_groups(uint32_t prims, bool auction) { return auction || prims <= kGroupMaxPrims; }
+inline bool takes_groups(uint32_t prims, bool auction) {
+    return prims <= (auction ? kAuctionGroupMaxPrims : kGroupMaxPrims);
+}
 
 template <typename Seg, bool AUCTION, bool KIDS>
 cudaError_t configure_smem() {
@@ -1200,9 +1207,12 @@ cudaError_t launch_bvh8(const Node2* bvh2, uint32_t n, Node8* out, uint32_t cap,
     if (child_pairs && lists && takes_lists(n, auction))
         return launch_group<SingleMesh, false, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr,
                                                      nullptr, err, s, child_pairs, lists);
-    if (child_pairs && auction)
+    if (child_pairs && auction && takes_groups(n, true))
         return launch_group<SingleMesh, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr, err,
                                               s, child_pairs);
+    if (child_pairs && auction)
+        return launch_wide<SingleMesh, true, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr, nullptr,
+                                                   err, s, child_pairs);
     if (child_pairs)
         return launch_wide<SingleMesh, false, true>(bvh2, seg, n, out, cap, n, prim_idx, pairs, ctr, nullptr,
                                                     nullptr, err, s, child_pairs);
@@ -1226,6 +1236,9 @@ cudaError_t launch_bvh8_batch(const Node2* bvh2, const MeshBatch& batch, uint32_
         return launch_group<MeshBatch, false>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
                                               mesh_leaves, err, s, child_pairs);
     }
+    if (child_pairs && auction)
+        return launch_wide<MeshBatch, true, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
+                                                  mesh_leaves, err, s, child_pairs);
     if (child_pairs)
         return launch_wide<MeshBatch, false, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr,
                                                    mesh_nodes, mesh_leaves, err, s, child_pairs);
