@@ -138,6 +138,15 @@ cudaError_t load_setup_kernels();
 cudaError_t load_sort_kernels();
 cudaError_t load_collapse_kernels();
 
+// Launches a kernel and, like the cudaGetLastError() after a <<<>>> launch,
+// leaves no error behind for the next call to find.
+template <typename... P, typename... A>
+cudaError_t launch_ex(const cudaLaunchConfig_t& c, void (*kernel)(P...), A... args) {
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+    if (e) cudaGetLastError();
+    return e;
+}
+
 // Launches a kernel that begins with after_previous(); if the build of n
 // primitives is small, its CTAs are set up while the kernel before it in the
 // stream still runs, otherwise as usual.  Whole builds, usual / early:
@@ -159,9 +168,7 @@ cudaError_t launch_after(uint32_t n, void (*kernel)(P...), dim3 grid, dim3 block
     c.stream = s;
     c.attrs = &attr;
     c.numAttrs = n <= kAfterMaxPrims ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
-    if (e) cudaGetLastError();
-    return e;
+    return launch_ex(c, kernel, static_cast<P>(args)...);
 }
 
 struct DeviceInfo {

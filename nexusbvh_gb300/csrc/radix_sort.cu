@@ -1090,7 +1090,7 @@ cudaError_t launch_local(K* keys, uint32_t* vals, uint32_t n, uint32_t shift, in
     const uint32_t ctas = (n + T - 1) / T;
     cudaLaunchAttribute attr[2]{};
     cudaLaunchConfig_t c = local_config(ctas, ctas, smem, s, attr, true);
-    return cudaLaunchKernelEx(&c, sort_cluster_kernel<K, RB, KPT>, keys, vals, n, shift, passes);
+    return launch_ex(c, sort_cluster_kernel<K, RB, KPT>, keys, vals, n, shift, passes);
 }
 template <int RB, int KPT>
 cudaError_t launch_local_batch(uint64_t* keys, uint32_t* vals, const MeshBatch& batch, uint32_t max_mesh, uint32_t shift,
@@ -1102,7 +1102,7 @@ cudaError_t launch_local_batch(uint64_t* keys, uint32_t* vals, const MeshBatch& 
     const uint32_t ctas = (max_mesh + T - 1) / T;
     cudaLaunchAttribute attr[2]{};
     cudaLaunchConfig_t c = local_config(ctas * batch.meshes, ctas, smem, s, attr, false);
-    return cudaLaunchKernelEx(&c, sort_cluster_batch_kernel<RB, KPT>, keys, vals, batch, ctas, shift, passes);
+    return launch_ex(c, sort_cluster_batch_kernel<RB, KPT>, keys, vals, batch, ctas, shift, passes);
 }
 // Keys per thread: as few as the largest cluster (one mesh, where a pass is a
 // chain of steps) or one CTA (a batch, whose meshes share the SMs) can hold.

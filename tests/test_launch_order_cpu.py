@@ -64,3 +64,12 @@ def test_helpers(name):
             assert "__restrict__" not in m.group(0), f.name
             assert "__ldg" not in block(text, m.end() - 1), f.name
     assert found
+
+
+def test_launches_with_attributes_leave_no_error_behind():
+    """cudaLaunchKernelEx returns its error and also keeps it for the next
+    cudaGetLastError, which would fail the launch after it."""
+    for f in sorted(CSRC.iterdir()):
+        text = f.read_text()
+        for m in re.finditer(r"cudaLaunchKernelEx\(", text):
+            assert f.name == "pipeline.h" and "cudaGetLastError();" in text[m.start():m.start() + 120], f.name
