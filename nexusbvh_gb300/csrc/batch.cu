@@ -40,8 +40,8 @@ uint32_t mesh_bits_of(uint32_t meshes) { return meshes > 1 ? 32u - (uint32_t)__b
 
 // Segment offsets of an arena, in allocation order.
 struct Segments {
-    size_t off, off8, ctrl, scene, zero_end, parent, look, ctr8, mnodes, mleaves, trng, ka, kb, va, vb, pairs, kids,
-        bvh2, bvh8, prim, res, total;
+    size_t off, off8, ctrl, scene, zero_end, parent, look, ctr8, mnodes, mleaves, trng, ka, kb, va, vb, sort_end, pairs,
+        kids, bvh2, bvh8, prim, res, total;
 };
 
 Segments segments_of(const BatchArena& a) {
@@ -64,10 +64,13 @@ Segments segments_of(const BatchArena& a) {
     g.mnodes = seg(4 * M);
     g.mleaves = seg(4 * M);
     g.trng = seg(8 * ((n + 127) / 128));
+    // the sort's buffers, one after the other: the collapse's lists lie in all
+    // of them (BatchArena::lists)
     g.ka = seg(8 * n);
     g.kb = seg(8 * n);
     g.va = seg(4 * n);
     g.vb = seg(4 * n);
+    g.sort_end = at;
     g.pairs = seg(8ull * a.slots);
     g.kids = seg(sizeof(ChildPair) * n);
     g.bvh2 = seg(sizeof(Node2) * 2 * n);
@@ -126,6 +129,7 @@ void batch_bind(unsigned char* p, BatchArena* a) {
     a->keys_b = reinterpret_cast<uint64_t*>(p + g.kb);
     a->vals_a = reinterpret_cast<uint32_t*>(p + g.va);
     a->vals_b = reinterpret_cast<uint32_t*>(p + g.vb);
+    a->lists = g.sort_end - g.ka >= 24ull * a->total ? a->keys_a : nullptr;
     a->pairs = reinterpret_cast<uint64_t*>(p + g.pairs);
     a->kids = reinterpret_cast<ChildPair*>(p + g.kids);
     a->bvh2 = reinterpret_cast<Node2*>(p + g.bvh2);
@@ -202,10 +206,9 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
         const bool in_a = (plan.passes % 2) == 0;
         uint64_t* keys = in_a ? a.keys_a : a.keys_b;
         uint32_t* perm = in_a ? a.vals_a : a.vals_b;
-        // a whole batch's collapse has the sort's buffers (24 bytes per
-        // primitive) for its lists; that of a group has not, as the climb of
-        // the next group still reads them
-        uint64_t* lists = g.count == 1 ? a.keys_a : nullptr;
+        // a whole batch's collapse has the sort's buffers for its lists; that of
+        // a group has not, as the climb of the next group still reads them
+        uint64_t* lists = g.count == 1 ? a.lists : nullptr;
         // H-PLOC group by group on s; the collapse of group k follows it on
         // the side stream (ordered by an event, no wait inside any kernel),
         // overlapping H-PLOC of group k+1

@@ -402,6 +402,7 @@ struct BatchArena {
     uint64_t* keys_b = nullptr;
     uint32_t* vals_a = nullptr;
     uint32_t* vals_b = nullptr;
+    uint64_t* lists = nullptr;  // 24 bytes per primitive: keys and values, which the climb is the last to read
     uint64_t* pairs = nullptr;
     ChildPair* kids = nullptr;  // child-pair records (one per primitive, 64-byte aligned)
     Node2* bvh2 = nullptr;
