@@ -416,7 +416,9 @@ typedef struct nxb_batch_arrays {      /* device views owned by the batch */
 } nxb_batch_arrays;
 
 typedef struct nxb_batch_tuning {
-    uint32_t sort_digit_bits;   /* 4..8: bits per radix sort pass (at most 10 passes) */
+    uint32_t sort_digit_bits;   /* 4..8: bits per radix sort pass (at most 10 passes) of batches sorted as a
+                                   whole: many small meshes, fewer than 1,536 primitives on average.
+                                   Others are sorted mesh by mesh and do not use it */
     uint32_t search_radius;     /* H-PLOC radius in use */
     uint32_t hploc_ctas_per_sm; /* cap on the H-PLOC persistent grid (0 = occupancy) */
     uint32_t fusion_groups;     /* BVH2/BVH8 fusion point: 0 or 1 = collapse after H-PLOC has built
@@ -453,7 +455,8 @@ nxb_status nxb_batch_get_arrays(const nxb_batch* batch, nxb_batch_arrays* out_ar
 /* Times candidate settings on this batch and input (each: one warm-up build,
  * then the median of `repeats` builds) and keeps the fastest.  Without
  * NXB_TUNE_RADIUS only settings that leave the results unchanged are tried
- * (sort digit width, H-PLOC grid size, BVH2/BVH8 fusion point). */
+ * (sort digit width where the batch uses one, H-PLOC grid size, BVH2/BVH8
+ * fusion point). */
 nxb_status nxb_batch_autotune(nxb_batch* batch, const void* d_prims, uint32_t tune_flags, uint32_t repeats,
                               struct CUstream_st* stream, nxb_batch_tuning* out_choice);
 nxb_status nxb_batch_set_tuning(nxb_batch* batch, const nxb_batch_tuning* tuning);

@@ -156,6 +156,17 @@ void batch_groups(const uint32_t* h_off, const uint32_t* h_off8, uint32_t meshes
     }
 }
 
+BatchSort batch_sort(const BatchArena& a, uint32_t digit_bits) {
+    BatchSort s{};
+    const bool fits = segment_sort_takes(a.total, a.meshes, a.lookback, a.lookback_words_per_pass * kMaxSortPasses,
+                                         &s.segments);
+    s.form = local_sort_takes_batch(a.max_mesh, a.meshes, a.total, fits) ? BatchSort::kClusters
+             : fits                                                      ? BatchSort::kSegments
+                                                                         : BatchSort::kWhole;
+    if (s.form == BatchSort::kWhole) s.plan = make_sort_plan(2, 32 + a.mesh_bits, digit_bits);
+    return s;
+}
+
 nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type type, const BatchTuning& t,
                          uint32_t* h_err, cudaStream_t s, const MeshGroups* groups, const BatchFork* fork) {
     MeshGroups one{};
@@ -165,12 +176,8 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
     one.slot[1] = a.slots;
     const MeshGroups& g = (groups && fork && groups->count > 1) ? *groups : one;
     const MeshBatch mb{a.off, a.off8, a.meshes};
-    SegmentPlan segments{};
-    const bool fits = segment_sort_takes(a.total, a.meshes, a.lookback, a.lookback_words_per_pass * kMaxSortPasses,
-                                         &segments);
-    const bool local = local_sort_takes_batch(a.max_mesh, a.meshes, a.total, fits);
-    const bool seg = fits && !local;
-    const SortPlan plan = local || seg ? SortPlan{} : make_sort_plan(2, 32 + a.mesh_bits, t.digit_bits);
+    const BatchSort sort = batch_sort(a, t.digit_bits);
+    const SortPlan& plan = sort.plan;
     const BatchBegin begin{reinterpret_cast<uint4*>(a.zero_begin), a.zero_bytes / 16, a.tile_rng, t.block, a.total,
                            a.pairs, a.slots, a.ctr8, a.mesh_nodes, a.mesh_leaves, g};
     NXB_TRY(launch_batch_begin(begin, mb, s));
@@ -181,19 +188,19 @@ nxb_status batch_enqueue(const BatchArena& a, const void* prims, nxb_prim_type t
         f.zero_words = align_up(4 * a.lookback_words_per_pass * plan.passes) / 4;
         f.ones_ptr = a.parent;
         f.ones_words = a.ones_words;
-        if (seg) {
-            f.zero_ptr = segments.lookback;
-            f.zero_words = segments.lookback_words;
-            NXB_TRY(launch_segment_prepare(segments, mb, s));
-            NXB_TRY(launch_segment_morton(a.bvh2, mb, a.scene_ord, reinterpret_cast<uint32_t*>(a.keys_b), segments, f,
-                                          t.block, s));
-            NXB_TRY(launch_segment_sort(segments, mb, a.total, a.keys_a, a.keys_b, a.vals_a, a.vals_b,
+        if (sort.form == BatchSort::kSegments) {
+            f.zero_ptr = sort.segments.lookback;
+            f.zero_words = sort.segments.lookback_words;
+            NXB_TRY(launch_segment_prepare(sort.segments, mb, s));
+            NXB_TRY(launch_segment_morton(a.bvh2, mb, a.scene_ord, reinterpret_cast<uint32_t*>(a.keys_b), sort.segments,
+                                          f, t.block, s));
+            NXB_TRY(launch_segment_sort(sort.segments, mb, a.total, a.keys_a, a.keys_b, a.vals_a, a.vals_b,
                                         a.ctrl->tile_ctr, &a.ctrl->error_word, s));
         } else {
             NXB_TRY(launch_batch_morton(a.bvh2, mb, a.total, a.scene_ord, a.keys_a, a.vals_a, plan,
                                         &a.ctrl->hist[0][0], f, t.block, a.tile_rng, s));
         }
-        if (local) NXB_TRY(launch_local_sort_batch(a.keys_a, a.vals_a, mb, a.max_mesh, s));
+        if (sort.form == BatchSort::kClusters) NXB_TRY(launch_local_sort_batch(a.keys_a, a.vals_a, mb, a.max_mesh, s));
         for (int p = 0; p < plan.passes; ++p) {
             const bool even = (p % 2) == 0;
             NXB_TRY(launch_sort_pass(8, even ? a.keys_a : a.keys_b, even ? a.keys_b : a.keys_a,
@@ -462,8 +469,10 @@ nxb_status nxb_batch_autotune(nxb_batch* b, const void* prims, uint32_t flags, u
     // is (and the radius, when asked for)
     const nxb_batch_tuning start = b->tuning;
     std::vector<nxb_batch_tuning> cand;
+    std::vector<uint32_t> digits = {8, 7, 6, 5, 4};
+    if (batch_sort(b->arena, start.sort_digit_bits).form != BatchSort::kWhole) digits = {start.sort_digit_bits};
     for (uint32_t r : radii)
-        for (uint32_t d : {8u, 7u, 6u, 5u, 4u}) {
+        for (uint32_t d : digits) {
             if (!batch_digit_ok(b->arena.mesh_bits, d)) continue;
             for (uint32_t c : {0u, 4u})
                 for (uint32_t g : {1u, 2u, 4u})

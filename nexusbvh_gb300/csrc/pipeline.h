@@ -410,6 +410,14 @@ struct BatchArena {
     uint32_t* prim_idx = nullptr;
     nxb_batch_mesh* results = nullptr;
 };
+// How a batch is sorted: a cluster per mesh, passes within every mesh, or
+// passes over mesh << 32 | code (the only ones that have a digit width).
+struct BatchSort {
+    enum Form { kClusters, kSegments, kWhole } form;
+    SegmentPlan segments;  // kSegments
+    SortPlan plan;         // kWhole, else no passes
+};
+BatchSort batch_sort(const BatchArena& a, uint32_t digit_bits);
 struct BatchTuning {
     uint32_t digit_bits = 8, radius = 8, hploc_ctas_per_sm = 0;
     bool auction = false;
