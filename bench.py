@@ -193,6 +193,8 @@ def run_ours(args, world, rank, local):
     b = nxb.Builder()
     sz = b.sizes(n, cfg)
     ws = b.workspace(sz.workspace_bytes)
+    launches = nxb.CLaunchInfo()
+    nxb.check(lib.nxb_query_build_launches(n, ctypes.byref(c), 1, ctypes.byref(launches)), "nxb_query_build_launches")
     b2 = torch.empty((sz.bvh2_node_count, 32), dtype=torch.uint8, device="cuda")
     b8 = torch.empty((sz.bvh8_node_capacity, 80), dtype=torch.uint8, device="cuda")
     prim_idx = torch.empty(n, dtype=torch.int32, device="cuda")
@@ -387,11 +389,7 @@ def run_ours(args, world, rank, local):
                 "d2h_bytes_per_step": ctypes.sizeof(nxb.CResult),
                 "call": "nxb_build_bvh8 (C ABI, allocates outputs) after a pinned host->device copy",
                 "copy_ms": round(copy_ms, 3), "h2d_gbs": round(36 * n / (copy_ms * 1e-3) / 1e9, 1)},
-        # per build: bounds, Morton, the sort (up to 65,536 primitives one
-        # launch; 30-bit: 4 passes; 63-bit: 4 passes, the bucket sort and the
-        # fallback launch), H-PLOC (which also initialises the BVH8 work
-        # queue), the lists of small greedy collapses, BVH8, finalize
-        "gpu_launches": (5 + (1 if n <= 65_536 else 4 if key_bits == 30 else 6) + (n <= 800_000)) * args.steps,
+        "gpu_launches": launches.kernels * args.steps,
         "clocks": clk,
     }
     if not args.no_cpu_baseline:
@@ -538,7 +536,9 @@ def measure_batch(args, world, rank, local, steps: int, warmup: int, autotune: b
         torch.cuda.synchronize()
         t_loop_async = start.elapsed_time(stop) / 1e3
         del ws, b2, b8, pidx, rbuf
-    passes, kb, sort_launches = batch_sort(counts, int(tuning.sort_digit_bits))
+    launches = nxb.CLaunchInfo()
+    nxb.check(nxb.load().nxb_query_batch_launches(batch._handle, ctypes.byref(launches)), "nxb_query_batch_launches")
+    passes, kb = launches.sort_passes, launches.sort_key_bytes
     # 32-bit codes become 64-bit keys in the last pass
     per_tri = (algorithmic_bytes("scene_bounds", 8, passes, 0) + algorithmic_bytes("morton", kb, passes, 0)
                + 4.0 + algorithmic_bytes("radix_sort", kb, passes, 0) + 8 - kb + algorithmic_bytes("hploc", 8, passes, 0)
@@ -546,7 +546,7 @@ def measure_batch(args, world, rank, local, steps: int, warmup: int, autotune: b
     ms = elapsed / steps
     out_d = {
         "value": value, "ms": ms, "n": n, "n_all": n_all, "meshes": meshes, "meshes_all": meshes_all,
-        "tuning": tuning, "passes": passes, "sort_launches": sort_launches, "fusion": fusion, "t_tune": t_tune, "n8": n8,
+        "tuning": tuning, "passes": passes, "launches": launches.kernels, "fusion": fusion, "t_tune": t_tune, "n8": n8,
         "gbs": per_tri * n / (ms * 1e-3) / 1e9, "e2e": e2e_value, "t_loop": t_loop, "t_loop_async": t_loop_async,
         "clocks": clocks.summary(),
     }
@@ -591,18 +591,6 @@ def batch_summary(b: dict) -> dict:
     }
 
 
-def batch_sort(counts, digit_bits: int) -> tuple[int, int, int]:
-    """Passes, key bytes and launches of a batch's sort: a cluster per mesh,
-    7-bit passes over 32-bit codes within the meshes (after one launch that
-    lists the tiles), or passes over 64-bit keys mesh << 32 | code."""
-    if max(counts) <= 65_536:
-        return 4, 4, 1
-    if len(counts) * 1536 <= sum(counts):
-        return 4, 4, 5
-    passes = -(-(30 + max(1, (len(counts) - 1).bit_length())) // digit_bits)
-    return passes, 8, passes
-
-
 def run_batch(args, world, rank, local):
     """Batched form: the batch1024 line."""
     b = measure_batch(args, world, rank, local, args.steps, args.warmup, autotune=not args.no_autotune,
@@ -638,9 +626,7 @@ def run_batch(args, world, rank, local):
         "e2e": {"value": round(b["e2e"], 2), "unit": "Mtris/s", "h2d_bytes_per_step": 36 * n,
                 "d2h_bytes_per_step": 52 * meshes + 4,
                 "call": "nxb_batch_build (graph replay + wait + per-mesh results) after a pinned host->device copy"},
-        # per build: begin, bounds, Morton, the sort, H-PLOC, the lists of
-        # small collapses, BVH8, finalize (one mesh group)
-        "gpu_launches": (6 + b["sort_launches"] + (b["n"] <= 800_000)) * args.steps,
+        "gpu_launches": b["launches"] * args.steps,
         "clocks": b["clocks"],
     }
     if "cpu_baseline" in b:

@@ -533,6 +533,17 @@ nxb_status nxb_server_poll(nxb_server* server, uint64_t ticket, nxb_server_resul
 nxb_status nxb_server_release(nxb_server* server, uint64_t ticket);
 nxb_status nxb_server_get_stats(nxb_server* server, nxb_server_stats* out);
 
+/* Diagnostics: what one build launches on the current device (for reports). */
+typedef struct nxb_launch_info {
+    uint32_t kernels;        /* in all */
+    uint32_t sort_passes;    /* over the keys */
+    uint32_t sort_key_bytes; /* of a key in those passes */
+} nxb_launch_info;
+/* Of nxb_build_async (wide: with a BVH8) and of a batch with its present tuning. */
+nxb_status nxb_query_build_launches(uint32_t prim_count, const nxb_build_config* config, int wide,
+                                    nxb_launch_info* out_info);
+nxb_status nxb_query_batch_launches(const nxb_batch* batch, nxb_launch_info* out_info);
+
 /* Library version and the compile flags that define its numerics. */
 const char* nxb_version(void);
 

@@ -73,6 +73,10 @@ class CConfig(ctypes.Structure):
                 ("flags", ctypes.c_uint32), ("reserved", ctypes.c_uint32)]
 
 
+class CLaunchInfo(ctypes.Structure):
+    _fields_ = [("kernels", ctypes.c_uint32), ("sort_passes", ctypes.c_uint32), ("sort_key_bytes", ctypes.c_uint32)]
+
+
 class CSizes(ctypes.Structure):
     _fields_ = [("workspace_bytes", ctypes.c_size_t), ("bvh2_node_count", ctypes.c_size_t),
                 ("bvh8_node_capacity", ctypes.c_size_t)]
@@ -147,6 +151,8 @@ _SIG = {
     "nxb_free_device_bvh2": (ctypes.c_int, [ctypes.POINTER(CBVH2)]),
     "nxb_free_device_bvh8": (ctypes.c_int, [ctypes.POINTER(CBVH8)]),
     "nxb_query_build_sizes": (ctypes.c_int, [_U32, _P, ctypes.POINTER(CSizes)]),
+    "nxb_query_build_launches": (ctypes.c_int, [_U32, _P, ctypes.c_int, ctypes.POINTER(CLaunchInfo)]),
+    "nxb_query_batch_launches": (ctypes.c_int, [_P, ctypes.POINTER(CLaunchInfo)]),
     "nxb_build_async": (ctypes.c_int, [_P, ctypes.c_int, _U32, _P, _P, ctypes.c_size_t, _P, _P, _P, _P, _P]),
     "nxb_build_async_timed": (ctypes.c_int, [_P, ctypes.c_int, _U32, _P, _P, ctypes.c_size_t, _P, _P, _P, _P, _P,
                                              _P]),

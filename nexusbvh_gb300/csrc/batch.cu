@@ -432,6 +432,27 @@ nxb_status nxb_batch_get_arrays(const nxb_batch* b, nxb_batch_arrays* out) {
     return NXB_OK;
 }
 
+nxb_status nxb_query_batch_launches(const nxb_batch* b, nxb_launch_info* out) {
+    if (!b || !out) return NXB_ERR_INVALID_ARGUMENT;
+    const BatchArena& a = b->arena;
+    const BatchSort sort = batch_sort(a, b->tuning.sort_digit_bits);
+    const bool whole = sort.form == BatchSort::kWhole;
+    out->sort_passes = whole ? (uint32_t)sort.plan.passes : kSegmentPasses;
+    out->sort_key_bytes = whole ? 8 : 4;
+    out->kernels = 2;  // begin, finalize
+    if (a.total == 0) return NXB_OK;
+    // bounds, Morton, the sort (and the list of its tiles), then H-PLOC and
+    // the collapse of every group
+    out->kernels += 2 + (sort.form == BatchSort::kClusters ? 1u : sort.form == BatchSort::kSegments ? 1 + kSegmentPasses
+                                                                                                     : out->sort_passes);
+    const MeshGroups& g = b->groups;
+    for (uint32_t k = 0; k < std::max(1u, g.count); ++k) {
+        const uint32_t prims = g.count > 1 ? g.prim[k + 1] - g.prim[k] : a.total;
+        out->kernels += (prims ? 1 : 0) + bvh8_launches(prims, b->auction, g.count <= 1 && a.lists);
+    }
+    return NXB_OK;
+}
+
 nxb_status nxb_batch_set_tuning(nxb_batch* b, const nxb_batch_tuning* t) {
     if (!b || !t) return NXB_ERR_INVALID_ARGUMENT;
     if (!batch_digit_ok(b->arena.mesh_bits, t->sort_digit_bits)) return NXB_ERR_UNSUPPORTED;

@@ -583,6 +583,22 @@ nxb_status nxb_read_bvh8(const char* path, nxb_bvh8* h) {
     return NXB_OK;
 }
 
+nxb_status nxb_query_build_launches(uint32_t n, const nxb_build_config* config, int wide, nxb_launch_info* out) {
+    if (!out || n == 0) return NXB_ERR_INVALID_ARGUMENT;
+    if (n > kMaxPrims) return NXB_ERR_UNSUPPORTED;
+    const nxb_status st = check_config(config);
+    if (st != NXB_OK) return st;
+    const uint32_t key_bits = key_bits_of(config);
+    const bool local = local_sort_takes(n);
+    out->sort_key_bytes = key_bits == 30 ? 4 : 8;
+    // 63-bit keys: four passes, the buckets' sort, which reads and writes the
+    // keys once more, and the launch of the fallback
+    out->sort_passes = local ? (key_bits == 30 ? 4 : 7) : (key_bits == 30 ? 4 : 5);
+    // bounds, Morton, the sort, H-PLOC, the collapse, finalize
+    out->kernels = 2 + (local ? 1 : key_bits == 30 ? 4 : 6) + 1 + (wide ? bvh8_launches(n, auction_of(config), true) : 0) + 1;
+    return NXB_OK;
+}
+
 nxb_status nxb_query_build_sizes(uint32_t n, const nxb_build_config* config, nxb_build_sizes* out) {
     if (!out || n == 0) return NXB_ERR_INVALID_ARGUMENT;
     if (n > kMaxPrims) return NXB_ERR_UNSUPPORTED;

@@ -305,6 +305,8 @@ cudaError_t launch_bvh8_init(uint64_t* pairs, uint32_t n, uint32_t* ctr, cudaStr
 cudaError_t launch_bvh8(const Node2* bvh2, uint32_t n, Node8* out, uint32_t cap, uint32_t* prim_idx, uint64_t* pairs,
                         uint32_t* ctr, uint32_t* err, bool auction, cudaStream_t s,
                         const ChildPair* child_pairs = nullptr, uint64_t* lists = nullptr);
+// Kernels that launch_bvh8 (batch: launch_bvh8_batch) launches with child pairs.
+uint32_t bvh8_launches(uint32_t prims, bool auction, bool lists);
 // ---------------------------------------------------------------- batches
 // The same stages over independent meshes laid end to end (MeshBatch in
 // common.cuh): one launch per stage for the whole batch.

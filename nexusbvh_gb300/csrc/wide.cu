@@ -1200,6 +1200,8 @@ cudaError_t launch_bvh8_init(uint64_t* pairs, uint32_t n, uint32_t* ctr, cudaStr
     return cudaGetLastError();
 }
 
+uint32_t bvh8_launches(uint32_t prims, bool auction, bool lists) { return lists && takes_lists(prims, auction) ? 2 : 1; }
+
 cudaError_t launch_bvh8(const Node2* bvh2, uint32_t n, Node8* out, uint32_t cap, uint32_t* prim_idx, uint64_t* pairs,
                         uint32_t* ctr, uint32_t* err, bool auction, cudaStream_t s, const ChildPair* child_pairs,
                         uint64_t* lists) {
