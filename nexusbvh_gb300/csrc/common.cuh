@@ -138,15 +138,7 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release_u32(uint32_t* p, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-__device__ __forceinline__ uint32_t atom_exch_acq_rel(uint32_t* p, uint32_t v) {
-    uint32_t old;
-    asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
-}
 
 // For kernels launched by launch_after (pipeline.h): waits for the kernel
 // before in the stream, which has then finished and whose writes are seen,
@@ -175,15 +167,6 @@ __device__ __forceinline__ float4 ld_stream(const float4* p) {
     float4 v;
     asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
-}
-__device__ __forceinline__ Box load_box_cg(const Node2* nodes, uint32_t i) {
-    const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    float4 a = __ldcg(p);
-    float2 b = __ldcg(reinterpret_cast<const float2*>(p + 1));
-    Box r;
-    r.mn = make_float3(a.x, a.y, a.z);
-    r.mx = make_float3(a.w, b.x, b.y);
-    return r;
 }
 __device__ __forceinline__ Box load_box(const Node2* nodes, uint32_t i) {
     const float4* p = reinterpret_cast<const float4*>(nodes + i);

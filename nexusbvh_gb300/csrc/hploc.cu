@@ -351,9 +351,10 @@ __device__ __forceinline__ void publish(Node2* rec, uint32_t pos, const Box& b, 
 // warp.  Gap j of a tile lies between its positions j-1 and j (0..cnt).
 // Largest tile and resident warps, measured on GB300 (H-PLOC of 12.58M
 // clustered triangles, 63-bit): 128 leaves x 31 warps (64 registers, spills)
-// 2.23 ms, 144 x 28 (72 registers, no spills at radius 8) 2.12, 160 x 26
-// 2.16, 176 x 24 2.17, 192 x 22 2.22.  Four CTAs of 7 warps and one of 28
-// measure the same; the small CTA leaves room beside it on the SM.
+// 2.23 ms, 144 x 28 (72 registers; a few spilled at radius 16 and in the
+// batched forms) 2.12, 160 x 26 2.16, 176 x 24 2.17, 192 x 22 2.22.  Four CTAs
+// of 7 warps and one of 28 measure the same; the small CTA leaves room beside
+// it on the SM.
 constexpr int kTile = 144;
 constexpr int kTileWarps = 7;  // per CTA
 constexpr int kTileCtas = 4;   // per SM

@@ -50,9 +50,8 @@ constexpr uint32_t kHybridTopShift = 28;
 // Small per-build state, cleared by one memset at the start of a build.
 struct Control {
     uint32_t scene_ord[6];  // [0..2]: ~ordered(min) (atomicMax), [3..5]: ordered(max)
-    uint32_t cluster_count; // H-PLOC node allocator
     uint32_t error_word;
-    uint32_t pad0[16];
+    uint32_t pad0[17];
     alignas(128) uint32_t bvh8_ctr[160];  // BVH8 counters, one per 128-byte line (kBvh8* below)
     uint32_t parent_of_last; // H-PLOC: the node whose child is node 2n-2 (seeded INVALID)
     uint32_t hploc_tile_ctr; // H-PLOC: next unclaimed tile
@@ -363,12 +362,12 @@ cudaError_t launch_batch_begin(const BatchBegin& b, const MeshBatch& batch, cuda
 // The collapse of the meshes of `batch` (a whole batch, or one group's view:
 // off, off8, mesh_nodes and mesh_leaves advanced to the group's first mesh,
 // pairs to its first slot, ctr to its counters).  child_pairs: as for
-// launch_bvh8, the records launch_hploc_batch wrote (mesh m's at off[m]).
-// lists: as for launch_bvh8, only for a whole batch.
+// launch_bvh8, the records launch_hploc_batch wrote (mesh m's at off[m]);
+// always there.  lists: as for launch_bvh8, only for a whole batch.
 cudaError_t launch_bvh8_batch(const Node2* bvh2, const MeshBatch& batch, uint32_t total, Node8* out, uint32_t slots,
                               uint32_t* prim_idx, uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
                               uint32_t* mesh_leaves, uint32_t* err, bool auction, cudaStream_t s,
-                              const ChildPair* child_pairs = nullptr, uint64_t* lists = nullptr);
+                              const ChildPair* child_pairs, uint64_t* lists = nullptr);
 cudaError_t launch_batch_finalize(const MeshBatch& batch, const uint32_t* scene_ord, const uint32_t* mesh_nodes,
                                   const uint32_t* mesh_leaves, nxb_batch_mesh* out, cudaStream_t s);
 // One batched build's device memory (a single allocation carved into

@@ -1126,9 +1126,10 @@ cudaError_t by_keys_per_thread(uint32_t n, uint32_t ctas, F f) {
 // the values from the positions, the last writes mesh << 32 | code, which
 // the climb reads.  Bound by ranking and its shared-memory traffic, not by
 // DRAM: 16 keys per thread and four CTAs per SM (five for the first pass,
-// which holds no values).  1,024 meshes of 36.5M triangles together: 193 +
-// 3 x 214 us, where five passes over 64-bit keys took 1,701; with five CTAs
-// throughout the later passes spill and take 223 each, with three 250.
+// which holds no values; each form spills a register or two).  1,024 meshes of
+// 36.5M triangles together: 193 + 3 x 214 us, where five passes over 64-bit
+// keys took 1,701; with five CTAs throughout the later passes spill more and
+// take 223 each, with three 250.
 constexpr uint32_t kSegmentMinMean = 1536;
 
 __global__ __launch_bounds__(kThreads) void segment_prepare_kernel(SegmentPlan plan, MeshBatch batch) {

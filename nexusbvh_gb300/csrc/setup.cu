@@ -149,10 +149,10 @@ struct MortonArgs {
     int seed;
 };
 
-// PASSES > 0: the pass count of the plan, known at compile time (4 for
-// 30-bit keys, 4 for the 9-bit top passes of 63-bit keys), so the histogram
-// loop unrolls.  BINS: digits per pass (256, or 512 for 9-bit digits); the
-// histograms are laid out pass after pass, BINS words each.
+// PASSES: the pass count of the plan (four for 30-bit keys, four for the 9-bit
+// top passes of 63-bit keys), known when compiled so that the histogram loop
+// unrolls.  BINS: words per pass (256, or 512 for 9-bit digits); the
+// histograms are laid out pass after pass.
 template <typename K, bool HIST, int PASSES = 0, int BINS = kRadixBins>
 __global__ __launch_bounds__(kThreads) void morton_kernel(const Node2* nodes, uint32_t n, Control* ctrl,
                                                           K* keys, MortonArgs a) {
@@ -170,10 +170,7 @@ __global__ __launch_bounds__(kThreads) void morton_kernel(const Node2* nodes, ui
     const float3 smin = make_float3(s_scene[0], s_scene[1], s_scene[2]);
     const float3 smax = make_float3(s_scene[3], s_scene[4], s_scene[5]);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (a.seed) {
-            ctrl->cluster_count = n;
-            ctrl->parent_of_last = kInvalid;
-        }
+        if (a.seed) ctrl->parent_of_last = kInvalid;
         if (a.scene_out) {
             a.scene_out->bmin[0] = smin.x;
             a.scene_out->bmin[1] = smin.y;
@@ -202,22 +199,14 @@ __global__ __launch_bounds__(kThreads) void morton_kernel(const Node2* nodes, ui
             if (a.parent) a.parent[i] = kInvalid;
         }
         if (HIST) {
-            if constexpr (PASSES > 0) {
 #pragma unroll
-                for (int p = 0; p < PASSES; ++p) {
-                    const uint32_t d = (uint32_t)(key >> a.pd.shift[p]) & a.pd.mask[p];
-                    if (p < PASSES / 2) {
-                        // low digits: neighbouring keys rarely share them,
-                        // so the warp-uniform test seldom pays for itself
-                        if (valid) atomicAdd(&s_hist[p * BINS + d], 1u);
-                    } else {
-                        hist_add(s_hist + p * BINS, d, valid);
-                    }
-                }
-            } else {
-#pragma unroll 1
-                for (int p = 0; p < a.pd.passes; ++p) {
-                    uint32_t d = (uint32_t)(key >> a.pd.shift[p]) & a.pd.mask[p];
+            for (int p = 0; p < PASSES; ++p) {
+                const uint32_t d = (uint32_t)(key >> a.pd.shift[p]) & a.pd.mask[p];
+                if (p < PASSES / 2) {
+                    // low digits: neighbouring keys rarely share them,
+                    // so the warp-uniform test seldom pays for itself
+                    if (valid) atomicAdd(&s_hist[p * BINS + d], 1u);
+                } else {
                     hist_add(s_hist + p * BINS, d, valid);
                 }
             }
@@ -744,16 +733,15 @@ cudaError_t launch_morton(const Node2* nodes, uint32_t n, Control* ctrl, int key
     auto go = [&](auto* kernel, auto* out) {
         return launch_after(n, kernel, grid, kThreads, 0, s, nodes, n, ctrl, out, a);
     };
+    // the plans of the pipeline's sorts: four 7-bit digits, four 9-bit digits
+    if (f.plan && (a.pd.passes != 4 || a.pd.mask[0] != (1u << (key_bits == 30 ? kSegmentBits : kMaxRadixBits)) - 1u))
+        return cudaErrorInvalidValue;
     if (key_bits == 30) {
         uint32_t* out = (uint32_t*)keys;
-        if (!f.plan) return go(morton_kernel<uint32_t, false>, out);
-        return a.pd.passes == 4 ? go(morton_kernel<uint32_t, true, 4>, out) : go(morton_kernel<uint32_t, true>, out);
+        return f.plan ? go(morton_kernel<uint32_t, true, 4>, out) : go(morton_kernel<uint32_t, false>, out);
     }
     uint64_t* out = (uint64_t*)keys;
-    if (!f.plan) return go(morton_kernel<uint64_t, false>, out);
-    if (a.pd.passes == 4 && a.pd.mask[0] == (1u << kMaxRadixBits) - 1u)
-        return go(morton_kernel<uint64_t, true, 4, 1 << kMaxRadixBits>, out);
-    return a.pd.passes == 8 ? go(morton_kernel<uint64_t, true, 8>, out) : go(morton_kernel<uint64_t, true>, out);
+    return f.plan ? go(morton_kernel<uint64_t, true, 4, 1 << kMaxRadixBits>, out) : go(morton_kernel<uint64_t, false>, out);
 }
 
 cudaError_t launch_morton_scene(const Node2* nodes, uint32_t n, const nxb_aabb* scene, int key_bits, void* keys,

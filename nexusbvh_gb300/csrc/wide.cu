@@ -1228,27 +1228,20 @@ cudaError_t launch_bvh8_batch(const Node2* bvh2, const MeshBatch& batch, uint32_
                               uint32_t* prim_idx, uint64_t* pairs, uint32_t* ctr, uint32_t* mesh_nodes,
                               uint32_t* mesh_leaves, uint32_t* err, bool auction, cudaStream_t s,
                               const ChildPair* child_pairs, uint64_t* lists) {
-    if (child_pairs && lists && takes_lists(total, auction))
+    if (lists && takes_lists(total, auction))
         return launch_group<MeshBatch, false, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr,
                                                     mesh_nodes, mesh_leaves, err, s, child_pairs, lists);
-    if (child_pairs && takes_groups(total, auction)) {
-        if (auction)
-            return launch_group<MeshBatch, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
-                                                 mesh_leaves, err, s, child_pairs);
+    if (takes_groups(total, auction) && auction)
+        return launch_group<MeshBatch, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
+                                             mesh_leaves, err, s, child_pairs);
+    if (takes_groups(total, auction))
         return launch_group<MeshBatch, false>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
                                               mesh_leaves, err, s, child_pairs);
-    }
-    if (child_pairs && auction)
+    if (auction)
         return launch_wide<MeshBatch, true, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
                                                   mesh_leaves, err, s, child_pairs);
-    if (child_pairs)
-        return launch_wide<MeshBatch, false, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr,
-                                                   mesh_nodes, mesh_leaves, err, s, child_pairs);
-    if (auction)
-        return launch_wide<MeshBatch, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
-                                            mesh_leaves, err, s);
-    return launch_wide<MeshBatch, false>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
-                                         mesh_leaves, err, s);
+    return launch_wide<MeshBatch, false, true>(bvh2, batch, total, out, 0u, slots, prim_idx, pairs, ctr, mesh_nodes,
+                                               mesh_leaves, err, s, child_pairs);
 }
 
 cudaError_t load_collapse_kernels() {
