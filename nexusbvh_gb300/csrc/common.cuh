@@ -152,7 +152,18 @@ __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// Streaming loads (evicted first) that stay behind after_previous().
+// Loads through L2 and streaming loads (evicted first) that stay behind
+// after_previous().
+__device__ __forceinline__ uint32_t ld_l2(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint64_t ld_l2(const uint64_t* p) {
+    uint64_t v;
+    asm volatile("ld.global.cg.u64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ float ld_stream(const float* p) {
     float v;
     asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p));

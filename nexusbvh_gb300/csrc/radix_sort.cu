@@ -998,16 +998,10 @@ __global__ __launch_bounds__(kLocalThreads) void sort_cluster_kernel(K* keys, ui
     using S = LocalSmem<Element<K>, RB, KPT>;
     S& sm = *reinterpret_cast<S*>(smem);
     const uint32_t me = cluster_rank(), first = me * S::kTile;
-    K key[KPT];  // every load before the stores: an ordinary load does not pass a store
-#pragma unroll
-    for (int j = 0; j < KPT; ++j) {
-        const uint32_t k = first + threadIdx.x + j * kLocalThreads;
-        key[j] = k < n ? keys[k] : (K)0;
-    }
 #pragma unroll
     for (int j = 0; j < KPT; ++j) {
         const uint32_t k = threadIdx.x + j * kLocalThreads;
-        make_element(sm.key[k], key[j], first + k);
+        make_element(sm.key[k], first + k < n ? ld_l2(keys + first + k) : (K)0, first + k);
     }
     __syncthreads();
     local_sort<Element<K>, RB, KPT>(sm, n, shift, passes, gridDim.x, me);
